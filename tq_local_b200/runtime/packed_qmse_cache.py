@@ -30,7 +30,7 @@ import torch
 from transformers.cache_utils import Cache, CacheLayerMixin
 
 from tq_local_b200.runtime.codec import Codec
-from tq_local_b200.runtime.packed_store import PackedStore, key_norm_mean
+from tq_local_b200.runtime.packed_store import PackedStore, key_norm_mean, key_norm_means
 from tq_local_b200.runtime.sharding import HeadShard
 
 
@@ -675,7 +675,7 @@ def build_packed_mse_cache(
     head_dim = int(pairs[0][0].shape[-1]) if pairs else 128
     threshold = _auto_norm_threshold(bits, head_dim) if norm_guard else float("inf")
     if norm_guard and pairs:
-        means = torch.stack([key_norm_mean(k) for k, _ in pairs]).tolist()
+        means = key_norm_means([k for k, _ in pairs])
     else:
         means = [0.0] * len(pairs)
 

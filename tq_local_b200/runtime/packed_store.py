@@ -409,6 +409,20 @@ class PackedStore:
         return out
 
 
+def _add_key_norm_sum(k: torch.Tensor, acc_ptr: int) -> int:
+    """Queue the sum of the L2 norms of all vectors of ``k`` [B, H, T, 128] into the float64 at
+    ``acc_ptr`` on its device; returns how many vectors there are."""
+    if k.stride(-1) != 1:
+        k = k.contiguous()
+    kd = dense_desc(k)
+    b, h, t = int(k.shape[0]), int(k.shape[1]), int(k.shape[2])
+    with torch.cuda.device(k.device):
+        ffi.check(ffi.lib().tq_key_norm_sum(C.byref(kd), b, h, t, acc_ptr,
+                                            C.c_void_p(torch.cuda.current_stream(k.device).cuda_stream)),
+                  "tq_key_norm_sum")
+    return b * h * t
+
+
 def key_norm_mean(k: torch.Tensor) -> torch.Tensor:
     """Mean L2 norm over all vectors of ``k`` [B, H, T, 128] as a 0-dim float64 device tensor
     (no host sync); the norm-guard statistic of ``build_packed_mse_cache``
@@ -416,12 +430,22 @@ def key_norm_mean(k: torch.Tensor) -> torch.Tensor:
     if k.device.type != "cuda":
         raise ffi.TQError("TurboQuant-B200 runs on CUDA devices only; there is no CPU path")
     acc = torch.zeros((), dtype=torch.float64, device=k.device)
-    if k.stride(-1) != 1:
-        k = k.contiguous()
-    kd = dense_desc(k)
-    b, h, t = int(k.shape[0]), int(k.shape[1]), int(k.shape[2])
-    with torch.cuda.device(k.device):
-        ffi.check(ffi.lib().tq_key_norm_sum(C.byref(kd), b, h, t, acc.data_ptr(),
-                                            C.c_void_p(torch.cuda.current_stream(k.device).cuda_stream)),
-                  "tq_key_norm_sum")
-    return acc / (b * h * t)
+    return acc / _add_key_norm_sum(k, acc.data_ptr())
+
+
+def key_norm_means(keys: list[torch.Tensor]) -> list[float]:
+    """``key_norm_mean`` of every tensor of a list, fetched with one host synchronisation per device (the sums of all
+    layers share one buffer, and nothing but the library's kernel runs per layer)."""
+    means = [0.0] * len(keys)
+    by_device: dict[torch.device, list[int]] = {}
+    for i, k in enumerate(keys):
+        if k.device.type != "cuda":
+            raise ffi.TQError("TurboQuant-B200 runs on CUDA devices only; there is no CPU path")
+        by_device.setdefault(k.device, []).append(i)
+    sums = {dev: torch.zeros(len(idx), dtype=torch.float64, device=dev) for dev, idx in by_device.items()}
+    counts = {i: _add_key_norm_sum(keys[i], sums[dev].data_ptr() + 8 * j)
+              for dev, idx in by_device.items() for j, i in enumerate(idx)}
+    for dev, idx in by_device.items():
+        for i, total in zip(idx, sums[dev].tolist()):
+            means[i] = total / counts[i]
+    return means
