@@ -66,3 +66,41 @@ def test_key_norm_mean(dtype, shape, form):
     both = key_norm_means([x, x[:, :, :1]])
     assert abs(both[0] - want) <= 128 * 2.0 ** -24 * want and both[1] > 0
 
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("groups", [1, 4, 5, 8])
+@pytest.mark.parametrize("n_tail", [1, 63, 64, 255, 256, 257, 700])
+def test_dense_tail(setup_golden, dtype, groups, n_tail):
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(4, True, setup_golden), make_codec(4, True, setup_golden)
+    store = PackedStore(codec, 2, 2, capacity=256)
+    store.pack(vectors((2, 2, 70, 128), 1, dtype), vectors((2, 2, 70, 128), 2, dtype))
+    q = query((2, 2 * groups, 1), 3, dtype)
+    tk, tv = vectors((2, 2, n_tail, 128), 4, dtype), vectors((2, 2, n_tail, 128), 5, dtype)
+    want = attend64(store, p, q, groups, tk, tv)
+    got = store.decode_attn(q, tail_k=tk, tail_v=tv)
+    assert rel_inf(got, want) <= ATTN_TOL[dtype]
+    # the same values, a row stride that is no multiple of the row and unaligned rows: the same bits
+    wide = torch.zeros(2, 2, n_tail, 136, dtype=dtype, device="cuda")
+    wide[..., :128] = tk
+    assert torch.equal(got, store.decode_attn(q, tail_k=wide[..., :128], tail_v=off_by_one(tv)))
+    store.length = 0  # nothing packed: the tail alone
+    k, v = tk.cpu().double().repeat_interleave(groups, dim=1), tv.cpu().double().repeat_interleave(groups, dim=1)
+    alone = torch.softmax(q.cpu().double() @ k.transpose(-1, -2) / math.sqrt(128), dim=-1) @ v
+    assert rel_inf(store.decode_attn(q, tail_k=tk, tail_v=tv), alone) <= ATTN_TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("splits", [1, 2, 8, 9, 31, 32, 33, 41, 70])
+def test_split_merge(setup_golden, dtype, splits):
+    """Every remainder of the merge's batches of 8 and 32 partials (one long row, so that the splits are used)."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(3, True, setup_golden), make_codec(3, True, setup_golden)
+    n = 512 * (splits - 1) + 3 if splits > 1 else 77
+    store = PackedStore(codec, 1, 1, capacity=n)
+    store.pack(vectors((1, 1, n, 128), 1, dtype), vectors((1, 1, n, 128), 2, dtype))
+    q = query((1, 5, 1), 3, dtype)
+    assert rel_inf(store.decode_attn(q, splits=splits), attend64(store, p, q, 5)) <= ATTN_TOL[dtype]
+

@@ -222,69 +222,6 @@ __global__ void __launch_bounds__(TQ_D) tq_qprep_kernel(const T *q, const float 
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(TQ_D) tq_combine_kernel(CombineArgs a) {
-    extern __shared__ float s_dyn[];  // tail logits
-    __shared__ float s_o[TQ_D];
-    __shared__ float s_q[TQ_D];
-    __shared__ float s_red[4];
-    const int64_t row = blockIdx.x;  // b * Hq + hq
-    const int e = threadIdx.x;
-    const int warp = e >> 5, lane = e & 31;
-    const int b = (int)(row / a.Hq), hq = (int)(row % a.Hq);
-    const float hs = 0.08838834764831845f;
-
-    int n_valid = a.n_splits;
-    if (a.seg_chunk > 0) {
-        const int64_t lo = (row / a.G) * (int64_t)a.seg_npad;
-        n_valid = (int)((lo + a.seg_npad - 1) / a.seg_chunk - lo / a.seg_chunk) + 1;
-    }
-    float M = -INFINITY;
-    for (int s = 0; s < n_valid; ++s) M = fmaxf(M, a.part_m[row * a.n_splits + s]);
-
-    // dense tail logits (quantize_decode = False buffer)
-    const T *tk = nullptr, *tv = nullptr;
-    if (a.n_tail > 0) {
-        const int hkv = hq / a.G;
-        tk = (const T *)a.tail_k + b * a.tk_sb + hkv * a.tk_sh;
-        tv = (const T *)a.tail_v + b * a.tv_sb + hkv * a.tv_sh;
-        s_q[e] = tq_to_float<T>(((const T *)a.q)[row * TQ_D + e]);
-        __syncthreads();
-        float wmax = -INFINITY;
-        for (int t = warp; t < a.n_tail; t += 4) {
-            const T *kr = tk + (int64_t)t * a.tk_st + 4 * lane;
-            float dsum = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) dsum = fmaf(s_q[4 * lane + i], tq_to_float<T>(kr[i]), dsum);
-            dsum = tq_warp_sum(dsum) * hs;
-            if (lane == 0) s_dyn[t] = dsum;
-            wmax = fmaxf(wmax, dsum);
-        }
-        if (lane == 0) s_red[warp] = wmax;
-        __syncthreads();
-        M = fmaxf(M, fmaxf(fmaxf(s_red[0], s_red[1]), fmaxf(s_red[2], s_red[3])));
-    }
-
-    float L = 0.f, o = 0.f;
-    for (int s = 0; s < n_valid; ++s) {
-        const float ms = a.part_m[row * a.n_splits + s];
-        const float w = (ms == -INFINITY) ? 0.f : expf(ms - M);
-        L += a.part_l[row * a.n_splits + s] * w;
-        o += a.part_acc[(row * a.n_splits + s) * TQ_D + e] * w;
-    }
-    s_o[e] = o;
-    __syncthreads();
-    float out = 0.f;
-#pragma unroll 8
-    for (int d = 0; d < TQ_D; ++d) out = fmaf(s_o[d], __ldg(a.rot_v + d * TQ_D + e), out);
-    for (int t = 0; t < a.n_tail; ++t) {
-        const float p = expf(s_dyn[t] - M);
-        L += p;
-        out = fmaf(p, tq_to_float<T>(tv[(int64_t)t * a.tv_st + e]), out);
-    }
-    ((T *)a.out)[row * TQ_D + e] = tq_from_float<T>(out / fmaxf(L, 1e-8f));
-}
-
 // Query preparation for the tensor-core kernel (see tq_qprep_block): kv_rows * ceil(G / 4) blocks
 // rotate, another kv_rows blocks project when the keys carry a QJL sketch.  Launched as a
 // programmatic dependent of whatever precedes it in the stream: a block fetches its matrix
@@ -304,8 +241,9 @@ __global__ void __launch_bounds__(4 * TQ_D, 2) tq_step_prologue_kernel(TqQprepAr
         tq_pack_small_block<T, QJL>(pa, (int64_t)blockIdx.x - n_qprep);
 }
 
-// Split combine for up to four heads of one (batch, KV head) row per block (no dense tail):
-// the un-rotation matrix is read once for the G heads.
+// Split combine for up to four heads of one (batch, KV head) row per block: the un-rotation
+// matrix is read once for the G heads, and the un-quantised tail of the row, if there is one
+// (TAIL), is attended by the same block.
 // Publishing rows to the peers and waiting for theirs (system scope, PTX memory model):
 // a block's threads store their rows with plain stores, the block barrier orders those stores
 // before thread 0, which adds the block's row count to the flag word with a RELEASE reduction at
@@ -322,7 +260,136 @@ __device__ __forceinline__ unsigned tq_acquire_load_sys(const unsigned *word) {
     return v;
 }
 
+// Eight consecutive elements as floats: one (16-bit types) or two (fp32) 16-byte loads when the
+// tensor is 16-byte aligned (`vec`, uniform over the launch), else element by element.
+template <typename T> __device__ __forceinline__ void tq_load8(const T *p, bool vec, float (&v)[8]) {
+    if (vec) {
+        uint4 raw[sizeof(T) / 2];
+#pragma unroll
+        for (int i = 0; i < (int)sizeof(T) / 2; ++i) raw[i] = __ldg(reinterpret_cast<const uint4 *>(p) + i);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = tq_to_float<T>(reinterpret_cast<const T *>(raw)[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = tq_to_float<T>(p[i]);
+    }
+}
+
+// Attention of up to four heads of one KV row over the row's un-quantised tail tokens, by the 512
+// threads of a combine block, 256 tokens at a time with an online softmax.  Logits: eight lanes
+// share a token, so a warp reads four whole rows per load and sums each over three shuffles;
+// values: sixteen threads cover a row with 16-byte loads and 32 rows are read side by side.
+// Returns this thread's element (head threadIdx.x / 128, column threadIdx.x % 128) of the
+// unnormalised sum; the maximum and the sum of every head are left in s_tm / s_tl.
+// What bounds it is the latency of two dependent trips to memory per 256 tokens.  The whole kernel for
+// a tail of 300 tokens, 8 KV rows: 17 us; one thread per output column walking the tail alone: 59 us.
+constexpr int kTailChunk = 256;
+struct TailShared {
+    float p[4][kTailChunk];
+    float corr[4], m[4], l[4];
+    float acc[16][4][TQ_D];
+};
 template <typename T>
+__device__ __forceinline__ float tq_attend_tail(const CombineArgs &a, TailShared &sm, int64_t R, int h0, int n_heads) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t row0 = R * a.G + h0;
+    const int b = (int)(row0 / a.Hq), hkv = (int)(row0 % a.Hq) / a.G;
+    const T *tk = (const T *)a.tail_k + b * a.tk_sb + hkv * a.tk_sh;
+    const T *tv = (const T *)a.tail_v + b * a.tv_sb + hkv * a.tv_sh;
+    const float hs = 0.08838834764831845f;
+    const int sub = lane & 7, tg = tid >> 4, dc = 8 * (tid & 15);
+    float acc[4][8];
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
+    float q[4][16];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const T *qr = (const T *)a.q + (row0 + (g < n_heads ? g : 0)) * TQ_D + 16 * sub;  // (q is 16-byte aligned)
+        float lo[8], hi[8];
+        tq_load8<T>(qr, true, lo), tq_load8<T>(qr + 8, true, hi);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) q[g][i] = lo[i], q[g][8 + i] = hi[i];
+    }
+    float m_run = -INFINITY, l_run = 0.f;  // warp g < 4: head g
+    for (int c0 = 0; c0 < a.n_tail; c0 += kTailChunk) {
+        const int n = min(kTailChunk, a.n_tail - c0);
+#pragma unroll
+        for (int it = 0; it < kTailChunk / 64; ++it) {
+            const int t = 64 * it + 4 * warp + (lane >> 3);
+            float d[4] = {0.f, 0.f, 0.f, 0.f};
+            if (t < n) {
+                const T *kr = tk + (int64_t)(c0 + t) * a.tk_st + 16 * sub;
+                float lo[8], hi[8];
+                tq_load8<T>(kr, a.tail_vec, lo), tq_load8<T>(kr + 8, a.tail_vec, hi);
+#pragma unroll
+                for (int g = 0; g < 4; ++g)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) d[g] = fmaf(q[g][i], lo[i], d[g]), d[g] = fmaf(q[g][8 + i], hi[i], d[g]);
+            }
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) d[g] += __shfl_xor_sync(0xffffffffu, d[g], o);
+                if (sub == 0) sm.p[g][t] = t < n ? d[g] * hs : -INFINITY;
+            }
+        }
+        __syncthreads();
+        if (warp < 4) {
+            float x[kTailChunk / 32], mx = -INFINITY, sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < kTailChunk / 32; ++i) x[i] = sm.p[warp][32 * i + lane], mx = fmaxf(mx, x[i]);
+            const float nm = fmaxf(m_run, tq_warp_max(mx));  // (finite: a chunk holds at least one token)
+            const float corr = expf(m_run - nm);
+#pragma unroll
+            for (int i = 0; i < kTailChunk / 32; ++i) {
+                const float p = expf(x[i] - nm);
+                sm.p[warp][32 * i + lane] = p, sum += p;
+            }
+            l_run = l_run * corr + tq_warp_sum(sum), m_run = nm;
+            if (lane == 0) sm.corr[warp] = corr;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const float corr = sm.corr[g];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[g][i] *= corr;
+        }
+#pragma unroll 4
+        for (int t = tg; t < n; t += 32) {
+            float v[8];
+            tq_load8<T>(tv + (int64_t)(c0 + t) * a.tv_st + dc, a.tail_vec, v);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const float p = sm.p[g][t];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[g][i] = fmaf(p, v[i], acc[g][i]);
+            }
+        }
+        __syncthreads();  // the weights are free for the next chunk
+    }
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[g][i] += __shfl_xor_sync(0xffffffffu, acc[g][i], 16);
+    if (lane < 16) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+#pragma unroll
+            for (int i = 0; i < 8; i += 4)
+                *reinterpret_cast<float4 *>(&sm.acc[warp][g][dc + i]) = make_float4(acc[g][i], acc[g][i + 1], acc[g][i + 2], acc[g][i + 3]);
+    }
+    if (warp < 4 && lane == 0) sm.m[warp] = m_run, sm.l[warp] = l_run;
+    __syncthreads();
+    float o = 0.f;
+#pragma unroll
+    for (int w = 0; w < 16; ++w) o += sm.acc[w][tid >> 7][tid & (TQ_D - 1)];
+    return o;
+}
+
+template <typename T, bool TAIL>
 __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs a) {
     __shared__ __align__(16) float s_o[4][TQ_D];
     __shared__ float s_part[4][4][TQ_D];  // [quarter of d][head][column]
@@ -331,7 +398,15 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
     const int64_t R = blockIdx.x / groups;
     const int h0 = 4 * (blockIdx.x % groups);
     const int n_heads = a.G - h0 < 4 ? a.G - h0 : 4;
-    const int tid = threadIdx.x, e = tid & (TQ_D - 1), dq = tid >> 7;
+    const int tid = threadIdx.x, e = tid & (TQ_D - 1), dq = tid >> 7, lane = tid & 31;
+    float tail_o = 0.f, tail_m = -INFINITY, tail_l = 0.f;  // of head dq, column e
+    if (TAIL) {
+        extern __shared__ __align__(16) uint8_t s_dyn[];
+        TailShared &ts = *reinterpret_cast<TailShared *>(s_dyn);
+        tq_grid_dependency_wait();  // (the query and the tail may come from any earlier kernel of the stream)
+        tail_o = tq_attend_tail<T>(a, ts, R, h0, n_heads);
+        tail_m = ts.m[dq], tail_l = ts.l[dq];
+    }
     float rv[32];  // this thread's un-rotation elements, fetched while the decode kernel drains
     tq_load_column(rv, a.rot_v, dq, e);
     tq_grid_dependency_wait();
@@ -346,37 +421,31 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
         const int64_t lo = R * (int64_t)seg_npad;
         n_valid = (int)((lo + seg_npad - 1) / seg_chunk - lo / seg_chunk) + 1;
     }
-    {   // thread (e, dq) merges the splits of head dq
+    {   // thread (e, dq) merges the splits of head dq, 32 at a time: lane s of each warp holds split s's
+        // maximum and weight, the accumulator columns are requested eight splits at a time.  (The kernel
+        // takes 5.6 us for 33 splits of 4 rows; with one thread walking all splits twice it took 10.8.)
         const int g = dq;
         float o = 0.f, L = 0.f, Mx = -INFINITY;
         if (g < n_heads) {
-            const int64_t row = R * a.G + h0 + g;
-            if (n_valid <= 4) {  // the usual case: everything is requested in one batch of loads
-                float pm[4], pl[4], pa[4];
+            const int64_t slot0 = (R * a.G + h0 + g) * a.n_splits;
+            for (int s0 = 0; s0 < n_valid; s0 += 32) {
+                const int n = min(32, n_valid - s0);
+                const float *acc = a.part_acc + (slot0 + s0) * TQ_D + e;
+                float pa[8];
 #pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const bool on = s < n_valid;
-                    pm[s] = on ? a.part_m[row * a.n_splits + s] : -INFINITY;
-                    pl[s] = on ? a.part_l[row * a.n_splits + s] : 0.f;
-                    pa[s] = on ? a.part_acc[(row * a.n_splits + s) * TQ_D + e] : 0.f;
-                }
-                const float M = fmaxf(fmaxf(pm[0], pm[1]), fmaxf(pm[2], pm[3]));
-                Mx = M;
+                for (int i = 0; i < 8; ++i) pa[i] = i < n ? acc[i * TQ_D] : 0.f;
+                const float pm = lane < n ? a.part_m[slot0 + s0 + lane] : -INFINITY;
+                const float pl = lane < n ? a.part_l[slot0 + s0 + lane] : 0.f;
+                const float M = fmaxf(Mx, tq_warp_max(pm));
+                const float corr = Mx == -INFINITY ? 0.f : expf(Mx - M);
+                const float w = pm == -INFINITY ? 0.f : expf(pm - M);
+                L = L * corr + tq_warp_sum(pl * w), o *= corr, Mx = M;
+                for (int i0 = 0; i0 < n; i0 += 8) {
+                    float cur[8];
 #pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const float w = (pm[s] == -INFINITY) ? 0.f : expf(pm[s] - M);
-                    L += pl[s] * w;
-                    o += pa[s] * w;
-                }
-            } else {
-                float M = -INFINITY;
-                for (int s = 0; s < n_valid; ++s) M = fmaxf(M, a.part_m[row * a.n_splits + s]);
-                Mx = M;
-                for (int s = 0; s < n_valid; ++s) {
-                    const float ms = a.part_m[row * a.n_splits + s];
-                    const float w = (ms == -INFINITY) ? 0.f : expf(ms - M);
-                    L += a.part_l[row * a.n_splits + s] * w;
-                    o += a.part_acc[(row * a.n_splits + s) * TQ_D + e] * w;
+                    for (int i = 0; i < 8; ++i) cur[i] = pa[i], pa[i] = i0 + 8 + i < n ? acc[(i0 + 8 + i) * TQ_D] : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o = fmaf(cur[i], __shfl_sync(0xffffffffu, w, i0 + i), o);
                 }
             }
         }
@@ -422,13 +491,19 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
     __syncthreads();
     if (dq < n_heads) {
         const int g = dq;
-        const float v = (s_part[0][g][e] + s_part[1][g][e]) + (s_part[2][g][e] + s_part[3][g][e]);
-        const T res = tq_from_float<T>(v / fmaxf(s_L[g], 1e-8f));
+        float v = (s_part[0][g][e] + s_part[1][g][e]) + (s_part[2][g][e] + s_part[3][g][e]);
+        float L = s_L[g];
+        if (TAIL) {  // (tail_m is finite: a tail has at least one token)
+            const float M = fmaxf(s_M[g], tail_m), wt = expf(tail_m - M);
+            const float wp = s_M[g] == -INFINITY ? 0.f : expf(s_M[g] - M);
+            v = v * wp + tail_o * wt, L = L * wp + tail_l * wt;
+        }
+        const T res = tq_from_float<T>(v / fmaxf(L, 1e-8f));
         const int64_t row = R * a.G + h0 + g;  // = batch index * local query heads + local head
         if (a.gather_world > 0) {
             reinterpret_cast<T *>(&s_o[0][0])[g * TQ_D + e] = res;  // staged: the peers get 16-byte stores below
         } else if (a.out_f32) {
-            a.out_f32[row * TQ_D + e] = v / fmaxf(s_L[g], 1e-8f);
+            a.out_f32[row * TQ_D + e] = v / fmaxf(L, 1e-8f);
         } else {
             ((T *)a.out)[row * TQ_D + e] = res;
         }
@@ -530,15 +605,15 @@ static void configure_small_kernels() {
     prefer_max_shared(tq_qprep_kernel<float>);
     prefer_max_shared(tq_qprep_kernel<__half>);
     prefer_max_shared(tq_qprep_kernel<__nv_bfloat16>);
-    prefer_max_shared(tq_combine_kernel<float>);
-    prefer_max_shared(tq_combine_kernel<__half>);
-    prefer_max_shared(tq_combine_kernel<__nv_bfloat16>);
     prefer_max_shared(tq_qprep_frag_kernel<float>);
     prefer_max_shared(tq_qprep_frag_kernel<__half>);
     prefer_max_shared(tq_qprep_frag_kernel<__nv_bfloat16>);
-    prefer_max_shared(tq_combine_group_kernel<float>);
-    prefer_max_shared(tq_combine_group_kernel<__half>);
-    prefer_max_shared(tq_combine_group_kernel<__nv_bfloat16>);
+    prefer_max_shared(tq_combine_group_kernel<float, false>);
+    prefer_max_shared(tq_combine_group_kernel<__half, false>);
+    prefer_max_shared(tq_combine_group_kernel<__nv_bfloat16, false>);
+    prefer_max_shared(tq_combine_group_kernel<float, true>);
+    prefer_max_shared(tq_combine_group_kernel<__half, true>);
+    prefer_max_shared(tq_combine_group_kernel<__nv_bfloat16, true>);
     prefer_max_shared(tq_step_prologue_kernel<float, true>);
     prefer_max_shared(tq_step_prologue_kernel<float, false>);
     prefer_max_shared(tq_step_prologue_kernel<__half, true>);
@@ -590,25 +665,37 @@ int32_t tq_launch_qprep_frag(tq_ctx *ctx, const void *q, int32_t q_dtype, int64_
     return TQ_OK;
 }
 
+template <typename T>
+static cudaError_t launch_combine(const CombineArgs &a, dim3 grid, cudaStream_t stream, bool programmatic) {
+    if (a.n_tail == 0)
+        return tq_launch_kernel(tq_combine_group_kernel<T, false>, grid, dim3(4 * TQ_D), 0, stream, programmatic, a);
+    return tq_launch_kernel(tq_combine_group_kernel<T, true>, grid, dim3(4 * TQ_D), sizeof(TailShared), stream, programmatic, a);
+}
+
 int32_t tq_launch_combine(const CombineArgs &a, int32_t q_dtype, int64_t rows, cudaStream_t stream, bool programmatic) {
-    if (a.n_tail == 0 && a.G <= 8) {  // grouped variant: one block per four heads of a KV row
-        const dim3 grid((unsigned)(rows / a.G) * ((a.G + 3) / 4)), block(4 * TQ_D);
-        cudaError_t e;
-        if (q_dtype == TQ_DTYPE_F32) e = tq_launch_kernel(tq_combine_group_kernel<float>, grid, block, 0, stream, programmatic, a);
-        else if (q_dtype == TQ_DTYPE_F16) e = tq_launch_kernel(tq_combine_group_kernel<__half>, grid, block, 0, stream, programmatic, a);
-        else e = tq_launch_kernel(tq_combine_group_kernel<__nv_bfloat16>, grid, block, 0, stream, programmatic, a);
-        TQ_CUDA_CHECK(e);
-        return TQ_OK;
-    }
-    const size_t dyn = (size_t)a.n_tail * sizeof(float);
-    if (dyn > 40 * 1024) return TQ_ERR_UNSUPPORTED;
-    if (q_dtype == TQ_DTYPE_F32)
-        tq_combine_kernel<float><<<(unsigned)rows, TQ_D, dyn, stream>>>(a);
-    else if (q_dtype == TQ_DTYPE_F16)
-        tq_combine_kernel<__half><<<(unsigned)rows, TQ_D, dyn, stream>>>(a);
-    else
-        tq_combine_kernel<__nv_bfloat16><<<(unsigned)rows, TQ_D, dyn, stream>>>(a);
-    TQ_CUDA_CHECK(cudaGetLastError());
+    configure_small_kernels();
+    if (a.G > 8) return TQ_ERR_UNSUPPORTED;
+    const dim3 grid((unsigned)(rows / a.G) * ((a.G + 3) / 4));  // one block per four heads of a KV row
+    cudaError_t e;
+    if (q_dtype == TQ_DTYPE_F32) e = launch_combine<float>(a, grid, stream, programmatic);
+    else if (q_dtype == TQ_DTYPE_F16) e = launch_combine<__half>(a, grid, stream, programmatic);
+    else e = launch_combine<__nv_bfloat16>(a, grid, stream, programmatic);
+    TQ_CUDA_CHECK(e);
+    return TQ_OK;
+}
+
+// The tail fields of the combine arguments: `tail_vec` when every row of both tensors starts on a 16-byte boundary.
+int32_t tq_set_combine_tail(CombineArgs &c, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tail, int32_t q_dtype) {
+    c.n_tail = n_tail, c.tail_k = c.tail_v = nullptr, c.tail_vec = false;
+    c.tk_sb = c.tk_sh = c.tk_st = c.tv_sb = c.tv_sh = c.tv_st = 0;
+    if (n_tail == 0) return TQ_OK;
+    if (k->dtype != q_dtype || v->dtype != q_dtype) return TQ_ERR_ARG;
+    c.tail_k = k->data, c.tail_v = v->data;
+    c.tk_sb = k->stride_b, c.tk_sh = k->stride_h, c.tk_st = k->stride_t;
+    c.tv_sb = v->stride_b, c.tv_sh = v->stride_h, c.tv_st = v->stride_t;
+    const int64_t strides = c.tk_sb | c.tk_sh | c.tk_st | c.tv_sb | c.tv_sh | c.tv_st;
+    const int64_t elem = q_dtype == TQ_DTYPE_F32 ? 4 : 2;
+    c.tail_vec = !((strides * elem | (int64_t)(uintptr_t)k->data | (int64_t)(uintptr_t)v->data) & 15);
     return TQ_OK;
 }
 
@@ -704,15 +791,7 @@ int32_t tq_launch_decode_exact(tq_ctx *ctx, const void *q, int32_t q_dtype, int3
     c.gather_world = 0, c.parts = 0, c.part = 0, c.head_group = 0, c.exch_rows = 0;
     c.rot_v = ctx->rot_v;
     c.q = q, c.out = out, c.out_f32 = nullptr;
-    c.n_tail = n_tail;
-    c.tail_k = n_tail ? tail_k->data : nullptr;
-    c.tail_v = n_tail ? tail_v->data : nullptr;
-    if (n_tail) {
-        if (tail_k->dtype != q_dtype || tail_v->dtype != q_dtype) return TQ_ERR_ARG;
-        c.tk_sb = tail_k->stride_b, c.tk_sh = tail_k->stride_h, c.tk_st = tail_k->stride_t;
-        c.tv_sb = tail_v->stride_b, c.tv_sh = tail_v->stride_h, c.tv_st = tail_v->stride_t;
-    } else {
-        c.tk_sb = c.tk_sh = c.tk_st = c.tv_sb = c.tv_sh = c.tv_st = 0;
-    }
+    rc = tq_set_combine_tail(c, tail_k, tail_v, n_tail, q_dtype);
+    if (rc) return rc;
     return tq_launch_combine(c, q_dtype, rows, stream);
 }

@@ -33,7 +33,7 @@
 //           tokens are interleaved with bit-selects so one look-up yields the (token a,
 //           token b) f16x2 that the MMA wants along its K axis.
 // Softmax is online, base 2, in registers; P*|v| goes to f16 and is transposed with
-// movmatrix.  Per-CTA partials (max, sum, acc) go to the workspace; tq_combine_kernel
+// movmatrix.  Per-CTA partials (max, sum, acc) go to the workspace; tq_combine_group_kernel
 // merges splits, un-rotates and casts.
 #include <math.h>
 
@@ -759,15 +759,7 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
     c.rot_v = ctx->rot_v;
     c.q = q, c.out = out, c.out_f32 = extras ? extras->out_f32 : nullptr;
     if (c.out_f32 && (gather || n_tail)) return TQ_ERR_UNSUPPORTED;
-    c.n_tail = n_tail;
-    c.tail_k = n_tail ? tail_k->data : nullptr;
-    c.tail_v = n_tail ? tail_v->data : nullptr;
-    if (n_tail) {
-        if (tail_k->dtype != q_dtype || tail_v->dtype != q_dtype) return TQ_ERR_ARG;
-        c.tk_sb = tail_k->stride_b, c.tk_sh = tail_k->stride_h, c.tk_st = tail_k->stride_t;
-        c.tv_sb = tail_v->stride_b, c.tv_sh = tail_v->stride_h, c.tv_st = tail_v->stride_t;
-    } else {
-        c.tk_sb = c.tk_sh = c.tk_st = c.tv_sb = c.tv_sh = c.tv_st = 0;
-    }
+    rc = tq_set_combine_tail(c, tail_k, tail_v, n_tail, q_dtype);
+    if (rc) return rc;
     return tq_launch_combine(c, q_dtype, rows, stream, /*programmatic=*/true);
 }
