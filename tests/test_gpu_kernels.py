@@ -104,3 +104,17 @@ def test_split_merge(setup_golden, dtype, splits):
     q = query((1, 5, 1), 3, dtype)
     assert rel_inf(store.decode_attn(q, splits=splits), attend64(store, p, q, 5)) <= ATTN_TOL[dtype]
 
+
+@pytest.mark.parametrize("bits,qjl", [(2, False), (3, False), (4, False), (2, True), (3, True), (4, True)])
+@pytest.mark.parametrize("groups", [1, 3, 4, 5, 8])
+@pytest.mark.parametrize("n", [1, 31, 33, 511, 513])
+def test_fp32_attention(setup_golden, bits, qjl, groups, n):
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(bits, qjl, setup_golden), make_codec(bits, qjl, setup_golden)
+    store = PackedStore(codec, 2, 2, capacity=n)
+    store.pack(vectors((2, 2, n, 128), 1, F32), vectors((2, 2, n, 128), 2, F32))
+    q = query((2, 2 * groups, 1), 3, F32)
+    want = attend64(store, p, q, groups)
+    assert rel_inf(store.decode_attn(q), want) <= 1e-5
+    assert rel_inf(store.decode_attn(q, splits=3), want) <= 1e-5

@@ -11,7 +11,7 @@
 
 namespace {
 
-constexpr int kExactWarps = 4;
+constexpr int kExactWarps = 16;
 
 struct ExactArgs {
     const uint8_t *k_codes;
@@ -36,29 +36,44 @@ template <int BITS> __device__ __forceinline__ uint32_t code_at(const uint32_t *
     return v & ((1u << BITS) - 1u);
 }
 
-template <int KB, int VB, bool QJL>
-__global__ void __launch_bounds__(kExactWarps * 32) tq_decode_exact_kernel(ExactArgs a) {
-    __shared__ float s_q[TQ_MAX_GROUPS][TQ_D];
-    __shared__ float s_qp[QJL ? TQ_MAX_GROUPS : 1][TQ_D];
-    __shared__ float s_ck[16], s_cv[16];
-    __shared__ float s_p[kExactWarps][TQ_MAX_GROUPS][32];
-    __shared__ float s_m[kExactWarps][TQ_MAX_GROUPS], s_l[kExactWarps][TQ_MAX_GROUPS];
-    __shared__ float s_acc[kExactWarps][TQ_MAX_GROUPS][TQ_D];
+// One warp attends 32 tokens at a time: first with a token per lane (all logits of its NG heads: a
+// centre look-up and NG multiply-adds per coordinate, the queries read as 16-byte broadcasts), then,
+// after the softmax, with four value coordinates per lane.  What bounds it is the chain of about 2000
+// instructions a warp runs per 32 tokens, so the work of a (split, KV row) is spread over 16 warps -
+// a whole 512-token split at once - and the value codes are requested before the logits are formed.
+// 1 x 8 x 4096 tokens, 4 heads each: 13 us; 53 us with four warps and value codes fetched token by token.
+template <int VB, int NG> struct ExactShared {
+    float q[NG][TQ_D];
+    float qp[NG][TQ_D];
+    float ck[16], cv[16];
+    float m[kExactWarps][NG], l[kExactWarps][NG];
+    float p[kExactWarps][32][NG];
+    union {
+        uint4 v[kExactWarps][32 * VB];  // the 32 tokens' value codes
+        float acc[kExactWarps][TQ_D];   // merge of the warps, one head at a time
+    };
+};
 
+template <int KB, int VB, bool QJL, int NG>
+__global__ void __launch_bounds__(kExactWarps * 32) tq_decode_exact_kernel(ExactArgs a) {
+    extern __shared__ __align__(16) uint8_t s_raw[];
+    ExactShared<VB, NG> &sm = *reinterpret_cast<ExactShared<VB, NG> *>(s_raw);
     const int split = blockIdx.x;
     const int bh = blockIdx.y;  // b * Hkv + h
     const int b = bh / a.Hkv, h = bh % a.Hkv;
-    const int G = a.G;
+    const int G = a.G;  // (> NG / 2 or NG == 4; heads >= G of the block attend a zero query)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t q_row0 = ((int64_t)b * a.Hkv + h) * G;  // first query head of this KV head
-
-    for (int i = threadIdx.x; i < G * TQ_D; i += blockDim.x) {
-        s_q[i / TQ_D][i % TQ_D] = a.qrot[q_row0 * TQ_D + i];
-        if (QJL) s_qp[i / TQ_D][i % TQ_D] = a.qproj[q_row0 * TQ_D + i];
-    }
     if (threadIdx.x < 16) {
-        s_ck[threadIdx.x] = a.centers_k[threadIdx.x];
-        s_cv[threadIdx.x] = a.centers_v[threadIdx.x];
+        sm.ck[threadIdx.x] = a.centers_k[threadIdx.x];
+        sm.cv[threadIdx.x] = a.centers_v[threadIdx.x];
+    }
+    tq_grid_dependency_wait();
+    tq_launch_dependents();
+    for (int i = threadIdx.x; i < NG * TQ_D; i += blockDim.x) {
+        const bool live = i < G * TQ_D;
+        (&sm.q[0][0])[i] = live ? a.qrot[q_row0 * TQ_D + i] : 0.f;
+        if (QJL) (&sm.qp[0][0])[i] = live ? a.qproj[q_row0 * TQ_D + i] : 0.f;
     }
     __syncthreads();
 
@@ -71,9 +86,9 @@ __global__ void __launch_bounds__(kExactWarps * 32) tq_decode_exact_kernel(Exact
     const float hs = 0.08838834764831845f;                    // 1/sqrt(128)
     const float qjl_scale = 1.2533141373155003f / (float)TQ_D;  // sqrt(pi/2)/D
 
-    float m[TQ_MAX_GROUPS], l[TQ_MAX_GROUPS], acc[TQ_MAX_GROUPS][4];
+    float m[NG], l[NG], acc[NG][4];
 #pragma unroll
-    for (int g = 0; g < TQ_MAX_GROUPS; ++g) {
+    for (int g = 0; g < NG; ++g) {
         m[g] = -INFINITY;
         l[g] = 0.f;
         acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0.f;
@@ -84,7 +99,8 @@ __global__ void __launch_bounds__(kExactWarps * 32) tq_decode_exact_kernel(Exact
         const int tok = base + lane;
         const bool valid = tok < a.N && tok >= t_lo;
         const int64_t row = row0 + (tok < a.N ? tok : base);
-        // ---- phase A: one token per lane, all G logits
+        const int n_here = min(32, a.N - base);
+        // ---- phase A: one token per lane, all logits
         uint32_t kw[4 * KB + 1];
         {
             const uint4 *src = (const uint4 *)(a.k_codes + row * (16 * KB));
@@ -95,58 +111,74 @@ __global__ void __launch_bounds__(kExactWarps * 32) tq_decode_exact_kernel(Exact
             }
             kw[4 * KB] = 0;
         }
-        float dot[TQ_MAX_GROUPS];
+        uint4 sw4 = make_uint4(0, 0, 0, 0);
+        float rn = 0.f;
+        if (QJL) sw4 = __ldg((const uint4 *)(a.k_signs + row * 16)), rn = tq_half_bits_to_float(a.k_rnorms[row]);
+        const float kn = tq_half_bits_to_float(a.k_norms[row]), vn = tq_half_bits_to_float(a.v_norms[row]);
+        uint4 vw[VB];  // the chunk's value codes are one contiguous piece of the row
 #pragma unroll
-        for (int g = 0; g < TQ_MAX_GROUPS; ++g) dot[g] = 0.f;
-#pragma unroll
-        for (int j = 0; j < TQ_D; ++j) {
-            const float cv = s_ck[code_at<KB>(kw, j)];
-#pragma unroll
-            for (int g = 0; g < TQ_MAX_GROUPS; ++g)
-                if (g < G) dot[g] = fmaf(cv, s_q[g][j], dot[g]);
+        for (int i = 0; i < VB; ++i) {
+            vw[i] = make_uint4(0, 0, 0, 0);
+            if (32 * i + lane < n_here * VB) vw[i] = __ldg((const uint4 *)(a.v_codes + (row0 + base) * (16 * VB)) + 32 * i + lane);
         }
-        const float kn = tq_half_bits_to_float(a.k_norms[row]);
-        float logit[TQ_MAX_GROUPS];
+        float dot[NG];
 #pragma unroll
-        for (int g = 0; g < TQ_MAX_GROUPS; ++g) logit[g] = dot[g] * kn * hs;
-        if (QJL) {
-            const uint4 sw4 = __ldg((const uint4 *)(a.k_signs + row * 16));
-            const uint32_t sw[4] = {sw4.x, sw4.y, sw4.z, sw4.w};
-            float dq[TQ_MAX_GROUPS];
+        for (int g = 0; g < NG; ++g) dot[g] = 0.f;
 #pragma unroll
-            for (int g = 0; g < TQ_MAX_GROUPS; ++g) dq[g] = 0.f;
+        for (int j = 0; j < TQ_D; j += 4) {
+            float cv[4];
 #pragma unroll
-            for (int j = 0; j < TQ_D; ++j) {
-                const float sg = ((sw[j >> 5] >> (j & 31)) & 1u) ? 1.0f : -1.0f;
+            for (int i = 0; i < 4; ++i) cv[i] = sm.ck[code_at<KB>(kw, j + i)];
 #pragma unroll
-                for (int g = 0; g < TQ_MAX_GROUPS; ++g)
-                    if (g < G) dq[g] = fmaf(sg, s_qp[g][j], dq[g]);
+            for (int g = 0; g < NG; ++g) {
+                const float4 q4 = *reinterpret_cast<const float4 *>(&sm.q[g][j]);
+                dot[g] = fmaf(cv[0], q4.x, dot[g]), dot[g] = fmaf(cv[1], q4.y, dot[g]);
+                dot[g] = fmaf(cv[2], q4.z, dot[g]), dot[g] = fmaf(cv[3], q4.w, dot[g]);
             }
-            const float rn = tq_half_bits_to_float(a.k_rnorms[row]);
+        }
+        float logit[NG];
 #pragma unroll
-            for (int g = 0; g < TQ_MAX_GROUPS; ++g) logit[g] += qjl_scale * rn * dq[g] * hs;
+        for (int g = 0; g < NG; ++g) logit[g] = dot[g] * kn * hs;
+        if (QJL) {
+            const uint32_t sw[4] = {sw4.x, sw4.y, sw4.z, sw4.w};
+            float dq[NG];
+#pragma unroll
+            for (int g = 0; g < NG; ++g) dq[g] = 0.f;
+#pragma unroll
+            for (int j = 0; j < TQ_D; j += 4) {
+                float sg[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sg[i] = ((sw[j >> 5] >> ((j + i) & 31)) & 1u) ? 1.0f : -1.0f;
+#pragma unroll
+                for (int g = 0; g < NG; ++g) {
+                    const float4 q4 = *reinterpret_cast<const float4 *>(&sm.qp[g][j]);
+                    dq[g] = fmaf(sg[0], q4.x, dq[g]), dq[g] = fmaf(sg[1], q4.y, dq[g]);
+                    dq[g] = fmaf(sg[2], q4.z, dq[g]), dq[g] = fmaf(sg[3], q4.w, dq[g]);
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < NG; ++g) logit[g] += qjl_scale * rn * dq[g] * hs;
         }
         // ---- phase B: online softmax over the 32 tokens of the chunk
-        const float vn = tq_half_bits_to_float(a.v_norms[row]);
         __syncwarp();
 #pragma unroll
-        for (int g = 0; g < TQ_MAX_GROUPS; ++g) {
-            if (g < G) {
-                const float lg = valid ? logit[g] : -INFINITY;
-                const float nm = fmaxf(m[g], tq_warp_max(lg));
-                const float corr = (m[g] == -INFINITY) ? 0.f : expf(m[g] - nm);
-                const float p = valid ? expf(lg - nm) : 0.f;
-                l[g] = l[g] * corr + tq_warp_sum(p);
-                acc[g][0] *= corr, acc[g][1] *= corr, acc[g][2] *= corr, acc[g][3] *= corr;
-                m[g] = nm;
-                s_p[warp][g][lane] = p * vn;
-            }
+        for (int i = 0; i < VB; ++i) sm.v[warp][32 * i + lane] = vw[i];
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            const float lg = valid ? logit[g] : -INFINITY;
+            const float nm = fmaxf(m[g], tq_warp_max(lg));
+            const float corr = (m[g] == -INFINITY) ? 0.f : expf(m[g] - nm);
+            const float p = valid ? expf(lg - nm) : 0.f;
+            l[g] = l[g] * corr + tq_warp_sum(p);
+            acc[g][0] *= corr, acc[g][1] *= corr, acc[g][2] *= corr, acc[g][3] *= corr;
+            m[g] = nm;
+            sm.p[warp][lane][g] = valid ? p * vn : 0.f;  // (a masked token's norm may be stale and not finite)
         }
         __syncwarp();
         // ---- phase C: lane owns value dims 4*lane..4*lane+3
-        const int n_here = min(32, a.N - base);
+#pragma unroll 4
         for (int t = 0; t < n_here; ++t) {
-            const uint8_t *vr = a.v_codes + (row0 + base + t) * (16 * VB);
+            const uint8_t *vr = reinterpret_cast<const uint8_t *>(&sm.v[warp][0]) + t * (16 * VB);
             uint32_t v;
             if (VB == 2) {
                 v = vr[lane];
@@ -158,43 +190,63 @@ __global__ void __launch_bounds__(kExactWarps * 32) tq_decode_exact_kernel(Exact
             }
             float cv[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) cv[i] = s_cv[(v >> (VB * i)) & ((1u << VB) - 1u)];
+            for (int i = 0; i < 4; ++i) cv[i] = sm.cv[(v >> (VB * i)) & ((1u << VB) - 1u)];
 #pragma unroll
-            for (int g = 0; g < TQ_MAX_GROUPS; ++g) {
-                if (g < G) {
-                    const float w = s_p[warp][g][t];
+            for (int g = 0; g < NG; g += 4) {
+                const float4 w = *reinterpret_cast<const float4 *>(&sm.p[warp][t][g]);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[g][i] = fmaf(w, cv[i], acc[g][i]);
+                for (int i = 0; i < 4; ++i) {
+                    acc[g][i] = fmaf(w.x, cv[i], acc[g][i]), acc[g + 1][i] = fmaf(w.y, cv[i], acc[g + 1][i]);
+                    acc[g + 2][i] = fmaf(w.z, cv[i], acc[g + 2][i]), acc[g + 3][i] = fmaf(w.w, cv[i], acc[g + 3][i]);
                 }
             }
         }
         __syncwarp();
     }
 
-    // ---- merge the warps of this CTA and write the split partial
+    // ---- merge the warps of this CTA, one head at a time, and write the split partial
 #pragma unroll
-    for (int g = 0; g < TQ_MAX_GROUPS; ++g) {
-        if (g < G) {
-            if (lane == 0) s_m[warp][g] = m[g], s_l[warp][g] = l[g];
+    for (int g = 0; g < NG; ++g)
+        if (lane == 0) sm.m[warp][g] = m[g], sm.l[warp][g] = l[g];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s_acc[warp][g][4 * lane + i] = acc[g][i];
+    for (int g = 0; g < NG; ++g) {
+        if (g >= G) break;
+        __syncthreads();  // (the value codes, then the previous head's accumulators, are done with)
+        *reinterpret_cast<float4 *>(&sm.acc[warp][4 * lane]) = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+        __syncthreads();
+        const int d = threadIdx.x;
+        if (d < TQ_D) {
+            float M = -INFINITY;
+            for (int w = 0; w < kExactWarps; ++w) M = fmaxf(M, sm.m[w][g]);
+            float L = 0.f, A = 0.f;
+            for (int w = 0; w < kExactWarps; ++w) {
+                const float sc = (sm.m[w][g] == -INFINITY) ? 0.f : expf(sm.m[w][g] - M);
+                L += sm.l[w][g] * sc;
+                A += sm.acc[w][d] * sc;
+            }
+            const int64_t prow = (q_row0 + g) * a.n_splits + split;
+            a.part_acc[prow * TQ_D + d] = A;
+            if (d == 0) a.part_m[prow] = M, a.part_l[prow] = L;
         }
     }
-    __syncthreads();
-    const int d = threadIdx.x;  // 128 threads == 128 dims
-    for (int g = 0; g < G; ++g) {
-        float M = -INFINITY;
-        for (int w = 0; w < kExactWarps; ++w) M = fmaxf(M, s_m[w][g]);
-        float L = 0.f, A = 0.f;
-        for (int w = 0; w < kExactWarps; ++w) {
-            const float sc = (s_m[w][g] == -INFINITY) ? 0.f : expf(s_m[w][g] - M);
-            L += s_l[w][g] * sc;
-            A += s_acc[w][g][d] * sc;
-        }
-        const int64_t prow = (q_row0 + g) * a.n_splits + split;
-        a.part_acc[prow * TQ_D + d] = A;
-        if (d == 0) a.part_m[prow] = M, a.part_l[prow] = L;
+}
+
+template <int KB, int VB, bool QJL, int NG>
+cudaError_t launch_exact_variant(const ExactArgs &a, int device, dim3 grid, cudaStream_t stream) {
+    const size_t smem = sizeof(ExactShared<VB, NG>);
+    // the attribute belongs to the (kernel, device) pair: one flag per device of this instantiation
+    static bool configured[TQ_MAX_DEVICES] = {};
+    if (device < 0 || device >= TQ_MAX_DEVICES) return cudaErrorInvalidDevice;
+    if (!configured[device]) {
+        cudaError_t e = cudaFuncSetAttribute(tq_decode_exact_kernel<KB, VB, QJL, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        configured[device] = true;
     }
+    return tq_launch_kernel(tq_decode_exact_kernel<KB, VB, QJL, NG>, grid, dim3(kExactWarps * 32), smem, stream, true, a);
+}
+template <int KB, int VB, bool QJL> cudaError_t launch_exact(const ExactArgs &a, int device, dim3 grid, cudaStream_t stream) {
+    return a.G > 4 ? launch_exact_variant<KB, VB, QJL, 8>(a, device, grid, stream)
+                   : launch_exact_variant<KB, VB, QJL, 4>(a, device, grid, stream);
 }
 
 }  // namespace
@@ -203,23 +255,34 @@ __global__ void __launch_bounds__(kExactWarps * 32) tq_decode_exact_kernel(Exact
 // Shared pieces: query preparation and split combine
 // ---------------------------------------------------------------------------
 
+// Rotated (first half of the grid) and projected (second half, with a QJL sketch) queries as plain
+// rows, four rows per block: a thread's 32 matrix elements come in one batch of loads.  One row per
+// block and a chain of loads over the 128 matrix rows took 4.8 us for 32 rows, this takes 2.4.
 template <typename T>
-__global__ void __launch_bounds__(TQ_D) tq_qprep_kernel(const T *q, const float *rot_k_t, const float *qjl_t,
-                                                       float *qrot, float *qproj, int use_qjl) {
-    __shared__ float s_q[TQ_D];
-    const int64_t row = blockIdx.x;
-    const int j = threadIdx.x;
-    s_q[j] = tq_to_float<T>(q[row * TQ_D + j]);
+__global__ void __launch_bounds__(4 * TQ_D, 2) tq_qprep_kernel(const T *q, const float *rot_k_t, const float *qjl_t,
+                                                              float *qrot, float *qproj, int64_t rows) {
+    __shared__ float s_q[4][TQ_D], s_part[4][4][TQ_D];
+    const int64_t groups = (rows + 3) / 4;
+    const bool proj = blockIdx.x >= groups;
+    const int64_t row0 = 4 * (proj ? blockIdx.x - groups : blockIdx.x);
+    const int tid = threadIdx.x, j = tid & (TQ_D - 1), dq = tid >> 7;
+    float m[32];
+    tq_load_column(m, proj ? qjl_t : rot_k_t, dq, j);  // (codec constants: fetched before the wait)
+    tq_grid_dependency_wait();
+    tq_launch_dependents();
+    s_q[dq][j] = row0 + dq < rows ? tq_to_float<T>(q[(row0 + dq) * TQ_D + j]) : 0.f;
     __syncthreads();
-    float r = 0.f, p = 0.f;
-#pragma unroll 8
-    for (int d = 0; d < TQ_D; ++d) r = fmaf(s_q[d], __ldg(rot_k_t + d * TQ_D + j), r);
-    qrot[row * TQ_D + j] = r;
-    if (use_qjl) {
-#pragma unroll 8
-        for (int d = 0; d < TQ_D; ++d) p = fmaf(s_q[d], __ldg(qjl_t + d * TQ_D + j), p);
-        qproj[row * TQ_D + j] = p;
-    }
+    float r[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+#pragma unroll
+        for (int g = 0; g < 4; ++g) r[g] = fmaf(s_q[g][32 * dq + i], m[i], r[g]);
+#pragma unroll
+    for (int g = 0; g < 4; ++g) s_part[dq][g][j] = r[g];
+    __syncthreads();
+    if (row0 + dq < rows)
+        (proj ? qproj : qrot)[(row0 + dq) * TQ_D + j] =
+            (s_part[0][dq][j] + s_part[1][dq][j]) + (s_part[2][dq][j] + s_part[3][dq][j]);
 }
 
 // Query preparation for the tensor-core kernel (see tq_qprep_block): kv_rows * ceil(G / 4) blocks
@@ -241,9 +304,6 @@ __global__ void __launch_bounds__(4 * TQ_D, 2) tq_step_prologue_kernel(TqQprepAr
         tq_pack_small_block<T, QJL>(pa, (int64_t)blockIdx.x - n_qprep);
 }
 
-// Split combine for up to four heads of one (batch, KV head) row per block: the un-rotation
-// matrix is read once for the G heads, and the un-quantised tail of the row, if there is one
-// (TAIL), is attended by the same block.
 // Publishing rows to the peers and waiting for theirs (system scope, PTX memory model):
 // a block's threads store their rows with plain stores, the block barrier orders those stores
 // before thread 0, which adds the block's row count to the flag word with a RELEASE reduction at
@@ -389,6 +449,9 @@ __device__ __forceinline__ float tq_attend_tail(const CombineArgs &a, TailShared
     return o;
 }
 
+// Split combine for up to four heads of one (batch, KV head) row per block: the un-rotation
+// matrix is read once for the G heads, and the un-quantised tail of the row, if there is one
+// (TAIL), is attended by the same block.
 template <typename T, bool TAIL>
 __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs a) {
     __shared__ __align__(16) float s_o[4][TQ_D];
@@ -622,19 +685,21 @@ static void configure_small_kernels() {
     prefer_max_shared(tq_step_prologue_kernel<__nv_bfloat16, false>);
 }
 
+template <typename T>
+static cudaError_t launch_qprep(tq_ctx *ctx, const void *q, int64_t rows, float *qrot, float *qproj, cudaStream_t stream) {
+    const unsigned grid = (unsigned)((rows + 3) / 4) * (ctx->use_qjl ? 2 : 1);
+    return tq_launch_kernel(tq_qprep_kernel<T>, dim3(grid), dim3(4 * TQ_D), 0, stream, true, (const T *)q, ctx->rot_k_t,
+                            ctx->qjl_t, qrot, qproj, rows);
+}
+
 int32_t tq_launch_qprep(tq_ctx *ctx, const void *q, int32_t q_dtype, int64_t rows, float *qrot, float *qproj,
                         cudaStream_t stream) {
     configure_small_kernels();
-    if (q_dtype == TQ_DTYPE_F32)
-        tq_qprep_kernel<float><<<(unsigned)rows, TQ_D, 0, stream>>>((const float *)q, ctx->rot_k_t, ctx->qjl_t, qrot,
-                                                                    qproj, ctx->use_qjl);
-    else if (q_dtype == TQ_DTYPE_F16)
-        tq_qprep_kernel<__half><<<(unsigned)rows, TQ_D, 0, stream>>>((const __half *)q, ctx->rot_k_t, ctx->qjl_t,
-                                                                     qrot, qproj, ctx->use_qjl);
-    else
-        tq_qprep_kernel<__nv_bfloat16><<<(unsigned)rows, TQ_D, 0, stream>>>((const __nv_bfloat16 *)q, ctx->rot_k_t,
-                                                                            ctx->qjl_t, qrot, qproj, ctx->use_qjl);
-    TQ_CUDA_CHECK(cudaGetLastError());
+    cudaError_t e;
+    if (q_dtype == TQ_DTYPE_F32) e = launch_qprep<float>(ctx, q, rows, qrot, qproj, stream);
+    else if (q_dtype == TQ_DTYPE_F16) e = launch_qprep<__half>(ctx, q, rows, qrot, qproj, stream);
+    else e = launch_qprep<__nv_bfloat16>(ctx, q, rows, qrot, qproj, stream);
+    TQ_CUDA_CHECK(e);
     return TQ_OK;
 }
 
@@ -767,21 +832,21 @@ int32_t tq_launch_decode_exact(tq_ctx *ctx, const void *q, int32_t q_dtype, int3
     a.part_m = w.part_m, a.part_l = w.part_l, a.part_acc = w.part_acc;
     a.centers_k = ctx->centers_k, a.centers_v = ctx->centers_v;
     dim3 grid(n_splits, cache->batch * cache->kv_heads);
-    const int threads = kExactWarps * 32;
     const int mode = ctx->use_qjl * 10 + ctx->bits;
     tq_prof_count(ctx, 3);
     tq_prof_begin(ctx, stream);
+    cudaError_t e;
     switch (mode) {
-        case 2: tq_decode_exact_kernel<2, 2, false><<<grid, threads, 0, stream>>>(a); break;
-        case 3: tq_decode_exact_kernel<3, 3, false><<<grid, threads, 0, stream>>>(a); break;
-        case 4: tq_decode_exact_kernel<4, 4, false><<<grid, threads, 0, stream>>>(a); break;
-        case 12: tq_decode_exact_kernel<1, 2, true><<<grid, threads, 0, stream>>>(a); break;
-        case 13: tq_decode_exact_kernel<2, 3, true><<<grid, threads, 0, stream>>>(a); break;
-        case 14: tq_decode_exact_kernel<3, 4, true><<<grid, threads, 0, stream>>>(a); break;
+        case 2: e = launch_exact<2, 2, false>(a, ctx->device, grid, stream); break;
+        case 3: e = launch_exact<3, 3, false>(a, ctx->device, grid, stream); break;
+        case 4: e = launch_exact<4, 4, false>(a, ctx->device, grid, stream); break;
+        case 12: e = launch_exact<1, 2, true>(a, ctx->device, grid, stream); break;
+        case 13: e = launch_exact<2, 3, true>(a, ctx->device, grid, stream); break;
+        case 14: e = launch_exact<3, 4, true>(a, ctx->device, grid, stream); break;
         default: return TQ_ERR_UNSUPPORTED;
     }
     tq_prof_end(ctx, stream);
-    TQ_CUDA_CHECK(cudaGetLastError());
+    TQ_CUDA_CHECK(e);
 
     CombineArgs c;
     c.part_m = w.part_m, c.part_l = w.part_l, c.part_acc = w.part_acc;
@@ -793,5 +858,5 @@ int32_t tq_launch_decode_exact(tq_ctx *ctx, const void *q, int32_t q_dtype, int3
     c.q = q, c.out = out, c.out_f32 = nullptr;
     rc = tq_set_combine_tail(c, tail_k, tail_v, n_tail, q_dtype);
     if (rc) return rc;
-    return tq_launch_combine(c, q_dtype, rows, stream);
+    return tq_launch_combine(c, q_dtype, rows, stream, /*programmatic=*/true);
 }
