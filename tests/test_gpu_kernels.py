@@ -118,3 +118,103 @@ def test_fp32_attention(setup_golden, bits, qjl, groups, n):
     want = attend64(store, p, q, groups)
     assert rel_inf(store.decode_attn(q), want) <= 1e-5
     assert rel_inf(store.decode_attn(q, splits=3), want) <= 1e-5
+
+
+MODES = [(2, False), (3, False), (4, False), (2, True), (3, True), (4, True)]
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("bits,qjl", MODES)
+@pytest.mark.parametrize("shape", [(1, 1, 1024), (1, 8, 129), (3, 5, 127)])
+def test_prefill_encoder(setup_golden, bits, qjl, dtype, shape):
+    """The tcgen05 encoder from its smallest size on: whole tiles, one vector over, one vector short."""
+    from helpers import check_packed
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(bits, qjl, setup_golden), make_codec(bits, qjl, setup_golden)
+    k, v = vectors((*shape, 128), 1, dtype, "cpu"), vectors((*shape, 128), 2, dtype, "cpu")
+    k[:, :, 5] = 0
+    store = PackedStore(codec, shape[0], shape[1], capacity=shape[2] + 9)
+    store.pack(k.cuda(), v.cuda())
+    assert codec.device_status() == 0
+    check_packed(store, O.pack_layer(k, v, p), k, v, p, f"{bits} {qjl} {dtype} {shape}")
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("qjl", [False, True])
+def test_prefill_encoder_extreme_rows(setup_golden, dtype, qjl):
+    """Rows whose norm underflows, overflows or is undefined: what the CUDA-core encoder gives (which takes the same
+    rows when they are not 16-byte aligned)."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec = make_codec(4, qjl, setup_golden)
+    k, v = vectors((1, 2, 1100, 128), 1, dtype), vectors((1, 2, 1100, 128), 2, dtype)
+    for x in (k, v):
+        x[:, :, 3] *= 1e-5 if dtype == F16 else 1e-30  # squares vanish (fp16: a norm that is subnormal in fp16)
+        x[:, :, 4] = 0
+        if dtype != F16:
+            x[:, :, 10] *= 1e18
+            x[:, :, 11] *= 1e22  # squares overflow
+        x[:, :, 12, 7] = float("inf")
+        x[:, :, 13, 100] = float("nan")
+        x[:, :, 14, 1] = -float("inf")
+    fast, exact = PackedStore(codec, 1, 2, 1100), PackedStore(codec, 1, 2, 1100)
+    fast.pack(k, v)
+    exact.pack(off_by_one(k), off_by_one(v))
+    rows = [3, 4, 10, 11, 12, 13, 14]
+    for name, a, b in zip(("k", "kn", "ks", "kr", "v", "vn") if qjl else ("k", "kn", "v", "vn"), fast.streams(), exact.streams()):
+        a, b = a[:, :, rows], b[:, :, rows]
+        if a.dtype == torch.float16:  # one ulp, as between any two orders of summation; undefined where undefined
+            assert torch.equal(a.isnan(), b.isnan()), name
+            a, b = a.nan_to_num(), b.nan_to_num()
+            assert (a.view(torch.int16).int() - b.view(torch.int16).int()).abs().max() <= 1, name
+        else:
+            assert torch.equal(a, b), name
+
+
+@pytest.mark.parametrize("form", ["transposed", "keys unaligned", "both unaligned"])
+def test_prefill_encoder_operand_forms(setup_golden, form):
+    """Strides and alignments the kernel takes or hands on: the same codes as from contiguous tensors, outside the 1e-6
+    band where the two encoders may differ."""
+    from helpers import check_packed
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(4, True, setup_golden), make_codec(4, True, setup_golden)
+    k, v = vectors((2, 3, 200, 128), 1, BF16, "cpu"), vectors((2, 3, 200, 128), 2, BF16, "cpu")
+    kd, vd = k.cuda(), v.cuda()
+    if form == "transposed":
+        kd, vd = (x.transpose(1, 2).contiguous().transpose(1, 2) for x in (kd, vd))
+    else:
+        kd = off_by_one(kd)
+        vd = off_by_one(vd) if form == "both unaligned" else vd
+    store = PackedStore(codec, 2, 3, capacity=216)
+    store.pack(vectors((2, 3, 3, 128), 3, BF16), vectors((2, 3, 3, 128), 4, BF16))  # (an odd position to append at)
+    store.pack(kd, vd)
+    view = PackedStore(codec, 2, 3, capacity=200)
+    for a, b in zip(view.streams(), store.streams()):
+        a[:, :, :200] = b[:, :, 3:203]
+    view.length = 200
+    check_packed(view, O.pack_layer(k, v, p), k, v, p, form)
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("bits,qjl", MODES)
+@pytest.mark.parametrize("shape", [(1, 1, 1024), (1, 8, 129), (3, 5, 127)])
+def test_dequantisation(setup_golden, bits, qjl, dtype, shape):
+    """The tcgen05 dequantisation from its smallest size on, and the CUDA-core one below it (a slice of few tokens)."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(bits, qjl, setup_golden), make_codec(bits, qjl, setup_golden)
+    store = PackedStore(codec, shape[0], shape[1], capacity=shape[2] + 9)
+    store.pack(vectors((*shape, 128), 1, dtype), vectors((*shape, 128), 2, dtype))
+    layer = store_to_layer(store, p, torch.float32)
+    # fp32 sums of 128 products against the oracle's, relative to the largest element; a 16-bit result may in addition
+    # be a neighbour of the oracle's, and a key's two rounded parts one each
+    ulp = {F32: 0.0, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
+    for which, want in (("keys", O.dequant_keys(layer)), ("values", O.dequant_values(layer))):
+        for lo in (0, shape[2] - 3):
+            got = store.dequant(which, lo, dtype=dtype).cpu().float()
+            ref = want[:, :, lo:]
+            room = 2e-6 * ref.abs().max() + ulp * (ref.abs() + 0.5 * ref.abs().amax(dim=-1, keepdim=True) * (which == "keys" and qjl))
+            assert ((got - ref).abs() <= room).all(), (which, lo, float((got - ref).abs().max()))
+    assert codec.device_status() == 0

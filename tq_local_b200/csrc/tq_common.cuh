@@ -30,12 +30,20 @@ struct tq_ctx {
     float *bounds_k;   // [16] (padded with +inf)
     float *centers_v;
     float *bounds_v;
-    // Shared-memory images for the tensor-core encoder: each [128][128] K-major operand split
-    // into three bf16 terms, two 64-wide slabs per term, 128-byte swizzle (96 KB per matrix).
-    uint16_t *img_rot_k;   // rows j, k = d:  R_k[j][d]      (B operand of u @ R_k^T)
-    uint16_t *img_rot_v;
-    uint16_t *img_rot_kt;  // rows d, k = j:  R_k[j][d]      (B operand of c @ R_k)
-    uint16_t *img_qjl;     // rows i, k = d:  S[i][d]        (B operand of r @ S^T)
+    // Shared-memory images of the tcgen05 kernels' B operands (64 KB each, see tq_build_operand_image): rows n and
+    // contraction index k of the [128][128] matrix behind vec[k] -> out[n], in two f16 terms, times a power of two.
+    struct Image {
+        uint16_t *data;
+        float unscale;  // what undoes the power of two
+    };
+    Image img_rot_k;    // n = j, k = d:  R_k[j][d]   u @ R_k^T
+    Image img_rot_v;
+    Image img_rot_kt;   // n = d, k = j:  R_k[j][d]   c @ R_k
+    Image img_rot_vt;
+    Image img_qjl;      // n = i, k = d:  S[i][d]     r @ S^T
+    Image img_qjl_t;    // n = d, k = i:  S[i][d]     signs @ S
+    float cen_k_scale, cen_v_scale;  // powers of two that bring the largest centre just below 2^14
+    float res_scale;    // power of two <= 1 that keeps a unit vector's scaled residual inside f16 whatever the centres
     void *base;       // one allocation holding everything above
     size_t base_bytes;
     struct tq_prof *prof;  // measurement hooks, see tq_profile_enable
@@ -145,8 +153,13 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
                               const tq_cache_desc *cache, int32_t seq_len, const tq_dense_desc *tail_k,
                               const tq_dense_desc *tail_v, int32_t n_tail, int32_t n_splits,
                               void *workspace, void *out, const TqStepExtras *extras, cudaStream_t stream);
-void tq_build_operand_image(const float *m, uint16_t *image);
-int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *x, int which, int32_t n_tokens,
+float tq_fit_power(float largest);  // the power of two that brings `largest` into [2^13, 2^14)
+float tq_build_operand_image(const float *m, uint16_t *image);
+// `k` null: values only.  TQ_ERR_UNSUPPORTED when a tensor's alignment rules the kernel out.
+int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tokens,
                           const tq_cache_desc *cache, int32_t pos0, cudaStream_t stream);
+// TQ_ERR_UNSUPPORTED when the output's alignment rules the kernel out.
+int32_t tq_launch_dequant_tc(tq_ctx *ctx, const tq_cache_desc *cache, int32_t which, int32_t pos0, int32_t n_tokens,
+                             const tq_dense_desc *out, cudaStream_t stream);
 int32_t tq_launch_dequant(tq_ctx *ctx, const tq_cache_desc *cache, int32_t which, int32_t pos0,
                           int32_t n_tokens, const tq_dense_desc *out, cudaStream_t stream);

@@ -383,8 +383,9 @@ int32_t tq_launch_pack(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc 
     a.first_kind = 0, a.n_kinds = 2;
     const int64_t n_vec = (int64_t)a.B * a.H * a.S;
     if (n_vec >= 1024) {
-        if (tq_launch_pack_tc(ctx, v, 1, n_tokens, cache, pos0, stream) == TQ_OK) a.n_kinds = 1;
-        if (a.n_kinds == 1 && tq_launch_pack_tc(ctx, k, 0, n_tokens, cache, pos0, stream) == TQ_OK) return TQ_OK;
+        const int32_t rc = tq_launch_pack_tc(ctx, k, v, n_tokens, cache, pos0, stream);
+        if (rc != TQ_ERR_UNSUPPORTED) return rc;
+        if (tq_launch_pack_tc(ctx, nullptr, v, n_tokens, cache, pos0, stream) == TQ_OK) a.n_kinds = 1;
     }
     const int64_t items = a.n_kinds * n_vec;
     if (n_vec < 1024) {  // appends: one block per vector
@@ -423,6 +424,10 @@ int32_t tq_launch_pack(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc 
 
 int32_t tq_launch_dequant(tq_ctx *ctx, const tq_cache_desc *cache, int32_t which, int32_t pos0,
                           int32_t n_tokens, const tq_dense_desc *out, cudaStream_t stream) {
+    if ((int64_t)cache->batch * cache->kv_heads * n_tokens >= 1024) {
+        const int32_t rc = tq_launch_dequant_tc(ctx, cache, which, pos0, n_tokens, out, stream);
+        if (rc != TQ_ERR_UNSUPPORTED) return rc;
+    }
     DequantArgs a;
     const bool key = which == 0;
     a.codes = key ? cache->k_codes : cache->v_codes;

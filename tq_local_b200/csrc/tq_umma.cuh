@@ -1,0 +1,152 @@
+// Helpers of the tcgen05 kernels (prefill encoder, dequantisation): mbarriers, bulk copies, matrix
+// descriptors, TMEM loads and stores, and the f16 operand images of the 128 x 128 matrices.
+//
+// Every contraction here is [128 vectors x 128] * M with fp32 accuracy on f16 tensor cores: an fp32
+// operand, scaled by a power of two so that its largest element is below 2^15, is split in two f16
+// terms hi + lo (22 bits, and an absolute floor of 2^-25), and the products hi*lo, lo*hi and hi*hi are
+// accumulated in fp32 in that order, so that the accumulator is small until the last eight steps.
+// The A operand (the vectors) lives in TMEM, the B operand (the matrix) in shared memory.
+#pragma once
+
+#include <cuda_fp16.h>
+#include <stdint.h>
+
+#include "tq_common.cuh"
+
+constexpr int kUmmaRows = 128;                         // vectors per tile: the rows of A and of the accumulator
+constexpr int kUmmaSlabBytes = 128 * 128;              // 128 rows x 64 f16 (one 128-byte swizzle row each): 16 KB
+constexpr int kUmmaTermBytes = 2 * kUmmaSlabBytes;     // one f16 term of a 128 x 128 matrix: 32 KB
+constexpr int kUmmaImageBytes = 2 * kUmmaTermBytes;    // hi and lo terms: 64 KB
+constexpr uint32_t kUmmaSpinLimit = 1u << 22;          // polls before a wait gives up
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < kUmmaSpinLimit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void tma_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// One matrix image to shared memory (one thread; `bar` counts one arrival and the bytes).
+__device__ __forceinline__ void umma_load_image(uint32_t dst, const uint16_t *image, uint32_t bar) {
+    mbar_expect_tx(bar, kUmmaImageBytes);
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i)
+        tma_load_1d(dst + i * kUmmaSlabBytes, reinterpret_cast<const uint8_t *>(image) + i * kUmmaSlabBytes, kUmmaSlabBytes, bar);
+}
+
+// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 B apart.
+__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
+           (2ull << 61);
+}
+// Instruction descriptor: D = f32, A = B = f16, both K-major, N = 128, M = 128.
+constexpr uint32_t kUmmaInstr = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+
+// D[128 x 128] (+)= A[128 x 16] (TMEM, two f16 per column) * B (shared memory)
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(kUmmaInstr), "r"(accumulate)
+        : "memory");
+}
+// The MMAs of one contraction (one thread): A in `terms` f16 terms at a_hi, a_lo, the matrix image at b_addr.
+__device__ __forceinline__ void umma_issue(uint32_t d, uint32_t a_hi, uint32_t a_lo, uint32_t b_addr, int terms) {
+    auto pass = [&](uint32_t a, uint32_t b, uint32_t first) {
+#pragma unroll 1
+        for (int s = 0; s < 8; ++s)
+            umma_f16(d, a + 8 * s, umma_desc(b + (s >> 2) * kUmmaSlabBytes + (s & 3) * 32), first | (s > 0));
+    };
+    pass(a_hi, b_addr + kUmmaTermBytes, 0);
+    if (terms == 2) pass(a_lo, b_addr, 1);
+    pass(a_hi, b_addr, 1);
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void umma_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void umma_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+
+// Byte offset of element (row, k) inside one f16 term of an image (two 64-wide slabs, 128-byte swizzle).
+__host__ __device__ inline int umma_operand_offset(int row, int k) {
+    const int slab = k >> 6, kk = k & 63;
+    return slab * kUmmaSlabBytes + (row >> 3) * 1024 + (row & 7) * 128 + (((kk >> 3) ^ (row & 7)) << 4) + (kk & 7) * 2;
+}
+
+// 32 consecutive accumulator columns of this thread's TMEM lane.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+// Eight columns (16 f16 of an A operand row) of this thread's TMEM lane; tmem_st_wait before anybody reads them.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+
+// Two floats at a time (one instruction for both on this architecture).
+__device__ __forceinline__ uint64_t f32x2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f32x2_split(uint64_t v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t f32x2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t f32x2_sub(uint64_t a, uint64_t b) {  // a - b
+    return f32x2_fma(b, f32x2(-1.f, -1.f), a);
+}
+
+// Two values as packed f16: rounded (hi) and what is left of them (lo).
+__device__ __forceinline__ uint32_t half2_bits(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ void split_half2(uint64_t v, uint32_t &hi, uint32_t &lo) {
+    float a, b;
+    f32x2_split(v, a, b);
+    hi = half2_bits(a, b);
+    const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
+    float ra, rb;
+    f32x2_split(f32x2_sub(v, f32x2(h.x, h.y)), ra, rb);
+    lo = half2_bits(ra, rb);
+}
