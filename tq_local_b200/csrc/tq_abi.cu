@@ -100,8 +100,8 @@ extern "C" int32_t tq_ctx_create(tq_ctx **out, int32_t device, const tq_codec_de
 
     const int kb = c->use_qjl ? c->bits - 1 : c->bits;
     const size_t M = (size_t)TQ_D * TQ_D;
-    // 6 plain matrices + 6 operand images of the same size + 4 tables of 16 floats.
-    const size_t n_float = 12 * M + 4 * 16 + 4;  // + the device status word
+    // 6 plain matrices + 3 operand images of the same size + 4 tables of 16 floats.
+    const size_t n_float = 9 * M + 4 * 16 + 4;  // + the device status word
     std::vector<float> h(n_float, 0.0f);
     auto mat = [&](int i) { return h.data() + (size_t)i * M; };
     auto transpose = [&](const float *src, float *dst) {
@@ -116,11 +116,10 @@ extern "C" int32_t tq_ctx_create(tq_ctx **out, int32_t device, const tq_codec_de
         memcpy(mat(4), c->qjl, M * 4);
         transpose(c->qjl, mat(5));
     }
-    // operand images (2 x 16384 f16 = 16384 floats each) in the 6 matrix-sized slots after the plain matrices
-    const int img_src[6] = {0, 2, 1, 3, 4, 5};  // R_k, R_v, R_k^T, R_v^T, S, S^T
-    float unscale[6];
-    for (int i = 0; i < 6; ++i) unscale[i] = tq_build_operand_image(mat(img_src[i]), reinterpret_cast<uint16_t *>(mat(6 + i)));
-    float *tab = h.data() + 12 * M;
+    // operand images (2 x 16384 f16 = 16384 floats each) in the matrix-sized slots after the plain matrices: R_k, R_v, S
+    float unscale[3];
+    for (int i = 0; i < 3; ++i) unscale[i] = tq_build_operand_image(mat(2 * i), reinterpret_cast<uint16_t *>(mat(6 + i)));
+    float *tab = h.data() + 9 * M;
     for (int i = 0; i < 16; ++i) {
         tab[i] = i < (1 << kb) ? c->centers_k[i] : 0.0f;
         tab[16 + i] = i < (1 << kb) - 1 ? c->bounds_k[i] : INFINITY;
@@ -160,8 +159,8 @@ extern "C" int32_t tq_ctx_create(tq_ctx **out, int32_t device, const tq_codec_de
     ctx->rot_v_t = dm(3);
     ctx->qjl = dm(4);
     ctx->qjl_t = dm(5);
-    tq_ctx::Image *images[6] = {&ctx->img_rot_k, &ctx->img_rot_v, &ctx->img_rot_kt, &ctx->img_rot_vt, &ctx->img_qjl, &ctx->img_qjl_t};
-    for (int i = 0; i < 6; ++i) images[i]->data = reinterpret_cast<uint16_t *>(dm(6 + i)), images[i]->unscale = unscale[i];
+    tq_ctx::Image *images[3] = {&ctx->img_rot_k, &ctx->img_rot_v, &ctx->img_qjl};
+    for (int i = 0; i < 3; ++i) images[i]->data = reinterpret_cast<uint16_t *>(dm(6 + i)), images[i]->unscale = unscale[i];
     float largest_k = 0.f, largest_v = 0.f, gain = 0.f;
     for (int i = 0; i < 16; ++i) largest_k = fmaxf(largest_k, fabsf(tab[i])), largest_v = fmaxf(largest_v, fabsf(tab[32 + i]));
     for (int dd = 0; dd < TQ_D; ++dd) {  // the largest column of R_k
@@ -170,10 +169,12 @@ extern "C" int32_t tq_ctx_create(tq_ctx **out, int32_t device, const tq_codec_de
         gain = fmaxf(gain, sqrtf(ss));
     }
     ctx->cen_k_scale = tq_fit_power(largest_k), ctx->cen_v_scale = tq_fit_power(largest_v);
+    if (!tq_fit_grid(tab + 16, (1 << kb) - 1, &ctx->grid_k)) ctx->grid_k.last = 0.f;
+    if (!tq_fit_grid(tab + 48, (1 << c->bits) - 1, &ctx->grid_v)) ctx->grid_v.last = 0.f;
     // |r_d| <= |x| (1 + |c| |column of R_k|), |c| <= sqrt(128) * largest centre; the encoder scales |x| below 2^13
     ctx->res_scale = 1.f;
     for (float reach = 1.f + gain * largest_k * 11.32f; reach > 7.9f && isfinite(reach); reach *= 0.5f) ctx->res_scale *= 0.5f;
-    ctx->centers_k = d + 12 * M;
+    ctx->centers_k = d + 9 * M;
     ctx->bounds_k = ctx->centers_k + 16;
     ctx->centers_v = ctx->centers_k + 32;
     ctx->bounds_v = ctx->centers_k + 48;

@@ -30,18 +30,17 @@ struct tq_ctx {
     float *bounds_k;   // [16] (padded with +inf)
     float *centers_v;
     float *bounds_v;
-    // Shared-memory images of the tcgen05 kernels' B operands (64 KB each, see tq_build_operand_image): rows n and
-    // contraction index k of the [128][128] matrix behind vec[k] -> out[n], in two f16 terms, times a power of two.
+    // Shared-memory images of the tcgen05 kernels' B operands (64 KB each, see tq_build_operand_image): R_k, R_v and S
+    // in two f16 terms, times a power of two.  A kernel reads one as it lies (vec R^T, vec S^T) or transposed (vec R, vec S).
     struct Image {
         uint16_t *data;
         float unscale;  // what undoes the power of two
     };
-    Image img_rot_k;    // n = j, k = d:  R_k[j][d]   u @ R_k^T
-    Image img_rot_v;
-    Image img_rot_kt;   // n = d, k = j:  R_k[j][d]   c @ R_k
-    Image img_rot_vt;
-    Image img_qjl;      // n = i, k = d:  S[i][d]     r @ S^T
-    Image img_qjl_t;    // n = d, k = i:  S[i][d]     signs @ S
+    Image img_rot_k, img_rot_v, img_qjl;
+    struct Grid {  // cell of z: round(clamp(z * scale + shift, 0, 1) * last); last == 0: no grid separates the boundaries
+        float scale, shift, last;
+    };
+    Grid grid_k, grid_v;
     float cen_k_scale, cen_v_scale;  // powers of two that bring the largest centre just below 2^14
     float res_scale;    // power of two <= 1 that keeps a unit vector's scaled residual inside f16 whatever the centres
     void *base;       // one allocation holding everything above
@@ -154,8 +153,9 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
                               const tq_dense_desc *tail_v, int32_t n_tail, int32_t n_splits,
                               void *workspace, void *out, const TqStepExtras *extras, cudaStream_t stream);
 float tq_fit_power(float largest);  // the power of two that brings `largest` into [2^13, 2^14)
+bool tq_fit_grid(const float *bounds, int n, tq_ctx::Grid *g);
 float tq_build_operand_image(const float *m, uint16_t *image);
-// `k` null: values only.  TQ_ERR_UNSUPPORTED when a tensor's alignment rules the kernel out.
+// `k` null: values only.  TQ_ERR_UNSUPPORTED when a tensor's alignment or the codebook rules the kernel out.
 int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tokens,
                           const tq_cache_desc *cache, int32_t pos0, cudaStream_t stream);
 // TQ_ERR_UNSUPPORTED when the output's alignment rules the kernel out.

@@ -3,10 +3,13 @@
 //   out = round_T(|x| * centres[codes] R)  [ + round_T(|r| * sqrt(pi/2)/128 * signs S), rounded again ]
 //
 // with the matrices in two f16 terms (tq_umma.cuh), the centres in two and the signs (+-1) in one.  The
-// structure is the prefill encoder's: one persistent CTA per SM, two groups of eight warps that each walk
-// their own tiles, A written to TMEM, the matrices resident in shared memory; the two contractions of a
-// key go one after the other through the group's one accumulator, the first result waiting as packed T.
+// structure is the prefill encoder's: one persistent CTA per SM, two groups of sixteen warps that each walk
+// their own tiles, four threads to a vector, A written to TMEM, the matrices resident in shared memory; the two
+// contractions of a key go one after the other through the group's one accumulator, the first result waiting as
+// packed T.  16-bit rows leave through shared memory, one bulk copy each.
 #include <math.h>
+
+#include <type_traits>
 
 #include "tq_common.cuh"
 #include "tq_umma.cuh"
@@ -14,9 +17,10 @@
 namespace {
 
 constexpr int kGroups = 2;
-constexpr int kGroupThreads = 256;
+constexpr int kGroupThreads = 512;
 constexpr int kThreads = kGroups * kGroupThreads;
-constexpr int kHalf = TQ_D / 2;  // coordinates per thread
+constexpr int kParts = kGroupThreads / kUmmaRows;  // threads per vector
+constexpr int kCoords = TQ_D / kParts;             // coordinates per thread
 
 struct DequantTcArgs {
     const uint8_t *codes;
@@ -24,10 +28,11 @@ struct DequantTcArgs {
     const uint8_t *signs;
     const uint16_t *rnorms;
     int64_t cache_sb, cache_sh;
-    int B, H, S, pos0, n_tiles;
+    VectorIndex vec;
+    int pos0, n_tiles;
     void *out;
     int64_t ob, oh, ot;
-    const uint16_t *image, *image2;  // R^T, S^T
+    const uint16_t *image, *image2;  // R, S
     float unscale, unscale2;         // undo the scales of R and the centres, and of S
     const float *centers;            // 16 floats
     float cen_scale;
@@ -74,27 +79,31 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
     __syncthreads();
     umma_fence_after();
 
-    const int vrow = tid & (kUmmaRows - 1), half = (tid >> 7) & 1;
+    const int vrow = tid & (kUmmaRows - 1), part = (tid / kUmmaRows) % kParts;
     const uint32_t acc = s_tmem + group * 256, a_hi = acc + 128, a_lo = acc + 192;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t my_acc = acc + lanes + kHalf * half, my_hi = a_hi + lanes + kHalf / 2 * half, my_lo = a_lo + lanes + kHalf / 2 * half;
+    const uint32_t my_acc = acc + lanes + kCoords * part, my_hi = a_hi + lanes + kCoords / 2 * part, my_lo = my_hi + 64;
     const uint32_t bar_mma = smem_u32(&s_bar_mma[group]);
     const bool issuer = (tid & (kGroupThreads - 1)) == 0;
     bool timed_out = false;
     uint32_t mma_phase = 0, landed = 0;
+    constexpr bool kStaged = sizeof(T) == 2;
+    const uint32_t my_stage = images + (QJL ? 2 : 1) * kUmmaImageBytes + group * kStageBytes + vrow * kStagePitch;
+    auto group_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + group), "r"(kGroupThreads) : "memory"); };
     // Everybody has stored its part of A and read the accumulators of the stage before: two products when A
     // has one term (the signs), three when it has two.
-    auto gemm = [&](int stage, int terms) {
+    auto gemm = [&](auto terms) {  // stage 0: the centres, two terms; stage 1: the signs, one
+        constexpr int kTerms = decltype(terms)::value, stage = 2 - kTerms;
         tmem_st_wait();
         umma_fence_before();
-        asm volatile("bar.sync %0, %1;\n" ::"r"(1 + group), "r"(kGroupThreads) : "memory");
+        group_sync();
         if (issuer) {
             umma_fence_after();
             if (!(landed >> stage & 1)) {
                 if (!mbar_wait(smem_u32(&s_bar_image[stage]), 0)) timed_out = true;
                 landed |= 1u << stage;
             }
-            umma_issue(acc, a_hi, a_lo, images + stage * kUmmaImageBytes, terms);
+            umma_issue<kTerms, true>(acc, a_hi, a_lo, images + stage * kUmmaImageBytes);
             umma_commit(bar_mma);
         }
     };
@@ -105,49 +114,38 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
         umma_fence_after();
     };
 
-    constexpr int kWords = 2 * BITS;  // of this thread's 64 codes
-    const int64_t n_vec = (int64_t)a.B * a.H * a.S;
-    uint32_t words[kWords + 1];
-    uint2 sw = make_uint2(0, 0);
+    // this thread's 32 codes
+    uint32_t words[BITS + 1];
+    uint32_t sw = 0;
     uint16_t nh = 0, rh = 0;
     T *dst = nullptr;
-    words[kWords] = 0;
+    words[BITS] = 0;
     auto fetch = [&](int tile) {
         const int64_t vid = (int64_t)tile * kUmmaRows + vrow;
-        const int64_t v = vid < n_vec ? vid : 0;
+        const int64_t v = vid < a.vec.n ? vid : 0;
         int t, h, b;
-        if (n_vec <= 0x7fffffff) {  // (32-bit divisions are several times cheaper)
-            const uint32_t q = (uint32_t)v / (uint32_t)a.S;
-            t = (int)((uint32_t)v - q * a.S), b = (int)(q / (uint32_t)a.H), h = (int)(q - (uint32_t)b * a.H);
-        } else {
-            t = (int)(v % a.S), h = (int)((v / a.S) % a.H), b = (int)(v / ((int64_t)a.S * a.H));
-        }
+        vector_at(a.vec, v, b, h, t);
         const int64_t row = b * a.cache_sb + h * a.cache_sh + a.pos0 + t;
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(a.codes + row * (16 * BITS) + half * (8 * BITS));
-        if constexpr (kWords % 4 == 0) {
-#pragma unroll
-            for (int w = 0; w < kWords; w += 4) {
-                const uint4 c = __ldg(reinterpret_cast<const uint4 *>(src + w));
-                words[w] = c.x, words[w + 1] = c.y, words[w + 2] = c.z, words[w + 3] = c.w;
-            }
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(a.codes + row * (16 * BITS)) + BITS * part;
+        if constexpr (BITS == 4) {
+            const uint4 c = __ldg(reinterpret_cast<const uint4 *>(src));
+            words[0] = c.x, words[1] = c.y, words[2] = c.z, words[3] = c.w;
         } else {
 #pragma unroll
-            for (int w = 0; w < kWords; w += 2) {
-                const uint2 c = __ldg(reinterpret_cast<const uint2 *>(src + w));
-                words[w] = c.x, words[w + 1] = c.y;
-            }
+            for (int w = 0; w < BITS; ++w) words[w] = __ldg(src + w);
         }
         nh = a.norms[row];
-        if (QJL) sw = __ldg(reinterpret_cast<const uint2 *>(a.signs + row * 16 + 8 * half)), rh = a.rnorms[row];
-        dst = vid < n_vec ? reinterpret_cast<T *>(a.out) + b * a.ob + h * a.oh + (int64_t)t * a.ot + kHalf * half : nullptr;
+        if (QJL) sw = __ldg(reinterpret_cast<const uint32_t *>(a.signs + row * 16) + part), rh = a.rnorms[row];
+        dst = vid < a.vec.n ? reinterpret_cast<T *>(a.out) + b * a.ob + h * a.oh + (int64_t)t * a.ot : nullptr;
     };
     const int first = (int)blockIdx.x + (int)gridDim.x * group, stride = (int)gridDim.x * kGroups;
     if (first < a.n_tiles) fetch(first);
     for (int tile = first; tile < a.n_tiles; tile += stride) {
         // ---------------- A = centres[codes]
+        if (kStaged) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
         __syncwarp();  // (tcgen05.st is warp-collective)
 #pragma unroll
-        for (int c = 0; c < kHalf / 16; ++c) {
+        for (int c = 0; c < kCoords / 16; ++c) {
             uint32_t hi[8], lo[8];
             auto centre = [&](int e) {
                 const int bit = e * BITS, w = bit >> 5, sh = bit & 31;
@@ -161,64 +159,75 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
             }
             tmem_st8(my_hi + 8 * c, hi), tmem_st8(my_lo + 8 * c, lo);
         }
-        gemm(0, 2);
+        gemm(std::integral_constant<int, 2>());
         const float nf = tq_half_bits_to_float(nh) * a.unscale;
         const float rf = tq_half_bits_to_float(rh);
-        const uint2 signs = sw;
+        const uint32_t signs = sw;
         T *const to = dst;
         if (tile + stride < a.n_tiles) fetch(tile + stride);
         gemm_wait();
-        constexpr int kOutWords = kHalf * (int)sizeof(T) / 4;
-        uint32_t o[kOutWords];  // this thread's 64 outputs
+        constexpr int kOutWords = kCoords * (int)sizeof(T) / 4;
+        uint32_t o[kOutWords];  // this thread's 32 outputs
         const uint64_t nf2 = f32x2(nf, nf);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            uint32_t y[32];
-            tmem_ld32(my_acc + 32 * q, y);
+        for (int q = 0; q < kCoords / 16; ++q) {
+            uint32_t y[16];
+            tmem_ld16(my_acc + 16 * q, y);
 #pragma unroll
-            for (int e = 0; e < 32; e += 2) {
+            for (int e = 0; e < 16; e += 2) {
                 float y0, y1;
                 f32x2_split(f32x2_mul(f32x2(__uint_as_float(y[e]), __uint_as_float(y[e + 1])), nf2), y0, y1);
-                if constexpr (sizeof(T) == 4) o[32 * q + e] = __float_as_uint(y0), o[32 * q + e + 1] = __float_as_uint(y1);
-                else o[16 * q + e / 2] = pack2<T>(y0, y1);
+                if constexpr (sizeof(T) == 4) o[16 * q + e] = __float_as_uint(y0), o[16 * q + e + 1] = __float_as_uint(y1);
+                else o[8 * q + e / 2] = pack2<T>(y0, y1);
             }
         }
         if constexpr (QJL) {
             // ---------------- A = signs: f16 1.0 with the complement of the sign bit on top
 #pragma unroll
-            for (int c = 0; c < kHalf / 16; ++c) {
-                const uint32_t w = ~(c < 2 ? signs.x : signs.y) >> (16 * (c & 1));
+            for (int c = 0; c < kCoords / 16; ++c) {
+                const uint32_t w = ~signs >> (16 * c);
                 uint32_t s[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) s[i] = 0x3C003C00u | ((w << (15 - 2 * i)) & 0x8000u) | ((w << (30 - 2 * i)) & 0x80000000u);
                 tmem_st8(my_hi + 8 * c, s);
             }
-            gemm(1, 1);
+            gemm(std::integral_constant<int, 1>());
             gemm_wait();
             const float scale = 1.2533141373155003f / (float)TQ_D;  // sqrt(pi/2)/D
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                uint32_t y[32];
-                tmem_ld32(my_acc + 32 * q, y);
+            for (int q = 0; q < kCoords / 16; ++q) {
+                uint32_t y[16];
+                tmem_ld16(my_acc + 16 * q, y);
 #pragma unroll
-                for (int e = 0; e < 32; e += 2) {
+                for (int e = 0; e < 16; e += 2) {
                     const float y0 = __uint_as_float(y[e]) * a.unscale2 * rf * scale, y1 = __uint_as_float(y[e + 1]) * a.unscale2 * rf * scale;
                     if constexpr (sizeof(T) == 4) {
-                        o[32 * q + e] = __float_as_uint(__uint_as_float(o[32 * q + e]) + y0);
-                        o[32 * q + e + 1] = __float_as_uint(__uint_as_float(o[32 * q + e + 1]) + y1);
+                        o[16 * q + e] = __float_as_uint(__uint_as_float(o[16 * q + e]) + y0);
+                        o[16 * q + e + 1] = __float_as_uint(__uint_as_float(o[16 * q + e + 1]) + y1);
                     } else {
-                        const float2 r = unpack2<T>(o[16 * q + e / 2]), c = unpack2<T>(pack2<T>(y0, y1));
-                        o[16 * q + e / 2] = pack2<T>(r.x + c.x, r.y + c.y);
+                        const float2 r = unpack2<T>(o[8 * q + e / 2]), c = unpack2<T>(pack2<T>(y0, y1));
+                        o[8 * q + e / 2] = pack2<T>(r.x + c.x, r.y + c.y);
                     }
                 }
             }
         }
-        if (to) {
+        if constexpr (kStaged) {
+            // (the rows of the tile before have left: their threads waited for that before this tile's first barrier)
+#pragma unroll
+            for (int i = 0; i < kOutWords; i += 4) sts128(my_stage + 2 * kCoords * part + 4 * i, o[i], o[i + 1], o[i + 2], o[i + 3]);
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            group_sync();
+            if (part == 0) {
+                if (to) tma_store_1d(to, my_stage, 2 * TQ_D);
+                asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+            }
+        } else if (to) {
 #pragma unroll
             for (int i = 0; i < kOutWords; i += 4)
-                *reinterpret_cast<uint4 *>(reinterpret_cast<uint32_t *>(to) + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+                *reinterpret_cast<uint4 *>(reinterpret_cast<uint32_t *>(to) + kOutWords * part + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
         }
     }
+    if (kStaged) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     if (timed_out) atomicExch(a.error_flag, 3);
     umma_fence_before();
     __syncthreads();
@@ -229,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
 }
 
 template <typename T, int BITS, bool QJL> cudaError_t launch(const DequantTcArgs &a, int grid, int device, cudaStream_t stream) {
-    const int smem = (QJL ? 2 : 1) * kUmmaImageBytes + 1024;
+    constexpr int smem = (QJL ? 2 : 1) * kUmmaImageBytes + (sizeof(T) == 2 ? kGroups * kStageBytes : 0) + 1024;
     // the attribute belongs to the (kernel, device) pair: one flag per device of this instantiation
     static bool configured[TQ_MAX_DEVICES] = {};
     if (device < 0 || device >= TQ_MAX_DEVICES) return cudaErrorInvalidDevice;
@@ -258,18 +267,17 @@ int32_t tq_launch_dequant_tc(tq_ctx *ctx, const tq_cache_desc *cache, int32_t wh
     const int64_t esize = out->dtype == TQ_DTYPE_F32 ? 4 : 2;
     if (((uintptr_t)out->data | (uintptr_t)((out->stride_b | out->stride_h | out->stride_t) * esize)) & 15) return TQ_ERR_UNSUPPORTED;
     const bool key = which == 0, qjl = key && ctx->use_qjl;
-    const int64_t n_vec = (int64_t)cache->batch * cache->kv_heads * n_tokens;
     DequantTcArgs a;
     a.codes = key ? cache->k_codes : cache->v_codes, a.norms = key ? cache->k_norms : cache->v_norms;
     a.signs = cache->k_signs, a.rnorms = cache->k_rnorms;
     a.cache_sb = cache->stride_b, a.cache_sh = cache->stride_h;
-    a.B = cache->batch, a.H = cache->kv_heads, a.S = n_tokens, a.pos0 = pos0;
-    a.n_tiles = (int)((n_vec + kUmmaRows - 1) / kUmmaRows);
+    a.vec = vector_index(cache->batch, cache->kv_heads, n_tokens), a.pos0 = pos0;
+    a.n_tiles = (int)((a.vec.n + kUmmaRows - 1) / kUmmaRows);
     a.out = const_cast<void *>(out->data), a.ob = out->stride_b, a.oh = out->stride_h, a.ot = out->stride_t;
-    const tq_ctx::Image &image = key ? ctx->img_rot_kt : ctx->img_rot_vt;
-    a.image = image.data, a.image2 = ctx->img_qjl_t.data;
+    const tq_ctx::Image &image = key ? ctx->img_rot_k : ctx->img_rot_v;
+    a.image = image.data, a.image2 = ctx->img_qjl.data;
     a.cen_scale = key ? ctx->cen_k_scale : ctx->cen_v_scale;
-    a.unscale = image.unscale / a.cen_scale, a.unscale2 = ctx->img_qjl_t.unscale;
+    a.unscale = kUmmaRestore * image.unscale / a.cen_scale, a.unscale2 = kUmmaRestore * ctx->img_qjl.unscale;
     a.centers = key ? ctx->centers_k : ctx->centers_v;
     a.error_flag = ctx->error_flag;
     const int grid = a.n_tiles < ctx->sm_count ? a.n_tiles : ctx->sm_count;

@@ -11,11 +11,13 @@
 // are, bf16 rows times the power of two that brings |x| to [2^12, 2^13), which is exact down to 2^-37 |x|.
 // Nothing is normalised before a contraction; the accumulators are multiplied by 1 / |x| instead.
 //
-// One CTA of 16 warps per SM: two groups of eight warps, each walking tiles of 128 vectors on its own, so
-// that one group's CUDA-core work runs beside the other group's MMAs.  Two threads share a vector (64
+// One CTA of 32 warps per SM: two groups of sixteen warps, each walking tiles of 128 vectors on its own, so
+// that one group's CUDA-core work runs beside the other group's MMAs.  Four threads share a vector (32
 // coordinates each).  The A operand is written to TMEM (tcgen05.st, no swizzle, no bank conflicts), so
-// shared memory is left for the matrices: the three of the sketch path (192 KB) stay resident and nothing
-// is reloaded between the stages.  A group owns 256 TMEM columns: 128 of accumulator, 64 for each term of A.
+// shared memory is left for the matrices: R_k (stage 1; stage 2 reads the same image transposed) and S stay
+// resident and nothing is reloaded between the stages.  Rows of 16-bit vectors come through shared memory, one
+// bulk copy each: read straight from global memory by the threads that own them they took 2048 of the 4500
+// L1 wavefronts of a value tile, which bounded it.  A group owns 256 TMEM columns: 128 of accumulator, 64 for each term of A.
 // The first CTAs of a launch encode keys and the others values, in the proportion of their costs.
 // Every mbarrier wait is bounded and reports through the device status word.
 #include <math.h>
@@ -29,9 +31,12 @@
 namespace {
 
 constexpr int kGroups = 2;
-constexpr int kGroupThreads = 256;
+constexpr int kGroupThreads = 512;
 constexpr int kThreads = kGroups * kGroupThreads;
-constexpr int kHalf = TQ_D / 2;  // coordinates per thread
+constexpr int kMaxCells = 64;
+constexpr int kCellCopies = 16;  // of the search table: lane l reads copy l % 16, so an 8-byte look-up has no bank conflicts
+constexpr int kParts = kGroupThreads / kUmmaRows;  // threads per vector
+constexpr int kCoords = TQ_D / kParts;             // coordinates per thread
 
 struct PackTcRole {
     const void *x;
@@ -41,38 +46,40 @@ struct PackTcRole {
     const uint16_t *image;  // the rotation
     float unscale;
     const float *bounds;    // 16 floats, padded with +inf
+    tq_ctx::Grid grid;      // the search grid of these boundaries
 };
 struct PackTcArgs {
     PackTcRole role[2];  // keys, values
     int key_ctas;        // CTAs [0, key_ctas) encode keys, the others values
-    int B, H, S, pos0;
+    VectorIndex vec;
+    int pos0;
     int64_t cache_sb, cache_sh;
     int n_tiles;
     int *error_flag;
     // the sketch
-    const uint16_t *image2, *image3;  // R_k^T (reconstruction), S (projection)
-    float unscale2;                   // undoes the scales of R_k^T and of the centres
+    const uint16_t *image_s;          // S (projection)
+    float unscale2;                   // undoes the scales of R_k and of the centres
     float cen_scale, res_scale;
     const float *centers;  // 16 floats
     uint8_t *signs;
     uint16_t *rnorms;
 };
 
-template <typename T> struct Raw;  // how many 32-bit words 64 coordinates take, and pairs of them as floats
+template <typename T> struct Raw;  // how many 32-bit words a thread's coordinates take, and pairs of them as floats
 template <> struct Raw<float> {
-    static constexpr int kWords = kHalf;
+    static constexpr int kWords = kCoords;
     static __device__ __forceinline__ uint64_t pair(const uint32_t (&w)[kWords], int i) {
         return f32x2(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
     }
 };
 template <> struct Raw<__nv_bfloat16> {
-    static constexpr int kWords = kHalf / 2;
+    static constexpr int kWords = kCoords / 2;
     static __device__ __forceinline__ uint64_t pair(const uint32_t (&w)[kWords], int i) {
         return f32x2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
     }
 };
 template <> struct Raw<__half> {
-    static constexpr int kWords = kHalf / 2;
+    static constexpr int kWords = kCoords / 2;
     static __device__ __forceinline__ uint64_t pair(const uint32_t (&w)[kWords], int i) {
         const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[i]));
         return f32x2(f.x, f.y);
@@ -103,54 +110,100 @@ __device__ __forceinline__ float fit_power(float v) {
     return __uint_as_float((uint32_t)min(254, 266 - e) << 23);
 }
 
-// 4 * (number of boundaries strictly below z), a byte offset into the tables of 16 floats.  The first two
-// levels of the search compare with registers, the others with shared memory (one bank per entry).
-template <int BITS> struct Search {
-    float top, lo, hi;
-    const float *table;
-    __device__ __forceinline__ explicit Search(const float *bounds) : table(bounds) {
-        top = bounds[(1 << (BITS - 1)) - 1];
-        lo = BITS > 1 ? bounds[(1 << BITS) / 4 - 1] : 0.f;
-        hi = BITS > 1 ? bounds[3 * (1 << BITS) / 4 - 1] : 0.f;
+// MUL * (number of boundaries strictly below z).  One or two bits: binary search in registers.  More: z's cell
+// in a uniform grid gives the number of boundaries in the cells before it and the one boundary that may lie
+// in its own (tq_fit_grid makes sure that there is no second one); the cell is a monotone function of z and
+// the boundaries' cells are formed by the same instructions, so the answer is that of comparing with all of them.
+// Against a binary search in shared memory this saves five instructions a coordinate at four bits.
+__device__ __forceinline__ uint32_t grid_cell(float z, const tq_ctx::Grid &g) {  // + 0x4B000000
+    float t;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;\n" : "=f"(t) : "f"(z), "f"(g.scale), "f"(g.shift));  // (NaN: 0)
+    return __float_as_uint(fmaf(t, g.last, 8388608.f));
+}
+template <int BITS, int MUL> struct Search {
+    float b0, b1, b2;
+    tq_ctx::Grid grid;
+    uint32_t table;
+    __device__ __forceinline__ Search(const float *bounds, const uint2 *cells, const tq_ctx::Grid &g) : grid(g) {
+        b0 = bounds[0], b1 = bounds[1], b2 = bounds[2];
+        table = smem_u32(cells) + 8 * (threadIdx.x % kCellCopies) - (0x4B000000u << 7);
     }
     __device__ __forceinline__ uint32_t operator()(float z) const {
-        const bool up = top < z;
-        uint32_t o = up ? 2u << BITS : 0u;
-        if (BITS > 1 && (up ? hi : lo) < z) o += 1u << BITS;
-#pragma unroll
-        for (int step = (1 << BITS) / 8; step > 0; step >>= 1)
-            if (*reinterpret_cast<const float *>(reinterpret_cast<const char *>(table + step - 1) + o) < z) o += 4 * step;
-        return o;
+        if (BITS == 1) return b0 < z ? MUL : 0u;
+        if (BITS == 2) {
+            const bool up = b1 < z;
+            return (up ? 2u * MUL : 0u) + ((up ? b2 : b0) < z ? MUL : 0u);
+        }
+        uint32_t bound, below;
+        asm("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(bound), "=r"(below) : "r"(grid_cell(z, grid) * (8u * kCellCopies) + table));
+        return below + (__uint_as_float(bound) < z ? MUL : 0u);
     }
 };
+// Fills the grid's table (all threads of the CTA; barriers around it are the caller's).
+__device__ __forceinline__ void build_cells(uint2 *cells, const float *bounds, int n_bounds, const tq_ctx::Grid &g, uint32_t mul) {
+    for (int i = threadIdx.x; i < kCellCopies * ((int)g.last + 1); i += kThreads) {
+        const int c = i / kCellCopies;
+        uint32_t below = 0;
+        float mine = INFINITY;
+        for (int e = 0; e < n_bounds; ++e) {
+            const int at = (int)(grid_cell(bounds[e], g) - 0x4B000000u);
+            below += at < c ? mul : 0u;
+            if (at == c) mine = bounds[e];
+        }
+        cells[i] = make_uint2(__float_as_uint(mine), below);
+    }
+}
 
-// ORs code c (given as 4 * c) into place i of a bitstream of BITS-bit codes
-template <int BITS, int N> __device__ __forceinline__ void put_code(uint32_t (&words)[N], int i, uint32_t c4) {
-    const int bit = i * BITS, w = bit >> 5, sh = bit & 31;
-    words[w] |= sh >= 2 ? c4 << (sh - 2) : c4 >> (2 - sh);
-    if (sh + BITS > 32) words[w + 1] |= c4 >> (34 - sh);
+// 32 codes of BITS bits (times MUL, a power of two) as a bitstream, LSB first, sixteen codes at a time.
+template <int BITS, int MUL> __device__ __forceinline__ void put_codes(uint32_t (&words)[BITS], int q, const uint32_t (&c)[16]) {
+    constexpr int kPer = BITS == 3 ? 8 : BITS == 4 ? 8 : 16;  // codes that fit one register
+    uint32_t piece[16 / kPer];
+#pragma unroll
+    for (int p = 0; p < 16 / kPer; ++p) {
+        uint32_t v = c[kPer * p + kPer - 1];
+        if (MUL > 1 && BITS != 3) v /= MUL;
+#pragma unroll
+        for (int i = kPer - 2; i >= 0; --i) v = v * (1u << BITS) + (MUL > 1 && BITS != 3 ? c[kPer * p + i] / MUL : c[kPer * p + i]);
+        piece[p] = MUL > 1 && BITS == 3 ? v / MUL : v;
+    }
+    if (BITS == 1) {
+        if (q == 0) words[0] = piece[0];
+        else words[0] |= piece[0] << 16;
+    } else if (BITS == 2) {
+        words[q % BITS] = piece[0];
+    } else if (BITS == 4) {
+        words[(2 * q) % BITS] = piece[0], words[(2 * q + 1) % BITS] = piece[1 % (16 / kPer)];
+    } else {  // 24-bit pieces
+        const uint32_t p0 = piece[0], p1 = piece[1 % (16 / kPer)];
+        if (q == 0) {
+            words[0] = p0 | p1 << 24, words[1 % BITS] = p1 >> 8;
+        } else {
+            words[1 % BITS] |= p0 << 16, words[2 % BITS] = p0 >> 16 | p1 << 8;
+        }
+    }
 }
 
 struct PackTcShared {
+    uint2 cells[kMaxCells * kCellCopies];  // {boundary, codes below}, see Search
     float bounds[16];
     uint32_t centers[16];  // f16 hi term | lo term << 16 of a scaled key centre
-    float sq[kGroups][2][2][kUmmaRows];  // squared norms: [group][tile parity][half of the coordinates][vector]
-    float big[kGroups][2][2][kUmmaRows];  // largest magnitudes of halves whose squared norm is zero
-    float rs[kGroups][2][kUmmaRows];     // squared residual norms
-    uint64_t bar_image[3], bar_mma[kGroups];
+    float sq[kGroups][2][kParts][kUmmaRows];   // squared norms: [group][tile parity][part of the coordinates][vector]
+    float big[kGroups][2][kParts][kUmmaRows];  // largest magnitudes of parts whose squared norm is zero
+    float rs[kGroups][kParts][kUmmaRows];         // squared residual norms
+    uint64_t bar_image[2], bar_mma[kGroups], bar_rows[kGroups];
     uint32_t tmem;
 };
 
 template <typename T, int BITS, bool QJL>
-__device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r, PackTcShared &sm, uint32_t images, int cta, int n_ctas) {
+__device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r, PackTcShared &sm, uint32_t images, uint32_t staged, int cta, int n_ctas) {
     using R = Raw<T>;
     constexpr int kTermsX = sizeof(T) == 4 ? 2 : 1;
     const int tid = threadIdx.x, group = tid / kGroupThreads, warp = tid >> 5;
     const int vrow = tid & (kUmmaRows - 1);            // this thread's vector within the tile (= its TMEM lane)
-    const int half = (tid >> 7) & 1;                   // which half of the coordinates it works on
+    const int part = (tid / kUmmaRows) % kParts;       // which part of the coordinates it works on
     const uint32_t acc = sm.tmem + group * 256, a_hi = acc + 128, a_lo = acc + 192;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t my_acc = acc + lanes + kHalf * half, my_hi = a_hi + lanes + kHalf / 2 * half, my_lo = a_lo + lanes + kHalf / 2 * half;
+    const uint32_t my_acc = acc + lanes + kCoords * part, my_hi = a_hi + lanes + kCoords / 2 * part, my_lo = my_hi + 64;
     const uint32_t bar_mma = smem_u32(&sm.bar_mma[group]);
     const bool issuer = (tid & (kGroupThreads - 1)) == 0;
     bool timed_out = false;
@@ -159,17 +212,17 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
 
     auto group_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + group), "r"(kGroupThreads) : "memory"); };
     // Everybody has stored its part of A (and read the accumulators of the stage before): issue the MMAs.
-    auto gemm_issue = [&](int stage, int terms) {
+    auto gemm_issue = [&](int image, auto terms, auto transposed) {
         tmem_st_wait();
         umma_fence_before();
         group_sync();
         if (issuer) {
             umma_fence_after();
-            if (!(landed >> stage & 1)) {
-                if (!mbar_wait(smem_u32(&sm.bar_image[stage]), 0)) timed_out = true;
-                landed |= 1u << stage;
+            if (!(landed >> image & 1)) {
+                if (!mbar_wait(smem_u32(&sm.bar_image[image]), 0)) timed_out = true;
+                landed |= 1u << image;
             }
-            umma_issue(acc, a_hi, a_lo, images + stage * kUmmaImageBytes, terms);
+            umma_issue<decltype(terms)::value, decltype(transposed)::value>(acc, a_hi, a_lo, images + image * kUmmaImageBytes);
             umma_commit(bar_mma);
         }
     };
@@ -179,58 +232,73 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
         __syncwarp();  // the issuer took its own path; tcgen05.ld is warp-collective
         umma_fence_after();
     };
+    const std::integral_constant<int, 1> one_term;
+    const std::integral_constant<int, 2> two_terms;
 
-    const int64_t n_vec = (int64_t)a.B * a.H * a.S;
-    struct RowRef {
-        const T *src;
-        int64_t row;
-        bool valid;
-    };
-    auto locate = [&](int tile) {  // this thread's vector of a tile: where it comes from, where it goes
+    // Rows of 16-bit vectors are staged in shared memory (requested by the threads of part 0, a row each); fp32
+    // rows, for which there is no room, come straight from global memory.
+    constexpr bool kStaged = sizeof(T) == 2;
+    const uint32_t my_stage = staged + group * kStageBytes + vrow * kStagePitch, bar_rows = smem_u32(&sm.bar_rows[group]);
+    uint32_t raw[R::kWords];  // this thread's part of the vector, as stored
+    int64_t row = 0;          // the vector's cache row (< 0: no vector)
+    uint32_t rows_phase = 0;
+    auto request = [&](int tile) {  // (the group is done with the rows before)
         const int64_t vid = (int64_t)tile * kUmmaRows + vrow;
-        RowRef ref;
-        ref.valid = vid < n_vec;
-        const int64_t v = ref.valid ? vid : 0;
+        const bool valid = vid < a.vec.n;
         int t, h, b;
-        if (n_vec <= 0x7fffffff) {  // (32-bit divisions are several times cheaper)
-            const uint32_t q = (uint32_t)v / (uint32_t)a.S;
-            t = (int)((uint32_t)v - q * a.S), b = (int)(q / (uint32_t)a.H), h = (int)(q - (uint32_t)b * a.H);
+        vector_at(a.vec, valid ? vid : 0, b, h, t);
+        const T *src = reinterpret_cast<const T *>(r.x) + b * r.sb + h * r.sh + (int64_t)t * r.st;
+        row = valid ? b * a.cache_sb + h * a.cache_sh + a.pos0 + t : -1;
+        if constexpr (kStaged) {
+            if (part == 0) {
+                mbar_expect_tx(bar_rows, 2 * TQ_D);
+                tma_load_1d(my_stage, src, 2 * TQ_D, bar_rows);
+            }
         } else {
-            t = (int)(v % a.S), h = (int)((v / a.S) % a.H), b = (int)(v / ((int64_t)a.S * a.H));
-        }
-        ref.src = reinterpret_cast<const T *>(r.x) + b * r.sb + h * r.sh + (int64_t)t * r.st + kHalf * half;
-        ref.row = b * a.cache_sb + h * a.cache_sh + a.pos0 + t;
-        return ref;
-    };
-    uint32_t raw[R::kWords];  // this thread's half of the vector, as stored
-    auto fetch = [&](const RowRef &ref) {
 #pragma unroll
-        for (int i = 0; i < R::kWords / 4; ++i) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(ref.src) + i);
-            raw[4 * i] = v.x, raw[4 * i + 1] = v.y, raw[4 * i + 2] = v.z, raw[4 * i + 3] = v.w;
+            for (int i = 0; i < R::kWords / 4; ++i) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(src + kCoords * part) + i);
+                raw[4 * i] = v.x, raw[4 * i + 1] = v.y, raw[4 * i + 2] = v.z, raw[4 * i + 3] = v.w;
+            }
         }
     };
-    // (keeps the compiler from holding the 64 converted values in registers from one use to the next)
+    auto read_rows = [&]() {
+        if constexpr (kStaged) {
+#pragma unroll
+            for (int i = 0; i < R::kWords / 4; ++i) {
+                const uint4 v = lds128(my_stage + 2 * kCoords * part + 16 * i);
+                raw[4 * i] = v.x, raw[4 * i + 1] = v.y, raw[4 * i + 2] = v.z, raw[4 * i + 3] = v.w;
+            }
+        }
+    };
+    auto rows_wait = [&]() {
+        if constexpr (kStaged) {
+            if (!mbar_wait(bar_rows, rows_phase)) timed_out = true;
+            rows_phase ^= 1;
+        }
+    };
+    // (keeps the compiler from holding the converted values in registers from one use to the next)
     auto forget_conversions = [&]() {
         if (sizeof(T) == 2) {
 #pragma unroll
             for (int i = 0; i < R::kWords; ++i) asm volatile("" : "+r"(raw[i]));
         }
     };
-    const Search<BITS> search(sm.bounds);
+    const Search<BITS, QJL ? 4 : 1> search(sm.bounds, sm.cells, r.grid);
     const int first = cta + n_ctas * group, stride = n_ctas * kGroups;
-    RowRef cur = locate(first);
-    if (first < a.n_tiles) fetch(cur);
+    if (first < a.n_tiles) request(first);
     int parity = 0;
     for (int tile = first; tile < a.n_tiles; tile += stride, parity ^= 1) {
         // ---------------- stage 1: A = x (scaled).  The rows were requested while the last tile's MMAs ran.
         const bool more = tile + stride < a.n_tiles;
-        RowRef nxt = cur;
+        const int64_t my_row = row;
+        rows_wait();
+        read_rows();
         float ss;
         {
             uint64_t s0 = 0, s1 = 0;
 #pragma unroll
-            for (int i = 0; i < kHalf / 2; i += 2) {
+            for (int i = 0; i < kCoords / 2; i += 2) {
                 const uint64_t p0 = R::pair(raw, i), p1 = R::pair(raw, i + 1);
                 s0 = f32x2_fma(p0, p0, s0), s1 = f32x2_fma(p1, p1, s1);
             }
@@ -239,33 +307,34 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
             ss = (s[0] + s[1]) + (s[2] + s[3]);
         }
         float (*sq)[kUmmaRows] = sm.sq[group][parity], (*big)[kUmmaRows] = sm.big[group][parity];
-        sq[half][vrow] = ss;
+        sq[part][vrow] = ss;
         float nrm, inv;  // |x|; z = accumulator * inv
+        auto norm = [&]() { return sqrtf((sq[0][vrow] + sq[1][vrow]) + (sq[2][vrow] + sq[3][vrow])); };
         if constexpr (!std::is_same<T, __half>::value) {
             if (ss == 0.f) {
                 float m = 0.f;
 #pragma unroll
-                for (int i = 0; i < kHalf / 2; ++i) {
+                for (int i = 0; i < kCoords / 2; ++i) {
                     float u, v;
                     f32x2_split(R::pair(raw, i), u, v);
                     m = fmaxf(m, fmaxf(fabsf(u), fabsf(v)));
                 }
-                big[half][vrow] = m;
+                big[part][vrow] = m;
             }
             group_sync();
             forget_conversions();
-            nrm = sqrtf(sq[0][vrow] + sq[1][vrow]);
+            nrm = norm();
             float scale = fit_power(nrm);
             if (nrm != 0.f) {  // (scale * nrm is exact and lies in [2^12, 2^13))
                 inv = r.unscale / (scale * nrm);
             } else {  // a zero vector, or one whose squares underflow: taken as it is (norm 1)
-                scale = fit_power(fmaxf(big[0][vrow], big[1][vrow]));
+                scale = fit_power(fmaxf(fmaxf(big[0][vrow], big[1][vrow]), fmaxf(big[2][vrow], big[3][vrow])));
                 inv = r.unscale / scale;
             }
             const uint64_t scale2 = f32x2(scale, scale);
             __syncwarp();  // (tcgen05.st is warp-collective)
 #pragma unroll
-            for (int c = 0; c < kHalf / 16; ++c) {
+            for (int c = 0; c < kCoords / 16; ++c) {
                 uint32_t hi[8], lo[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -281,127 +350,109 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
                 tmem_st8(my_hi + 8 * c, hi);
                 if (kTermsX == 2) tmem_st8(my_lo + 8 * c, lo);
             }
-            gemm_issue(0, kTermsX);
+            gemm_issue(0, std::integral_constant<int, kTermsX>(), std::false_type());
         } else {
             __syncwarp();
 #pragma unroll
-            for (int c = 0; c < kHalf / 16; ++c) {
+            for (int c = 0; c < kCoords / 16; ++c) {
                 uint32_t hi[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) hi[i] = raw[8 * c + i];
                 tmem_st8(my_hi + 8 * c, hi);
             }
-            gemm_issue(0, 1);
-            nrm = sqrtf(sq[0][vrow] + sq[1][vrow]);
+            gemm_issue(0, one_term, std::false_type());
+            nrm = norm();
             inv = nrm > 0.f ? r.unscale / nrm : r.unscale;
         }
         const float safe = nrm > 0.f ? nrm : 1.f;
         forget_conversions();
-        if (!QJL && more) {  // the rows are stored: fetch the next tile's under the MMAs
-            nxt = locate(tile + stride);
-            fetch(nxt);
-        }
+        if (!QJL && more) request(tile + stride);  // everybody has read its rows: request the next tile's under the MMAs
         gemm_wait();
 
         // ---------------- epilogue 1: this thread's accumulators -> codes (and, for the sketch, A = centres[codes])
-        constexpr int kWords = 2 * BITS;
-        uint32_t words[kWords + 1];
-#pragma unroll
-        for (int w = 0; w <= kWords; ++w) words[w] = 0;
+        uint32_t words[BITS];
         const uint64_t inv2 = f32x2(inv, inv);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            uint32_t z[32];
-            tmem_ld32(my_acc + 32 * q, z);
+        for (int q = 0; q < kCoords / 16; ++q) {
+            uint32_t z[16], code[16];
+            tmem_ld16(my_acc + 16 * q, z);
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int e = 0; e < 16; e += 2) {
+                float z0, z1;
+                f32x2_split(f32x2_mul(f32x2(__uint_as_float(z[e]), __uint_as_float(z[e + 1])), inv2), z0, z1);
+                code[e] = search(z0), code[e + 1] = search(z1);
+            }
+            put_codes<BITS, QJL ? 4 : 1>(words, q, code);
+            if (QJL) {
                 uint32_t hi[8], lo[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const int e = 16 * c + 2 * i;
-                    float z0, z1;
-                    f32x2_split(f32x2_mul(f32x2(__uint_as_float(z[e]), __uint_as_float(z[e + 1])), inv2), z0, z1);
-                    const uint32_t c0 = search(z0), c1 = search(z1);
-                    put_code<BITS>(words, 32 * q + e, c0), put_code<BITS>(words, 32 * q + e + 1, c1);
-                    if (QJL) {
-                        const uint32_t t0 = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(sm.centers) + c0);
-                        const uint32_t t1 = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(sm.centers) + c1);
-                        hi[i] = __byte_perm(t0, t1, 0x5410), lo[i] = __byte_perm(t0, t1, 0x7632);
-                    }
+                    const uint32_t t0 = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(sm.centers) + code[2 * i]);
+                    const uint32_t t1 = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(sm.centers) + code[2 * i + 1]);
+                    hi[i] = __byte_perm(t0, t1, 0x5410), lo[i] = __byte_perm(t0, t1, 0x7632);
                 }
-                if (QJL) tmem_st8(my_hi + 16 * q + 8 * c, hi), tmem_st8(my_lo + 16 * q + 8 * c, lo);
+                tmem_st8(my_hi + 8 * q, hi), tmem_st8(my_lo + 8 * q, lo);
             }
         }
         const uint16_t nh = tq_float_to_half_bits(safe);
-        if (QJL) gemm_issue(1, 2);
-        if (cur.valid) {
-            uint32_t *dst = reinterpret_cast<uint32_t *>(r.codes + cur.row * (int64_t)(16 * BITS) + half * (8 * BITS));
-            if constexpr (kWords % 4 == 0) {
+        if (QJL) gemm_issue(0, two_terms, std::true_type());
+        if (my_row >= 0) {
+            uint32_t *dst = reinterpret_cast<uint32_t *>(r.codes + my_row * (16 * BITS)) + BITS * part;
+            if constexpr (BITS == 4) *reinterpret_cast<uint4 *>(dst) = make_uint4(words[0], words[1], words[2], words[3]);
+            else if constexpr (BITS == 2) *reinterpret_cast<uint2 *>(dst) = make_uint2(words[0], words[1]);
+            else {
 #pragma unroll
-                for (int w = 0; w < kWords; w += 4)
-                    *reinterpret_cast<uint4 *>(dst + w) = make_uint4(words[w], words[w + 1], words[w + 2], words[w + 3]);
-            } else {
-#pragma unroll
-                for (int w = 0; w < kWords; w += 2) *reinterpret_cast<uint2 *>(dst + w) = make_uint2(words[w], words[w + 1]);
+                for (int w = 0; w < BITS; ++w) dst[w] = words[w];
             }
-            if (half == 0) r.norms[cur.row] = nh;
+            if (part == 0) r.norms[my_row] = nh;
         }
         if constexpr (QJL) {
+            read_rows();  // (again: cheaper than holding them through epilogue 1)
             gemm_wait();
             // ---------------- epilogue 2: the residual against the dtype-rounded reconstruction
             const float nf = tq_half_bits_to_float(nh) * a.unscale2, scale = fit_power(safe) * a.res_scale;
             const uint64_t nf2 = f32x2(nf, nf), scale2 = f32x2(scale, scale);
             uint64_t rs2 = 0;
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                uint32_t y[32];
-                tmem_ld32(my_acc + 32 * q, y);
+            for (int q = 0; q < kCoords / 16; ++q) {
+                uint32_t y[16], hi[8], lo[8];
+                tmem_ld16(my_acc + 16 * q, y);
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t hi[8], lo[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int e = 16 * c + 2 * i;
-                        const uint64_t rec = round_through2<T>(f32x2_mul(f32x2(__uint_as_float(y[e]), __uint_as_float(y[e + 1])), nf2));
-                        const uint64_t res = f32x2_sub(R::pair(raw, 16 * q + 8 * c + i), rec);
-                        rs2 = f32x2_fma(res, res, rs2);
-                        split_half2(f32x2_mul(res, scale2), hi[i], lo[i]);
-                    }
-                    tmem_st8(my_hi + 16 * q + 8 * c, hi), tmem_st8(my_lo + 16 * q + 8 * c, lo);
+                for (int i = 0; i < 8; ++i) {
+                    const uint64_t rec = round_through2<T>(f32x2_mul(f32x2(__uint_as_float(y[2 * i]), __uint_as_float(y[2 * i + 1])), nf2));
+                    const uint64_t res = f32x2_sub(R::pair(raw, 8 * q + i), rec);
+                    rs2 = f32x2_fma(res, res, rs2);
+                    split_half2(f32x2_mul(res, scale2), hi[i], lo[i]);
                 }
+                tmem_st8(my_hi + 8 * q, hi), tmem_st8(my_lo + 8 * q, lo);
             }
             float rs, rs_hi;
             f32x2_split(rs2, rs, rs_hi);
-            sm.rs[group][half][vrow] = rs + rs_hi;
+            sm.rs[group][part][vrow] = rs + rs_hi;
             // ---------------- stage 3: projection, sign bits
-            gemm_issue(2, 2);
-            const float rn = sqrtf(sm.rs[group][0][vrow] + sm.rs[group][1][vrow]);
-            if (more) {  // the residual is stored: fetch the next tile's rows under the MMAs
-                nxt = locate(tile + stride);
-                fetch(nxt);
-            }
+            gemm_issue(1, two_terms, std::false_type());
+            float (*rsq)[kUmmaRows] = sm.rs[group];
+            const float rn = sqrtf((rsq[0][vrow] + rsq[1][vrow]) + (rsq[2][vrow] + rsq[3][vrow]));
+            if (more) request(tile + stride);  // everybody has formed its residual: request the next tile's rows under the MMAs
             gemm_wait();
-            uint32_t sg[2];
+            uint32_t neg = 0;  // sign bits, shifted in from coordinate 31 down to 0; -0 counts as +0
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                uint32_t p[32];
-                tmem_ld32(my_acc + 32 * q, p);
-                uint32_t neg = 0;  // sign bits, shifted in from element 31 down to 0; -0 counts as +0
+            for (int q = kCoords / 16 - 1; q >= 0; --q) {
+                uint32_t p[16];
+                tmem_ld16(my_acc + 16 * q, p);
 #pragma unroll
-                for (int i = 30; i >= 0; i -= 2) {
+                for (int i = 14; i >= 0; i -= 2) {
                     float p0, p1;
                     f32x2_split(f32x2_fma(f32x2(__uint_as_float(p[i]), __uint_as_float(p[i + 1])), f32x2(1.f, 1.f), 0ull), p0, p1);
                     neg = __funnelshift_l(__float_as_uint(p1), neg, 1);
                     neg = __funnelshift_l(__float_as_uint(p0), neg, 1);
                 }
-                sg[q] = rn < INFINITY ? ~neg : 0u;  // (an infinite or undefined residual makes every projection undefined)
             }
-            if (cur.valid) {
-                *reinterpret_cast<uint2 *>(a.signs + cur.row * 16 + 8 * half) = make_uint2(sg[0], sg[1]);
-                if (half == 0) a.rnorms[cur.row] = tq_float_to_half_bits(rn > 0.f ? rn : 1.f);
+            if (my_row >= 0) {  // (an infinite or undefined residual makes every projection undefined: no bit is set)
+                reinterpret_cast<uint32_t *>(a.signs + my_row * 16)[part] = rn < INFINITY ? ~neg : 0u;
+                if (part == 0) a.rnorms[my_row] = tq_float_to_half_bits(rn > 0.f ? rn : 1.f);
             }
         }
-        cur = nxt;
     }
     if (timed_out) atomicExch(a.error_flag, 3);
 }
@@ -412,6 +463,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq_pack_tc_kernel(const __grid_co
     extern __shared__ uint8_t smem_raw[];
     __shared__ PackTcShared sm;
     const uint32_t images = (smem_u32(smem_raw) + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
+    const uint32_t staged = images + (QJL ? 2 : 1) * kUmmaImageBytes;
     const int tid = threadIdx.x, warp = tid >> 5;
     const bool keys = (int)blockIdx.x < a.key_ctas;
     const PackTcRole &r = a.role[keys ? 0 : 1];
@@ -428,21 +480,25 @@ __global__ void __launch_bounds__(kThreads, 1) tq_pack_tc_kernel(const __grid_co
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
     if (tid == 0) {
-        for (int i = 0; i < 3; ++i) mbar_init(smem_u32(&sm.bar_image[i]), 1);
-        for (int i = 0; i < kGroups; ++i) mbar_init(smem_u32(&sm.bar_mma[i]), 1);
+        for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&sm.bar_image[i]), 1);
+        for (int i = 0; i < kGroups; ++i) mbar_init(smem_u32(&sm.bar_mma[i]), 1), mbar_init(smem_u32(&sm.bar_rows[i]), kUmmaRows);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         umma_load_image(images, r.image, smem_u32(&sm.bar_image[0]));  // (every CTA has at least one tile)
-        if (QJL && keys) {
-            umma_load_image(images + kUmmaImageBytes, a.image2, smem_u32(&sm.bar_image[1]));
-            umma_load_image(images + 2 * kUmmaImageBytes, a.image3, smem_u32(&sm.bar_image[2]));
-        }
+        if (QJL && keys) umma_load_image(images + kUmmaImageBytes, a.image_s, smem_u32(&sm.bar_image[1]));
     }
     umma_fence_before();
     __syncthreads();
     umma_fence_after();
-    if (keys) encode<T, KEY_BITS, QJL>(a, r, sm, images, blockIdx.x, a.key_ctas);
-    else encode<T, BITS, false>(a, r, sm, images, blockIdx.x - a.key_ctas, gridDim.x - a.key_ctas);
+    {
+        const int bits = keys ? KEY_BITS : BITS;
+        if (bits > 2) {
+            build_cells(sm.cells, sm.bounds, (1 << bits) - 1, r.grid, QJL && keys ? 4 : 1);
+            __syncthreads();
+        }
+    }
+    if (keys) encode<T, KEY_BITS, QJL>(a, r, sm, images, staged, blockIdx.x, a.key_ctas);
+    else encode<T, BITS, false>(a, r, sm, images, staged, blockIdx.x - a.key_ctas, gridDim.x - a.key_ctas);
     umma_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -458,6 +514,29 @@ float tq_fit_power(float largest) {
     int e;
     frexpf(largest, &e);  // largest < 2^e
     return ldexpf(1.f, e < -100 ? 114 : e > 100 ? -86 : 14 - e);
+}
+
+// A uniform grid over n boundaries with at most one of them in any cell: see Search.  Its cells are formed by the
+// operations the kernel uses (fma rounds once on both sides), the clamp to [0, 1] included.
+bool tq_fit_grid(const float *bounds, int n, tq_ctx::Grid *g) {
+    for (int i = 0; i < n; ++i)
+        if (!isfinite(bounds[i]) || (i && !(bounds[i - 1] < bounds[i]))) return false;
+    for (int cells = 32; cells <= kMaxCells; cells *= 2) {
+        const float width = bounds[n - 1] - bounds[0];
+        g->last = (float)(cells - 1);
+        g->scale = width > 0.f ? (1.f - 2.f / cells) / width : 1.f;
+        g->shift = 1.f / cells - bounds[0] * g->scale;
+        if (!isfinite(g->scale) || !isfinite(g->shift)) return false;
+        bool single = true;
+        float before = -1.f;
+        for (int i = 0; i < n && single; ++i) {
+            const float t = fminf(fmaxf(fmaf(bounds[i], g->scale, g->shift), 0.f), 1.f), at = fmaf(t, g->last, 8388608.f);
+            single = at != before;
+            before = at;
+        }
+        if (single) return true;
+    }
+    return false;
 }
 
 // Host: the 64 KB shared-memory image of a [128 x 128] K-major operand `m[row][k]`, times a power of two, in
@@ -479,13 +558,12 @@ float tq_build_operand_image(const float *m, uint16_t *image) {
 
 template <typename T, int BITS, bool QJL>
 static cudaError_t launch_tc(const PackTcArgs &a, int grid, int device, cudaStream_t stream) {
-    const int smem = (QJL && a.key_ctas ? 3 : 1) * kUmmaImageBytes + 1024;
+    constexpr int smem = (QJL ? 2 : 1) * kUmmaImageBytes + (sizeof(T) == 2 ? kGroups * kStageBytes : 0) + 1024;
     // the attribute belongs to the (kernel, device) pair: one flag per device of this instantiation
     static bool configured[TQ_MAX_DEVICES] = {};
     if (device < 0 || device >= TQ_MAX_DEVICES) return cudaErrorInvalidDevice;
     if (!configured[device]) {
-        cudaError_t e = cudaFuncSetAttribute(tq_pack_tc_kernel<T, BITS, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (QJL ? 3 : 1) * kUmmaImageBytes + 1024);
+        cudaError_t e = cudaFuncSetAttribute(tq_pack_tc_kernel<T, BITS, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         configured[device] = true;
     }
@@ -506,20 +584,21 @@ int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_de
         const tq_ctx::Image &image = i == 0 ? ctx->img_rot_k : ctx->img_rot_v;
         r.x = x->data, r.sb = x->stride_b, r.sh = x->stride_h, r.st = x->stride_t;
         r.codes = i == 0 ? cache->k_codes : cache->v_codes, r.norms = i == 0 ? cache->k_norms : cache->v_norms;
-        r.image = image.data, r.unscale = image.unscale;
+        r.image = image.data, r.unscale = kUmmaRestore * image.unscale;
         r.bounds = i == 0 ? ctx->bounds_k : ctx->bounds_v;
+        r.grid = i == 0 ? ctx->grid_k : ctx->grid_v;
+        if ((i == 0 ? ctx->key_bits : ctx->bits) > 2 && r.grid.last == 0.f) return TQ_ERR_UNSUPPORTED;  // (boundaries too close)
     }
     const bool qjl = ctx->use_qjl && k;
-    a.B = cache->batch, a.H = cache->kv_heads, a.S = n_tokens, a.pos0 = pos0;
+    a.vec = vector_index(cache->batch, cache->kv_heads, n_tokens), a.pos0 = pos0;
     a.cache_sb = cache->stride_b, a.cache_sh = cache->stride_h;
     a.error_flag = ctx->error_flag;
-    a.image2 = ctx->img_rot_kt.data, a.image3 = ctx->img_qjl.data;
-    a.unscale2 = ctx->img_rot_kt.unscale / ctx->cen_k_scale;
+    a.image_s = ctx->img_qjl.data;
+    a.unscale2 = kUmmaRestore * ctx->img_rot_k.unscale / ctx->cen_k_scale;
     a.cen_scale = ctx->cen_k_scale, a.res_scale = ctx->res_scale;
     a.centers = ctx->centers_k;
     a.signs = cache->k_signs, a.rnorms = cache->k_rnorms;
-    const int64_t n_vec = (int64_t)a.B * a.H * a.S;
-    a.n_tiles = (int)((n_vec + kUmmaRows - 1) / kUmmaRows);
+    a.n_tiles = (int)((a.vec.n + kUmmaRows - 1) / kUmmaRows);
     // One CTA per SM.  With tiles enough for all of them, keys with the sketch get the share of the SMs that
     // their cost asks for; with few tiles each side gets a CTA per tile.
     const int sms = ctx->sm_count;
