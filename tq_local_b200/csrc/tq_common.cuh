@@ -80,17 +80,29 @@ struct TqRange {
 
 // Kernel launch with the optional "programmatic stream serialization" attribute: the kernel may
 // start while the preceding kernel of the stream is still running and must call
-// griddepcontrol.wait before it touches anything that kernel writes.
+// griddepcontrol.wait before it touches anything that kernel writes.  `cluster` > 1: CTAs per cluster (along x).
+template <typename... KArgs, typename... Args>
+cudaError_t tq_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              bool programmatic, int cluster, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    if (programmatic) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1, ++cfg.numAttrs;
+    }
+    cfg.attrs = attr;
+    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
 template <typename... KArgs, typename... Args>
 cudaError_t tq_launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                              bool programmatic, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr, cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+    return tq_launch_cluster(kernel, grid, block, smem, stream, programmatic, 1, args...);
 }
 
 template <typename T> __device__ __forceinline__ float tq_to_float(T x);

@@ -4,6 +4,7 @@
 //
 //   logit[n] = (1/sqrt(D)) * ( |k_n| * <q R_k^T, c_k[idx_n]> + sqrt(pi/2)/D * |r_n| * <q S^T, sign_n> )
 //   out      = ( sum_n softmax(logit)_n * |v_n| * c_v[idx_n] ) @ R_v
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include "tq_common.cuh"
@@ -341,16 +342,18 @@ template <typename T> __device__ __forceinline__ void tq_load8(const T *p, bool 
 // values: sixteen threads cover a row with 16-byte loads and 32 rows are read side by side.
 // Returns this thread's element (head threadIdx.x / 128, column threadIdx.x % 128) of the
 // unnormalised sum; the maximum and the sum of every head are left in s_tm / s_tl.
-// What bounds it is the latency of two dependent trips to memory per 256 tokens.  The whole kernel for
-// a tail of 300 tokens, 8 KV rows: 17 us; one thread per output column walking the tail alone: 59 us.
+// What bounds it is the latency of two dependent trips to memory per 256 tokens; the row's tail is shared
+// out over the CTAs of a cluster (tq_merge_tails).
 constexpr int kTailChunk = 256;
+constexpr int kTailTokensPerCta = 64;  // one pass of the logit loop; a CTA takes more only when all of them are used
+constexpr int kTailCtas = 4;           // CTAs of a cluster
 struct TailShared {
     float p[4][kTailChunk];
     float corr[4], m[4], l[4];
     float acc[16][4][TQ_D];
 };
 template <typename T>
-__device__ __forceinline__ float tq_attend_tail(const CombineArgs &a, TailShared &sm, int64_t R, int h0, int n_heads) {
+__device__ __forceinline__ float tq_attend_tail(const CombineArgs &a, TailShared &sm, int64_t R, int h0, int n_heads, int t_begin, int t_end) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t row0 = R * a.G + h0;
     const int b = (int)(row0 / a.Hq), hkv = (int)(row0 % a.Hq) / a.G;
@@ -373,8 +376,8 @@ __device__ __forceinline__ float tq_attend_tail(const CombineArgs &a, TailShared
         for (int i = 0; i < 8; ++i) q[g][i] = lo[i], q[g][8 + i] = hi[i];
     }
     float m_run = -INFINITY, l_run = 0.f;  // warp g < 4: head g
-    for (int c0 = 0; c0 < a.n_tail; c0 += kTailChunk) {
-        const int n = min(kTailChunk, a.n_tail - c0);
+    for (int c0 = t_begin; c0 < t_end; c0 += kTailChunk) {
+        const int n = min(kTailChunk, t_end - c0);
 #pragma unroll
         for (int it = 0; it < kTailChunk / 64; ++it) {
             const int t = 64 * it + 4 * warp + (lane >> 3);
@@ -449,26 +452,55 @@ __device__ __forceinline__ float tq_attend_tail(const CombineArgs &a, TailShared
     return o;
 }
 
+// The tails of a cluster's CTAs (each attended its share of the row's tail tokens) merged in its first CTA;
+// returns false in the others, which have nothing left to do.  `o` is the caller's element of its own share.
+__device__ __forceinline__ bool tq_merge_tails(TailShared &sm, float &o, float &m, float &l) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, g = tid >> 7, n = (int)cluster.num_blocks();
+    m = sm.m[g], l = sm.l[g];
+    if (n == 1) return true;
+    (&sm.acc[0][0][0])[tid] = o;  // (a thread reads the sum of its own element alone, so nobody else's is overwritten early)
+    cluster.sync();
+    if (cluster.block_rank() == 0) {
+        for (int r = 1; r < n; ++r) {
+            const TailShared &peer = *cluster.map_shared_rank(&sm, r);
+            const float pm = peer.m[g], pl = peer.l[g], po = (&peer.acc[0][0][0])[tid];
+            const float M = fmaxf(m, pm), w = expf(m - M), pw = expf(pm - M);  // (every share holds at least one token)
+            o = o * w + po * pw, l = l * w + pl * pw, m = M;
+        }
+    }
+    cluster.sync();
+    return cluster.block_rank() == 0;
+}
+
 // Split combine for up to four heads of one (batch, KV head) row per block: the un-rotation
-// matrix is read once for the G heads, and the un-quantised tail of the row, if there is one
-// (TAIL), is attended by the same block.
+// matrix is read once for the G heads.  An un-quantised tail of the row, if there is one (TAIL), is
+// attended by a cluster of CTAs before the splits are waited for: the decode kernel
+// releases this one as soon as the query and the tail are known to be there, so the tail is attended on
+// SMs that the decode kernel leaves free.  12001 packed + 300 dense tokens, 8 KV rows, launches recorded: 17.0 us
+// from query preparation to output; 28.2 us with one block per four heads that began after the decode kernel.
+// Four CTAs and not eight: a cluster's CTAs need free SMs of one GPC at the same time.
 template <typename T, bool TAIL>
 __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs a) {
     __shared__ __align__(16) float s_o[4][TQ_D];
     __shared__ float s_part[4][4][TQ_D];  // [quarter of d][head][column]
     __shared__ float s_L[4], s_M[4];
-    const int groups = (a.G + 3) >> 2;           // a block serves up to four heads of a KV row
-    const int64_t R = blockIdx.x / groups;
-    const int h0 = 4 * (blockIdx.x % groups);
+    const int groups = (a.G + 3) >> 2;           // a block (TAIL: a cluster) serves up to four heads of a KV row
+    const unsigned blk = TAIL ? blockIdx.x / (unsigned)a.tail_ctas : blockIdx.x;
+    const int64_t R = blk / groups;
+    const int h0 = 4 * (blk % groups);
     const int n_heads = a.G - h0 < 4 ? a.G - h0 : 4;
     const int tid = threadIdx.x, e = tid & (TQ_D - 1), dq = tid >> 7, lane = tid & 31;
     float tail_o = 0.f, tail_m = -INFINITY, tail_l = 0.f;  // of head dq, column e
     if (TAIL) {
         extern __shared__ __align__(16) uint8_t s_dyn[];
         TailShared &ts = *reinterpret_cast<TailShared *>(s_dyn);
-        tq_grid_dependency_wait();  // (the query and the tail may come from any earlier kernel of the stream)
-        tail_o = tq_attend_tail<T>(a, ts, R, h0, n_heads);
-        tail_m = ts.m[dq], tail_l = ts.l[dq];
+        // (no wait here: the kernel before this one releases it after its own dependency wait, when everything
+        // ordered before the query preparation - the query and the tail among it - has completed)
+        const int rank = (int)(blockIdx.x % (unsigned)a.tail_ctas), t0 = rank * a.tail_per_cta;
+        tail_o = tq_attend_tail<T>(a, ts, R, h0, n_heads, t0, min(a.n_tail, t0 + a.tail_per_cta));
+        if (!tq_merge_tails(ts, tail_o, tail_m, tail_l)) return;
     }
     float rv[32];  // this thread's un-rotation elements, fetched while the decode kernel drains
     tq_load_column(rv, a.rot_v, dq, e);
@@ -734,7 +766,8 @@ template <typename T>
 static cudaError_t launch_combine(const CombineArgs &a, dim3 grid, cudaStream_t stream, bool programmatic) {
     if (a.n_tail == 0)
         return tq_launch_kernel(tq_combine_group_kernel<T, false>, grid, dim3(4 * TQ_D), 0, stream, programmatic, a);
-    return tq_launch_kernel(tq_combine_group_kernel<T, true>, grid, dim3(4 * TQ_D), sizeof(TailShared), stream, programmatic, a);
+    return tq_launch_cluster(tq_combine_group_kernel<T, true>, dim3(grid.x * a.tail_ctas), dim3(4 * TQ_D), sizeof(TailShared),
+                             stream, programmatic, a.tail_ctas, a);
 }
 
 int32_t tq_launch_combine(const CombineArgs &a, int32_t q_dtype, int64_t rows, cudaStream_t stream, bool programmatic) {
@@ -751,10 +784,14 @@ int32_t tq_launch_combine(const CombineArgs &a, int32_t q_dtype, int64_t rows, c
 
 // The tail fields of the combine arguments: `tail_vec` when every row of both tensors starts on a 16-byte boundary.
 int32_t tq_set_combine_tail(CombineArgs &c, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tail, int32_t q_dtype) {
-    c.n_tail = n_tail, c.tail_k = c.tail_v = nullptr, c.tail_vec = false;
+    c.n_tail = n_tail, c.tail_k = c.tail_v = nullptr, c.tail_vec = false, c.tail_ctas = 0, c.tail_per_cta = 0;
     c.tk_sb = c.tk_sh = c.tk_st = c.tv_sb = c.tv_sh = c.tv_st = 0;
     if (n_tail == 0) return TQ_OK;
     if (k->dtype != q_dtype || v->dtype != q_dtype) return TQ_ERR_ARG;
+    // as many CTAs as there are passes of 64 tokens, kTailCtas at most; none of them empty
+    const int passes = (n_tail + kTailTokensPerCta - 1) / kTailTokensPerCta, ctas = passes < kTailCtas ? passes : kTailCtas;
+    c.tail_per_cta = (n_tail + ctas - 1) / ctas;
+    c.tail_ctas = (n_tail + c.tail_per_cta - 1) / c.tail_per_cta;
     c.tail_k = k->data, c.tail_v = v->data;
     c.tk_sb = k->stride_b, c.tk_sh = k->stride_h, c.tk_st = k->stride_t;
     c.tv_sb = v->stride_b, c.tv_sh = v->stride_h, c.tv_st = v->stride_t;

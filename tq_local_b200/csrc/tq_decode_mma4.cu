@@ -93,6 +93,7 @@ struct Mma4Args {
     float *part_m, *part_l, *part_acc;
     const float *centers_k, *centers_v;
     int *error_flag;  // set to 1 when a bounded wait ran out
+    bool release_early;  // let the combine kernel start once this kernel's dependencies are met (it attends a dense tail)
     int device;       // host side only: the context's device
 };
 
@@ -360,6 +361,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
     const int n_first = min(n_iter, kStages);
     if (first_segment) {
         tq_grid_dependency_wait();
+        if (a.release_early) tq_launch_dependents();
         TQ_STAMP(2);
         for (int it = 0; it < n_first; ++it)
             if (deferred >> it & 1) issue(sg, it);  // (only the issuing lane has bits set)
@@ -715,6 +717,7 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
     a.part_m = w.part_m, a.part_l = w.part_l, a.part_acc = w.part_acc;
     a.centers_k = ctx->centers_k, a.centers_v = ctx->centers_v;
     a.error_flag = ctx->error_flag;
+    a.release_early = n_tail > 0;
     a.device = ctx->device;
     // Length on the device: the kernel plans for its own grid.  One CTA per SM, except that a
     // single partial per row (n_splits == 1) means one CTA per row, however many rows there are.

@@ -36,6 +36,7 @@ struct CombineArgs {
     const void *tail_k, *tail_v;
     int64_t tk_sb, tk_sh, tk_st, tv_sb, tv_sh, tv_st;
     bool tail_vec;  // every tail row starts on a 16-byte boundary
+    int tail_ctas, tail_per_cta;  // CTAs of a cluster that share a row's tail, and how many tokens each takes
 };
 
 // Carved view of the caller's scratch buffer (see tq_decode_workspace_bytes).
