@@ -39,6 +39,7 @@ class PackedStore:
         self._alloc(max(8, _round_up(int(capacity), 8)))
         self._workspace: torch.Tensor | None = None
         self._step_plan = None
+        self._attn_plan = None  # (what it depends on, split count, scratch bytes) of the last decode_attn
 
     # ------------------------------------------------------------------ storage
     def _alloc(self, capacity: int) -> None:
@@ -100,6 +101,19 @@ class PackedStore:
     def _stream_ptr(self):
         return C.c_void_p(torch.cuda.current_stream(self.codec.device).cuda_stream)
 
+    def _call(self, name: str, *args) -> None:
+        """Library call on the current stream of the store's device.  (Entering the device costs as much as the call's
+        other host work, so a device that is current already is left alone.)"""
+        dev = self.codec.device
+        fn = getattr(ffi.lib(), name)
+        if torch.cuda.current_device() == dev.index:
+            rc = fn(*args, torch.cuda.current_stream(dev).cuda_stream)
+        else:
+            with torch.cuda.device(dev):
+                rc = fn(*args, torch.cuda.current_stream(dev).cuda_stream)
+        if rc:
+            ffi.check(rc, name)
+
     def pack(self, k: torch.Tensor, v: torch.Tensor) -> None:
         """Quantise ``k``/``v`` [B, Hkv, T, 128] and append them at the current length."""
         if k.shape != v.shape or k.dtype != v.dtype:
@@ -117,9 +131,7 @@ class PackedStore:
             v = v.contiguous()
         self.reserve(self.length + n)
         kd, vd = dense_desc(k), dense_desc(v)
-        with torch.cuda.device(self.codec.device):
-            ffi.check(ffi.lib().tq_pack(self.codec.handle, C.byref(kd), C.byref(vd), n, C.byref(self._desc),
-                                        self.length, self._stream_ptr()), "tq_pack")
+        self._call("tq_pack", self.codec.handle, C.byref(kd), C.byref(vd), n, self._desc_ref, self.length)
         self.length += n
 
     def pack_rows(self, k: torch.Tensor, v: torch.Tensor, b0: int, pos0: int = 0) -> None:
@@ -165,9 +177,7 @@ class PackedStore:
         b, hq = int(q.shape[0]), int(q.shape[1])
         if q.shape[-1] != 128 or q.numel() != b * hq * 128 or b != self.batch:
             raise ValueError(f"expected a single-token query [B={self.batch}, Hq, 1, 128], got {tuple(q.shape)}")
-        qc = q.reshape(b, hq, 128)
-        if not qc.is_contiguous():
-            qc = qc.contiguous()
+        qc = q if q.is_contiguous() else q.contiguous()
         n = self.length if seq_len is None else int(seq_len)
         n_tail = 0 if tail_k is None else int(tail_k.shape[2])
         if n_tail:
@@ -175,15 +185,19 @@ class PackedStore:
             tk_ref, tv_ref = C.byref(tkd), C.byref(tvd)
         else:
             tk_ref = tv_ref = None
-        splits = self.suggest_splits(n) if splits is None else int(splits)
-        ws = self._get_workspace(hq, splits)
+        # the split count and the scratch size only change when the length crosses a kernel step
+        key = (hq, splits, (n + 511) >> 9)
+        if self._attn_plan is None or self._attn_plan[0] != key:
+            splits = self.suggest_splits(n) if splits is None else int(splits)
+            self._attn_plan = (key, splits, int(ffi.lib().tq_decode_workspace_bytes(b, hq, splits)))
+        _, splits, need = self._attn_plan
+        ws = self._workspace
+        if ws is None or ws.numel() < need:
+            ws = self._get_workspace(hq, splits)
         if out is None:
             out = torch.empty(b, hq, 1, 128, dtype=q.dtype, device=q.device)
-        with torch.cuda.device(self.codec.device):
-            ffi.check(ffi.lib().tq_decode_attn(self.codec.handle, qc.data_ptr(), tq_dtype(q.dtype), hq,
-                                               C.byref(self._desc), n, tk_ref, tv_ref, n_tail, splits,
-                                               ws.data_ptr(), ws.numel(), out.data_ptr(), self._stream_ptr()),
-                      "tq_decode_attn")
+        self._call("tq_decode_attn", self.codec.handle, qc.data_ptr(), tq_dtype(q.dtype), hq, self._desc_ref, n, tk_ref,
+                   tv_ref, n_tail, splits, ws.data_ptr(), ws.numel(), out.data_ptr())
         return out
 
     def decode_attn_f32(self, q: torch.Tensor, *, seq_len: int | None = None, splits: int | None = None) -> torch.Tensor:
@@ -403,9 +417,7 @@ class PackedStore:
         out = torch.empty(self.batch, self.kv_heads, n, 128, dtype=dtype, device=self.codec.device)
         if n > 0:
             od = dense_desc(out)
-            with torch.cuda.device(self.codec.device):
-                ffi.check(ffi.lib().tq_dequant(self.codec.handle, C.byref(self._desc), 0 if which == "keys" else 1,
-                                               lo, n, C.byref(od), self._stream_ptr()), "tq_dequant")
+            self._call("tq_dequant", self.codec.handle, self._desc_ref, 0 if which == "keys" else 1, lo, n, C.byref(od))
         return out
 
 
