@@ -504,18 +504,17 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
     }
     float rv[32];  // this thread's un-rotation elements, fetched while the decode kernel drains
     tq_load_column(rv, a.rot_v, dq, e);
-    tq_grid_dependency_wait();
+    // (the length was there before the query preparation began, and the decode kernel has planned with it)
     int n_valid = a.n_splits;
-    int seg_chunk = a.seg_chunk, seg_npad = a.seg_npad;
-    if (a.len_ptr) {
-        const TqPlan plan = tq_make_plan(min(*a.len_ptr + a.len_add, a.capacity), a.plan_rows, a.plan_ctas, a.n_splits,
-                                         a.plan_step);
-        seg_chunk = plan.chunk, seg_npad = plan.n_pad;
+    TqPlan plan = {a.seg_npad, a.seg_chunk};
+    if (a.len_ptr) plan = tq_make_plan(min(*a.len_ptr + a.len_add, a.capacity), a.plan_rows, a.plan_ctas, a.n_splits, a.plan_step);
+    if (plan.chunk > 0) {
+        const int64_t lo = R * (int64_t)plan.n_pad, hi = lo + plan.n_pad - 1;
+        n_valid = 1 + (hi <= 0x7fffffff ? (int)((unsigned)hi / (unsigned)plan.chunk - (unsigned)lo / (unsigned)plan.chunk)
+                                        : (int)(hi / plan.chunk - lo / plan.chunk));
+        if (!TAIL && a.next_blocks && tq_leaves_idle(plan, a.plan_rows, a.sm_count, a.next_blocks)) tq_launch_dependents();
     }
-    if (seg_chunk > 0) {
-        const int64_t lo = R * (int64_t)seg_npad;
-        n_valid = (int)((lo + seg_npad - 1) / seg_chunk - lo / seg_chunk) + 1;
-    }
+    tq_grid_dependency_wait();
     {   // thread (e, dq) merges the splits of head dq, 32 at a time: lane s of each warp holds split s's
         // maximum and weight, the accumulator columns are requested eight splits at a time.  (The kernel
         // takes 5.6 us for 33 splits of 4 rows; with one thread walking all splits twice it took 10.8.)
@@ -890,6 +889,7 @@ int32_t tq_launch_decode_exact(tq_ctx *ctx, const void *q, int32_t q_dtype, int3
     c.n_splits = n_splits, c.Hq = q_heads, c.G = a.G;
     c.seg_chunk = 0, c.seg_npad = 0;
     c.len_ptr = nullptr, c.len_add = 0, c.capacity = 0, c.plan_rows = 0, c.plan_ctas = 0, c.plan_step = 0;
+    c.sm_count = 0, c.next_blocks = 0;
     c.gather_world = 0, c.parts = 0, c.part = 0, c.head_group = 0, c.exch_rows = 0;
     c.rot_v = ctx->rot_v;
     c.q = q, c.out = out, c.out_f32 = nullptr;

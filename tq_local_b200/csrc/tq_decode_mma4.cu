@@ -93,7 +93,10 @@ struct Mma4Args {
     float *part_m, *part_l, *part_acc;
     const float *centers_k, *centers_v;
     int *error_flag;  // set to 1 when a bounded wait ran out
-    bool release_early;  // let the combine kernel start once this kernel's dependencies are met (it attends a dense tail)
+    // Let the combine kernel start once this kernel's dependencies are met: it attends a dense tail, or there are idle SMs
+    // for it (see CombineArgs::next_blocks).  1 x 8 x 4099 tokens: 9 / 10 us of a step's 15.7 us chain remain.
+    bool has_tail;
+    int sm_count, next_blocks;
     int device;       // host side only: the context's device
 };
 
@@ -229,6 +232,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
         n_pad = plan.n_pad, chunk = plan.chunk;
     }
 
+    const bool release_early = a.has_tail || (a.next_blocks && tq_leaves_idle({n_pad, chunk}, a.rows, a.sm_count, a.next_blocks));
+
     // ---- this CTA's contiguous piece of the flattened (row, token) space
     const int64_t flat_begin = (int64_t)blockIdx.x * chunk;
     const int64_t flat_end = min(flat_begin + chunk, (int64_t)a.rows * n_pad);
@@ -361,7 +366,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
     const int n_first = min(n_iter, kStages);
     if (first_segment) {
         tq_grid_dependency_wait();
-        if (a.release_early) tq_launch_dependents();
+        if (release_early) tq_launch_dependents();
         TQ_STAMP(2);
         for (int it = 0; it < n_first; ++it)
             if (deferred >> it & 1) issue(sg, it);  // (only the issuing lane has bits set)
@@ -717,7 +722,11 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
     a.part_m = w.part_m, a.part_l = w.part_l, a.part_acc = w.part_acc;
     a.centers_k = ctx->centers_k, a.centers_v = ctx->centers_v;
     a.error_flag = ctx->error_flag;
-    a.release_early = n_tail > 0;
+    a.has_tail = n_tail > 0;
+    // (the wait for the peers that follows a gather is not one of the small kernels meant here)
+    const int combine_blocks = a.rows * ((a.G + 3) / 4);
+    const int prologue_blocks = combine_blocks * (ctx->use_qjl ? 2 : 1) + (append ? append->n_kinds * append->B * append->H * append->S : 0);
+    a.sm_count = ctx->sm_count, a.next_blocks = gather || n_tail ? 0 : combine_blocks + (prologue_blocks + 1) / 2;
     a.device = ctx->device;
     // Length on the device: the kernel plans for its own grid.  One CTA per SM, except that a
     // single partial per row (n_splits == 1) means one CTA per row, however many rows there are.
@@ -745,6 +754,7 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
     c.seg_chunk = a.chunk, c.seg_npad = a.n_pad;
     c.len_ptr = len_ptr, c.len_add = a.len_add, c.capacity = a.capacity;
     c.plan_rows = a.rows, c.plan_ctas = (int)grid.x, c.plan_step = step;
+    c.sm_count = a.sm_count, c.next_blocks = a.next_blocks;
     c.gather_world = 0, c.parts = 0, c.part = 0, c.head_group = 0, c.exch_rows = 0;
     if (gather && extras->parts > 0) {
         c.parts = extras->parts, c.part = gather->rank % extras->parts, c.head_group = gather->rank / extras->parts;

@@ -54,17 +54,29 @@ struct TqPlan {
 };
 __host__ __device__ inline TqPlan tq_make_plan(int seq_len, int rows, int n_ctas, int n_splits, int step) {
     TqPlan p;
-    p.n_pad = (seq_len + step - 1) / step * step;
+    if (seq_len < 0) seq_len = 0;
+    p.n_pad = (int)(((unsigned)seq_len + (unsigned)step - 1u) / (unsigned)step) * step;
     const long long total = (long long)rows * p.n_pad;
-    long long chunk = ((total + n_ctas - 1) / n_ctas + step - 1) / step * step;
+    long long chunk;
+    if (total <= 0x7fff0000ll)  // (32-bit divisions are several times cheaper, and the kernels plan on their critical path)
+        chunk = ((unsigned)total + (unsigned)n_ctas - 1u) / (unsigned)n_ctas;
+    else
+        chunk = (total + n_ctas - 1) / n_ctas;
+    chunk = (long long)(((unsigned)chunk + (unsigned)step - 1u) / (unsigned)step) * step;
     if (n_splits == 1) {
         chunk = p.n_pad;
     } else {
-        const long long floor_chunk = ((p.n_pad + n_splits - 2) / (n_splits - 1) + step - 1) / step * step;
+        const unsigned per_split = ((unsigned)p.n_pad + (unsigned)n_splits - 2u) / (unsigned)(n_splits - 1);
+        const long long floor_chunk = (long long)((per_split + (unsigned)step - 1u) / (unsigned)step) * step;
         if (chunk < floor_chunk) chunk = floor_chunk;
     }
     p.chunk = (int)chunk;
     return p;
+}
+// Whether the decode kernel's CTAs leave `blocks` SMs idle, so that the small kernels after it may be placed while it
+// runs (see CombineArgs::next_blocks).
+__host__ __device__ inline bool tq_leaves_idle(const TqPlan &p, int rows, int sm_count, int blocks) {
+    return (long long)(sm_count - blocks) * p.chunk >= (long long)rows * p.n_pad;
 }
 
 void tq_fill_pack_args(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tokens,
