@@ -105,6 +105,16 @@ cudaError_t tq_launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     return tq_launch_cluster(kernel, grid, block, smem, stream, programmatic, 1, args...);
 }
 
+// Lets a kernel use `smem` bytes of dynamic shared memory (an attribute of the kernel on one device: set once).
+template <auto KERNEL> cudaError_t tq_allow_shared(int device, int smem) {
+    static bool configured[TQ_MAX_DEVICES] = {};
+    if (device < 0 || device >= TQ_MAX_DEVICES) return cudaErrorInvalidDevice;
+    if (configured[device]) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    configured[device] = e == cudaSuccess;
+    return e;
+}
+
 template <typename T> __device__ __forceinline__ float tq_to_float(T x);
 template <> __device__ __forceinline__ float tq_to_float<float>(float x) { return x; }
 template <> __device__ __forceinline__ float tq_to_float<__half>(__half x) { return __half2float(x); }

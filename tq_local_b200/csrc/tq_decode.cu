@@ -297,12 +297,12 @@ __global__ void __launch_bounds__(4 * TQ_D, 2) tq_qprep_frag_kernel(TqQprepArgs 
 
 // The whole latency-bound front of a decode step in one launch: query preparation blocks
 // first, then one block per new key and value vector to append (tq_pack_small_block).
-template <typename T, bool QJL>
-__global__ void __launch_bounds__(4 * TQ_D, 2) tq_step_prologue_kernel(TqQprepArgs qa, TqPackArgs pa, int n_qprep) {
+template <typename T, bool QJL, bool STAGED>
+__global__ void __launch_bounds__(4 * TQ_D, STAGED ? 1 : 2) tq_step_prologue_kernel(TqQprepArgs qa, TqPackArgs pa, int n_qprep) {
     if ((int)blockIdx.x < n_qprep)
         tq_qprep_block<T>(qa, blockIdx.x);
     else
-        tq_pack_small_block<T, QJL>(pa, (int64_t)blockIdx.x - n_qprep);
+        tq_pack_small_block<T, QJL, STAGED>(pa, (int64_t)blockIdx.x - n_qprep);
 }
 
 // Publishing rows to the peers and waiting for theirs (system scope, PTX memory model):
@@ -708,12 +708,15 @@ static void configure_small_kernels() {
     prefer_max_shared(tq_combine_group_kernel<float, true>);
     prefer_max_shared(tq_combine_group_kernel<__half, true>);
     prefer_max_shared(tq_combine_group_kernel<__nv_bfloat16, true>);
-    prefer_max_shared(tq_step_prologue_kernel<float, true>);
-    prefer_max_shared(tq_step_prologue_kernel<float, false>);
-    prefer_max_shared(tq_step_prologue_kernel<__half, true>);
-    prefer_max_shared(tq_step_prologue_kernel<__half, false>);
-    prefer_max_shared(tq_step_prologue_kernel<__nv_bfloat16, true>);
-    prefer_max_shared(tq_step_prologue_kernel<__nv_bfloat16, false>);
+    prefer_max_shared(tq_step_prologue_kernel<float, true, true>);
+    prefer_max_shared(tq_step_prologue_kernel<float, true, false>);
+    prefer_max_shared(tq_step_prologue_kernel<float, false, false>);
+    prefer_max_shared(tq_step_prologue_kernel<__half, true, true>);
+    prefer_max_shared(tq_step_prologue_kernel<__half, true, false>);
+    prefer_max_shared(tq_step_prologue_kernel<__half, false, false>);
+    prefer_max_shared(tq_step_prologue_kernel<__nv_bfloat16, true, true>);
+    prefer_max_shared(tq_step_prologue_kernel<__nv_bfloat16, true, false>);
+    prefer_max_shared(tq_step_prologue_kernel<__nv_bfloat16, false, false>);
 }
 
 template <typename T>
@@ -739,11 +742,13 @@ static cudaError_t launch_prologue(tq_ctx *ctx, const TqQprepArgs &qa, const TqP
     const int n_qprep = (int)qa.kv_rows * ((qa.G + 3) / 4) * (qa.use_qjl ? 2 : 1);
     if (!append) return tq_launch_kernel(tq_qprep_frag_kernel<T>, dim3(n_qprep), dim3(4 * TQ_D), 0, stream, true, qa);
     const int n_pack = append->n_kinds * append->B * append->H * append->S;
-    if (ctx->use_qjl)
-        return tq_launch_kernel(tq_step_prologue_kernel<T, true>, dim3(n_qprep + n_pack), dim3(4 * TQ_D), 0, stream,
-                                true, qa, *append, n_qprep);
-    return tq_launch_kernel(tq_step_prologue_kernel<T, false>, dim3(n_qprep + n_pack), dim3(4 * TQ_D), 0, stream, true,
-                            qa, *append, n_qprep);
+    const dim3 grid(n_qprep + n_pack), block(4 * TQ_D);
+    if (!ctx->use_qjl) return tq_launch_kernel(tq_step_prologue_kernel<T, false, false>, grid, block, 0, stream, true, qa, *append, n_qprep);
+    if (!tq_stages_matrices(ctx, n_qprep + n_pack))
+        return tq_launch_kernel(tq_step_prologue_kernel<T, true, false>, grid, block, 0, stream, true, qa, *append, n_qprep);
+    const cudaError_t e = tq_allow_shared<tq_step_prologue_kernel<T, true, true>>(ctx->device, kStagedMatrices);
+    if (e != cudaSuccess) return e;
+    return tq_launch_kernel(tq_step_prologue_kernel<T, true, true>, grid, block, kStagedMatrices, stream, true, qa, *append, n_qprep);
 }
 
 int32_t tq_launch_qprep_frag(tq_ctx *ctx, const void *q, int32_t q_dtype, int64_t kv_rows, int G, uint32_t *frag,

@@ -37,6 +37,7 @@
 // merges splits, un-rotates and casts.
 #include <math.h>
 
+#include "tq_bulk.cuh"
 #include "tq_common.cuh"
 #include "tq_decode_shared.cuh"
 #include "tq_mma_utils.cuh"
@@ -68,7 +69,6 @@ constexpr int kGroupWarps = 4;  // warps that share a ring: one bulk copy per st
 constexpr int kGroups = kWarps / kGroupWarps;
 constexpr int kGroupTok = kGroupWarps * kStageTok;  // tokens per ring slot
 constexpr int kSlotWords = 64;  // table slot: 32 key words then 32 value words (256 B)
-constexpr uint32_t kSpinLimit = 1u << 22;  // mbarrier polls before a wait gives up
 
 struct Mma4Args {
     const uint8_t *k_codes;
@@ -94,9 +94,9 @@ struct Mma4Args {
     const float *centers_k, *centers_v;
     int *error_flag;  // set to 1 when a bounded wait ran out
     // Let the combine kernel start once this kernel's dependencies are met: it attends a dense tail, or there are idle SMs
-    // for it (see CombineArgs::next_blocks).  1 x 8 x 4099 tokens: 9 / 10 us of a step's 15.7 us chain remain.
-    bool has_tail;
-    int sm_count, next_blocks;
+    // for it (see CombineArgs::next_blocks): eight recorded layer steps at 4099 tokens 107 us, 126 us without.
+    bool release_early;
+    int sm_count, next_blocks;  // (a length on the device: the kernel decides)
     int device;       // host side only: the context's device
 };
 
@@ -110,43 +110,9 @@ template <int KB, int VB, bool QJL> struct StageLayout {
     static constexpr int kBytes = (kRN + (QJL ? kGroupTok * 2 : 0) + 127) / 128 * 128;
 };
 
-// ---- mbarrier / TMA bulk-copy wrappers (shared::cta addresses) ----
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
-// Bounded wait: returns false (and the caller flags an error) instead of spinning forever.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kSpinLimit; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-// Global -> shared bulk copy of `bytes` (multiple of 16, both addresses 16-byte aligned),
-// completion counted on `bar`.
-__device__ __forceinline__ void tma_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
 // The centre-pair table sits at shared-memory address kTableAddr, a multiple of 65536, so
 // that a complete address can be assembled without an add: bits 16+ are the table base,
 // byte 1 is the slot index (slot stride 256 B) and byte 0 the lane's offset inside the slot.
@@ -231,8 +197,6 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
         const TqPlan plan = tq_make_plan(N, a.rows, gridDim.x, a.n_splits, kWarps * kStageTok);
         n_pad = plan.n_pad, chunk = plan.chunk;
     }
-
-    const bool release_early = a.has_tail || (a.next_blocks && tq_leaves_idle({n_pad, chunk}, a.rows, a.sm_count, a.next_blocks));
 
     // ---- this CTA's contiguous piece of the flattened (row, token) space
     const int64_t flat_begin = (int64_t)blockIdx.x * chunk;
@@ -366,7 +330,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
     const int n_first = min(n_iter, kStages);
     if (first_segment) {
         tq_grid_dependency_wait();
-        if (release_early) tq_launch_dependents();
+        if (a.release_early || (a.len_ptr && a.next_blocks && tq_leaves_idle({n_pad, chunk}, a.rows, a.sm_count, a.next_blocks)))
+            tq_launch_dependents();
         TQ_STAMP(2);
         for (int it = 0; it < n_first; ++it)
             if (deferred >> it & 1) issue(sg, it);  // (only the issuing lane has bits set)
@@ -722,11 +687,11 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
     a.part_m = w.part_m, a.part_l = w.part_l, a.part_acc = w.part_acc;
     a.centers_k = ctx->centers_k, a.centers_v = ctx->centers_v;
     a.error_flag = ctx->error_flag;
-    a.has_tail = n_tail > 0;
     // (the wait for the peers that follows a gather is not one of the small kernels meant here)
     const int combine_blocks = a.rows * ((a.G + 3) / 4);
     const int prologue_blocks = combine_blocks * (ctx->use_qjl ? 2 : 1) + (append ? append->n_kinds * append->B * append->H * append->S : 0);
-    a.sm_count = ctx->sm_count, a.next_blocks = gather || n_tail ? 0 : combine_blocks + (prologue_blocks + 1) / 2;
+    a.sm_count = ctx->sm_count, a.next_blocks = gather || n_tail ? 0 : combine_blocks + (append && tq_stages_matrices(ctx, prologue_blocks) ? prologue_blocks : (prologue_blocks + 1) / 2);
+    a.release_early = n_tail > 0 || (!len_ptr && a.next_blocks && tq_leaves_idle(plan, a.rows, a.sm_count, a.next_blocks));
     a.device = ctx->device;
     // Length on the device: the kernel plans for its own grid.  One CTA per SM, except that a
     // single partial per row (n_splits == 1) means one CTA per row, however many rows there are.

@@ -7,6 +7,9 @@
 // their own tiles, four threads to a vector, A written to TMEM, the matrices resident in shared memory; the two
 // contractions of a key go one after the other through the group's one accumulator, the first result waiting as
 // packed T.  16-bit rows leave through shared memory, one bulk copy each.
+// Bound, like the encoder, by the chain of a tile with two in flight.  8 x 32768 bf16 keys with the sketch 57 us,
+// values 40 us (HBM floor 13 each); 1123 and 571 us with fp32 multiply-adds and the matrix read from L2 per vector,
+// 66 and 46 us with two threads a vector and direct stores.
 #include <math.h>
 
 #include <type_traits>

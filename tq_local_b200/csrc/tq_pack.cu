@@ -145,9 +145,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) tq_pack_rows_kernel(PackA
 
 // Latency-optimised encoder for a handful of vectors (the per-step append of decoded tokens):
 // one 512-thread block per vector, see tq_pack_small_block.
-template <typename T, bool QJL>
-__global__ void __launch_bounds__(4 * TQ_D, 2) tq_pack_small_kernel(PackArgs a) {
-    tq_pack_small_block<T, QJL>(a, blockIdx.x);
+template <typename T, bool QJL, bool STAGED>
+__global__ void __launch_bounds__(4 * TQ_D, STAGED ? 1 : 2) tq_pack_small_kernel(PackArgs a) {
+    tq_pack_small_block<T, QJL, STAGED>(a, blockIdx.x);
 }
 
 struct DequantArgs {
@@ -364,6 +364,15 @@ void tq_fill_pack_args(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc 
     a.pos_ptr = nullptr, a.capacity = cache->capacity, a.error_flag = ctx->error_flag;
 }
 
+// (staged matrices: one block per SM, see tq_pack_small_block)
+template <typename T> static cudaError_t launch_small(tq_ctx *ctx, const PackArgs &a, int64_t items, cudaStream_t stream) {
+    const dim3 grid((unsigned)items), block(4 * TQ_D);
+    if (!ctx->use_qjl) return tq_launch_kernel(tq_pack_small_kernel<T, false, false>, grid, block, 0, stream, false, a);
+    if (!tq_stages_matrices(ctx, items)) return tq_launch_kernel(tq_pack_small_kernel<T, true, false>, grid, block, 0, stream, false, a);
+    const cudaError_t e = tq_allow_shared<tq_pack_small_kernel<T, true, true>>(ctx->device, kStagedMatrices);
+    return e != cudaSuccess ? e : tq_launch_kernel(tq_pack_small_kernel<T, true, true>, grid, block, kStagedMatrices, stream, false, a);
+}
+
 int32_t tq_launch_pack(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tokens,
                        const tq_cache_desc *cache, int32_t pos0, cudaStream_t stream) {
     PackArgs a;
@@ -389,19 +398,14 @@ int32_t tq_launch_pack(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc 
     }
     const int64_t items = a.n_kinds * n_vec;
     if (n_vec < 1024) {  // appends: one block per vector
-#define TQ_LAUNCH_SMALL(T)                                                                   \
-    do {                                                                                     \
-        if (ctx->use_qjl)                                                                    \
-            tq_pack_small_kernel<T, true><<<(unsigned)items, 4 * TQ_D, 0, stream>>>(a);      \
-        else                                                                                 \
-            tq_pack_small_kernel<T, false><<<(unsigned)items, 4 * TQ_D, 0, stream>>>(a);     \
-    } while (0)
+        cudaError_t e;
+#define TQ_LAUNCH_SMALL(T) e = launch_small<T>(ctx, a, items, stream)
         if (k->dtype == TQ_DTYPE_F32) TQ_LAUNCH_SMALL(float);
         else if (k->dtype == TQ_DTYPE_F16) TQ_LAUNCH_SMALL(__half);
         else TQ_LAUNCH_SMALL(__nv_bfloat16);
 #undef TQ_LAUNCH_SMALL
         tq_prof_count(ctx, 1);
-        TQ_CUDA_CHECK(cudaGetLastError());
+        TQ_CUDA_CHECK(e);
         return TQ_OK;
     }
     const int grid = grid_for(items, ctx->sm_count);
@@ -424,6 +428,8 @@ int32_t tq_launch_pack(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc 
 
 int32_t tq_launch_dequant(tq_ctx *ctx, const tq_cache_desc *cache, int32_t which, int32_t pos0,
                           int32_t n_tokens, const tq_dense_desc *out, cudaStream_t stream) {
+    // (1024 vectors, keys with the sketch: 13.4 us there, 20 us here, launch and host call included; below that the
+    // matrices' way to shared memory costs as much as these few vectors)
     if ((int64_t)cache->batch * cache->kv_heads * n_tokens >= 1024) {
         const int32_t rc = tq_launch_dequant_tc(ctx, cache, which, pos0, n_tokens, out, stream);
         if (rc != TQ_ERR_UNSUPPORTED) return rc;

@@ -19,6 +19,10 @@
 // bulk copy each: read straight from global memory by the threads that own them they took 2048 of the 4500
 // L1 wavefronts of a value tile, which bounded it.  A group owns 256 TMEM columns: 128 of accumulator, 64 for each term of A.
 // The first CTAs of a launch encode keys and the others values, in the proportion of their costs.
+// What bounds it is the chain of a key tile - store A, MMA, read back, three times - with two tiles in flight, which
+// is what 512 TMEM columns hold (tensor pipe 34 %, issue slots 54 %, L1 33 % busy).  8 x 8 x 32768 bf16 keys and
+// values, 4 bits with the sketch: 907 us; 1306 us with two threads a vector that read their own rows and a binary search;
+// 2189 us with three-term bf16 operands in shared memory, one tile at a time.
 // Every mbarrier wait is bounded and reports through the device status word.
 #include <math.h>
 #include <string.h>
@@ -600,7 +604,8 @@ int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_de
     a.signs = cache->k_signs, a.rnorms = cache->k_rnorms;
     a.n_tiles = (int)((a.vec.n + kUmmaRows - 1) / kUmmaRows);
     // One CTA per SM.  With tiles enough for all of them, keys with the sketch get the share of the SMs that
-    // their cost asks for; with few tiles each side gets a CTA per tile.
+    // their cost asks for (a key tile takes 5.7 us of an SM, a value tile 2.4); with few tiles each side gets a CTA
+    // per tile, and no SM two (8 x 1000 vectors a tensor: 16 us, 31 us in two launches).
     const int sms = ctx->sm_count;
     int key_ctas = !k ? 0 : qjl ? sms * 7 / 10 : sms / 2, val_ctas = sms - key_ctas;
     if (k && a.n_tiles <= sms / 2) key_ctas = val_ctas = a.n_tiles;

@@ -9,6 +9,7 @@
 // (one trip to L2 instead of a chain of them) before the data they multiply is ready.
 #pragma once
 
+#include "tq_bulk.cuh"
 #include "tq_common.cuh"
 
 struct TqPackArgs {
@@ -110,7 +111,15 @@ __device__ __forceinline__ uint32_t tq_assemble_word(const uint8_t *codes, int w
 // Encode one vector (item < n_vec: kind first_kind, else the next kind) and write it at its
 // cache row.  fp32 arithmetic in a fixed order: partial sums over four 32-row quarters, then
 // (p0 + p1) + (p2 + p3).
-template <typename T, bool QJL> __device__ __forceinline__ void tq_pack_small_block(const TqPackArgs &a, int64_t item) {
+// A key with a sketch is a chain of three mat-vecs.  STAGED (128 KB of dynamic shared memory, for launches of no more
+// blocks than SMs): the matrices of the second and third are requested by bulk copy before anything else and wait in
+// shared memory; otherwise their columns are read from L2 in turn, 64 KB a mat-vec and a microsecond of the chain
+// (eight recorded layer steps at 4099 tokens, 32 blocks each: 104 us against 107).
+constexpr int kStagedMatrices = 2 * TQ_D * TQ_D * 4;
+inline bool tq_stages_matrices(const tq_ctx *ctx, int64_t blocks) { return ctx->use_qjl && blocks <= ctx->sm_count; }
+template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_pack_small_block(const TqPackArgs &a, int64_t item) {
+    extern __shared__ __align__(128) float s_matrices[];
+    __shared__ __align__(8) uint64_t s_bar;
     __shared__ float s_x[TQ_D], s_u[TQ_D], s_part[4][TQ_D], s_red[4];
     __shared__ uint8_t s_code[TQ_D];
     __shared__ float s_bnd[16], s_cen[16];
@@ -123,6 +132,16 @@ template <typename T, bool QJL> __device__ __forceinline__ void tq_pack_small_bl
     const int b = (int)(vid / ((int64_t)a.S * a.H));
     const T *src = (const T *)a.x[kind] + b * a.sb[kind] + h * a.sh[kind] + (int64_t)t * a.st[kind];
     const int bits = a.bits[kind];
+    const bool residual = QJL && kind == 0;
+    if (STAGED && residual && tid == 0) {
+        const uint32_t bar = smem_u32(&s_bar), dst = smem_u32(s_matrices);
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        mbar_expect_tx(bar, kStagedMatrices);
+        tma_load_1d(dst, a.rot_k, kStagedMatrices / 2, bar);
+        tma_load_1d(dst + kStagedMatrices / 2, a.qjl_t, kStagedMatrices / 2, bar);
+    }
     float m[32];
     tq_load_column(m, a.rot_t[kind], dq, j);  // (codec constants: fetched before the wait)
     if (tid < 16) s_bnd[tid] = a.bounds[kind][tid], s_cen[tid] = a.centers_k[tid];
@@ -131,8 +150,11 @@ template <typename T, bool QJL> __device__ __forceinline__ void tq_pack_small_bl
     tq_grid_dependency_wait();
     tq_launch_dependents();
     const int pos0 = a.pos_ptr ? *a.pos_ptr : a.pos0;
-    if (pos0 < 0 || pos0 + a.S > a.capacity) {  // (the whole block leaves together)
-        if (tid == 0) atomicExch(a.error_flag, 4);
+    if (pos0 < 0 || pos0 + a.S > a.capacity) {  // (the whole block leaves together, its copies landed)
+        if (tid == 0) {
+            atomicExch(a.error_flag, 4);
+            if (STAGED && residual) mbar_wait(smem_u32(&s_bar), 0);
+        }
         return;
     }
     const int64_t row = b * a.cache_sb + h * a.cache_sh + pos0 + t;
@@ -166,8 +188,16 @@ template <typename T, bool QJL> __device__ __forceinline__ void tq_pack_small_bl
     if (dq == 0) s_x[j] = x, s_u[j] = x / safe;
     __syncthreads();
     quarter(s_u);
-    const bool residual = QJL && kind == 0;
-    if (residual) tq_load_column(m, a.rot_k, dq, j);  // in flight while the codes are formed
+    auto next_column = [&](int i) {  // (a barrier separates the copies' request from every thread's wait)
+        if (STAGED) {
+            if (!mbar_wait(smem_u32(&s_bar), 0) && tid == 0) atomicExch(a.error_flag, 3);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) m[e] = s_matrices[i * TQ_D * TQ_D + (32 * dq + e) * TQ_D + j];
+        } else {
+            tq_load_column(m, i == 0 ? a.rot_k : a.qjl_t, dq, j);
+        }
+    };
+    if (residual) next_column(0);  // in flight while the codes are formed
     const float z = finish();
     int idx = 0;
 #pragma unroll
@@ -183,7 +213,7 @@ template <typename T, bool QJL> __device__ __forceinline__ void tq_pack_small_bl
         if (dq == 0) s_u[j] = s_cen[idx];
         __syncthreads();
         quarter(s_u);  // sum_j c[j] * R_k[j][d], d = this thread's column
-        tq_load_column(m, a.qjl_t, dq, j);
+        next_column(1);
         const float rec = finish();
         const float res = s_x[j] - tq_round_through<T>(rec * tq_half_bits_to_float(nh));
         const float rn = block_norm(res);

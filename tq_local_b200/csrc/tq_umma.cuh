@@ -1,5 +1,4 @@
-// Helpers of the tcgen05 kernels (prefill encoder, dequantisation): mbarriers, bulk copies, matrix
-// descriptors, TMEM loads and stores, and the f16 operand images of the 128 x 128 matrices.
+// Helpers of the tcgen05 kernels (prefill encoder, dequantisation): matrix descriptors, TMEM loads and stores, and the f16 operand images of the 128 x 128 matrices.
 //
 // Every contraction here is [128 vectors x 128] * M with fp32 accuracy on f16 tensor cores: an fp32
 // operand, scaled by a power of two so that its largest element is below 2^15, is split in two f16
@@ -11,41 +10,14 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "tq_bulk.cuh"
 #include "tq_common.cuh"
 
 constexpr int kUmmaRows = 128;                         // vectors per tile: the rows of A and of the accumulator
 constexpr int kUmmaSlabBytes = 128 * 128;              // 128 rows x 64 f16 (one 128-byte swizzle row each): 16 KB
 constexpr int kUmmaTermBytes = 2 * kUmmaSlabBytes;     // one f16 term of a 128 x 128 matrix: 32 KB
 constexpr int kUmmaImageBytes = 2 * kUmmaTermBytes;    // hi and lo terms: 64 KB
-constexpr uint32_t kUmmaSpinLimit = 1u << 22;          // polls before a wait gives up
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kUmmaSpinLimit; ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n.reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void tma_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
 // Shared memory to global (one thread; complete once its bulk group is).
 __device__ __forceinline__ void tma_store_1d(void *dst, uint32_t src, uint32_t bytes) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
