@@ -218,3 +218,54 @@ def test_dequantisation(setup_golden, bits, qjl, dtype, shape):
             room = 2e-6 * ref.abs().max() + ulp * (ref.abs() + 0.5 * ref.abs().amax(dim=-1, keepdim=True) * (which == "keys" and qjl))
             assert ((got - ref).abs() <= room).all(), (which, lo, float((got - ref).abs().max()))
     assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+def test_append_encoder_staging(setup_golden, dtype):
+    """Appends of no more vectors than SMs keep the matrices in shared memory, larger ones read them from L2: the same
+    bits (two 74-vector tensors against two of 76; 148 SMs)."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec = make_codec(4, True, setup_golden)
+    k, v = vectors((1, 2, 38, 128), 1, dtype), vectors((1, 2, 38, 128), 2, dtype)
+    few, more = PackedStore(codec, 1, 2, 40), PackedStore(codec, 1, 2, 40)
+    few.pack(k[:, :, :37], v[:, :, :37])
+    more.pack(k, v)
+    for a, b in zip(few.streams(), more.streams()):
+        assert torch.equal(a[:, :, :37], b[:, :, :37])
+    assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("batch,heads,tokens", [(1, 2, 33), (1, 8, 4099), (4, 8, 2000), (8, 8, 1500)])
+def test_recorded_steps_of_several_layers(setup_golden, batch, heads, tokens):
+    """Chained steps that release their successors early (few rows and tokens: idle SMs) and that do not: every layer's
+    replayed output and stored bytes are those of the same calls made one at a time."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec, layers = make_codec(4, True, setup_golden), 4
+    draw = lambda h, t, s: vectors((batch, h, t, 128), s, BF16)
+    stores, plain, new = [], [], []
+    for i in range(layers):
+        k, v = draw(heads, tokens, 10 * i), draw(heads, tokens, 10 * i + 1)
+        for group in (stores, plain):
+            group.append(PackedStore(codec, batch, heads, tokens + 8))
+            group[-1].pack(k, v)
+        new.append((query((batch, 4 * heads, 1), 10 * i + 2, BF16), draw(heads, 1, 10 * i + 3), draw(heads, 1, 10 * i + 4)))
+    pos = torch.tensor([tokens], dtype=torch.int32, device="cuda")
+    step = lambda: [s.decode_step_dev(*x, pos) for s, x in zip(stores, new)]
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = step()
+    for n in range(3):
+        pos.fill_(tokens + n)
+        graph.replay()
+        torch.cuda.synchronize()
+        for s, p, out, (q, k, v) in zip(stores, plain, outs, new):
+            p.pack(k, v)
+            torch.cuda.synchronize()
+            assert torch.equal(out, p.decode_attn(q, splits=s.suggest_splits(s.capacity)))
+            for a, b in zip(s.streams(), p.streams()):
+                assert torch.equal(a[:, :, :tokens + n + 1], b[:, :, :tokens + n + 1])
+    assert codec.device_status() == 0
