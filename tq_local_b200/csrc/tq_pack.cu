@@ -1,10 +1,10 @@
-// CUDA-core (fp32 FMA) encode / dequantise kernels: one warp per vector.
+// CUDA-core (fp32 FMA) encode / dequantise kernels: one warp per vector, or (append) one block.
 //
 // tq_pack_rows_kernel is the arithmetic-exact encoder: fp32 accumulation in a
 // fixed order, true division, the reference's tie rule (a value equal to a
 // boundary goes to the lower bin) and the reference's dtype round trip of the
-// reconstruction before the QJL residual.  It serves the O(1) append of decoded
-// tokens and small prefills; large prefills go to the tensor-core kernel.
+// reconstruction before the QJL residual.  It serves prefills whose tensors or
+// codebook the tensor-core kernel does not take; appends have a kernel of their own.
 #include "tq_common.cuh"
 #include "tq_step_blocks.cuh"
 
