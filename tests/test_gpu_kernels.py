@@ -91,6 +91,31 @@ def test_dense_tail(setup_golden, dtype, groups, n_tail):
     assert rel_inf(store.decode_attn(q, tail_k=tk, tail_v=tv), alone) <= ATTN_TOL[dtype]
 
 
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("n_tail,masked", [(1, (0, 1)), (64, (0, 64)), (130, (0, 44)), (130, (44, 130)), (1100, (0, 275)), (1100, (300, 600)),
+                                           (1100, (0, 1099))])
+def test_dense_tail_with_infinite_logits(setup_golden, dtype, n_tail, masked):
+    """Tail tokens whose logit is -inf weigh nothing, also where they fill a chunk or a CTA's whole share; with nothing
+    else to attend the result is undefined, as that softmax is."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(4, True, setup_golden), make_codec(4, True, setup_golden)
+    store = PackedStore(codec, 1, 2, capacity=80)
+    store.pack(vectors((1, 2, 70, 128), 1, dtype), vectors((1, 2, 70, 128), 2, dtype))
+    q = query((1, 10, 1), 3, dtype)
+    q[..., 7] = q[..., 7].abs() + 0.5
+    tk, tv = vectors((1, 2, n_tail, 128), 4, dtype), vectors((1, 2, n_tail, 128), 5, dtype)
+    tk[:, :, masked[0]:masked[1], 7] = -float("inf")
+    assert rel_inf(store.decode_attn(q, tail_k=tk, tail_v=tv), attend64(store, p, q, 5, tk, tv)) <= ATTN_TOL[dtype]
+    store.length = 0
+    k, v = tk.cpu().double().repeat_interleave(5, dim=1), tv.cpu().double().repeat_interleave(5, dim=1)
+    alone, got = torch.softmax(q.cpu().double() @ k.transpose(-1, -2) / math.sqrt(128), dim=-1) @ v, store.decode_attn(q, tail_k=tk, tail_v=tv)
+    if masked[1] - masked[0] == n_tail:
+        assert got.isnan().all() and alone.isnan().all()
+    else:
+        assert rel_inf(got, alone) <= ATTN_TOL[dtype]
+
+
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("splits", [1, 2, 8, 9, 31, 32, 33, 41, 70])
 def test_split_merge(setup_golden, dtype, splits):

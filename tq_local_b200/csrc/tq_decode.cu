@@ -403,11 +403,12 @@ __device__ __forceinline__ float tq_attend_tail(const CombineArgs &a, TailShared
             float x[kTailChunk / 32], mx = -INFINITY, sum = 0.f;
 #pragma unroll
             for (int i = 0; i < kTailChunk / 32; ++i) x[i] = sm.p[warp][32 * i + lane], mx = fmaxf(mx, x[i]);
-            const float nm = fmaxf(m_run, tq_warp_max(mx));  // (finite: a chunk holds at least one token)
-            const float corr = expf(m_run - nm);
+            const float nm = fmaxf(m_run, tq_warp_max(mx));
+            const float base = nm == -INFINITY ? 0.f : nm;  // (every logit so far is -inf: weights of 0, not undefined ones)
+            const float corr = expf(m_run - base);
 #pragma unroll
             for (int i = 0; i < kTailChunk / 32; ++i) {
-                const float p = expf(x[i] - nm);
+                const float p = expf(x[i] - base);
                 sm.p[warp][32 * i + lane] = p, sum += p;
             }
             l_run = l_run * corr + tq_warp_sum(sum), m_run = nm;
@@ -466,7 +467,7 @@ __device__ __forceinline__ bool tq_merge_tails(TailShared &sm, float &o, float &
         for (int r = 1; r < n; ++r) {
             const TailShared &peer = *cluster.map_shared_rank(&sm, r);
             const float pm = peer.m[g], pl = peer.l[g], po = (&peer.acc[0][0][0])[tid];
-            const float M = fmaxf(m, pm), w = expf(m - M), pw = expf(pm - M);  // (every share holds at least one token)
+            const float M = fmaxf(m, pm), w = m == -INFINITY ? 0.f : expf(m - M), pw = pm == -INFINITY ? 0.f : expf(pm - M);
             o = o * w + po * pw, l = l * w + pl * pw, m = M;
         }
     }
@@ -603,7 +604,7 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
         const int g = dq;
         float v = (s_part[0][g][e] + s_part[1][g][e]) + (s_part[2][g][e] + s_part[3][g][e]);
         float L = s_L[g];
-        if (TAIL) {  // (tail_m is finite: a tail has at least one token)
+        if (TAIL) {  // (when packed tokens and tail both have logits of -inf alone, the result is undefined, as a softmax is)
             const float M = fmaxf(s_M[g], tail_m), wt = expf(tail_m - M);
             const float wp = s_M[g] == -INFINITY ? 0.f : expf(s_M[g] - M);
             v = v * wp + tail_o * wt, L = L * wp + tail_l * wt;
