@@ -116,6 +116,59 @@ def test_dense_tail_with_infinite_logits(setup_golden, dtype, n_tail, masked):
         assert rel_inf(got, alone) <= ATTN_TOL[dtype]
 
 
+def attend_tail64(store, p, q, groups, tk, tv, starts):
+    """``attend64`` with the packed tokens before ``starts[b]`` left out."""
+    layer = store_to_layer(store, p, torch.float32)
+    k, v = O.dequant_keys(layer).double(), O.dequant_values(layer).double()
+    k, v = torch.cat((k, tk.cpu().double()), dim=2), torch.cat((v, tv.cpu().double()), dim=2)
+    k, v = k.repeat_interleave(groups, dim=1), v.repeat_interleave(groups, dim=1)
+    logits = q.cpu().double() @ k.transpose(-1, -2) / math.sqrt(128)
+    masked = torch.arange(logits.shape[-1])[None, None, None] < torch.tensor(starts)[:, None, None, None]
+    return torch.softmax(logits.masked_fill(masked, -float("inf")), dim=-1) @ v
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("batch,heads,groups,n_tail", [
+    (1, 2, 4, 85), (1, 2, 4, 86), (1, 2, 5, 1024), (1, 2, 4, 1025), (1, 2, 5, 1029), (1, 1, 1, 2500),  # one CTA, four, second chunks
+    (4, 8, 1, 128), (4, 8, 1, 129), (4, 8, 4, 513),                                                     # one, two, four CTAs
+    (8, 8, 1, 384), (8, 8, 4, 385), (8, 8, 1, 600),                                                     # one CTA, two
+    (16, 8, 4, 5), (16, 8, 4, 6), (16, 4, 7, 300), (32, 8, 4, 23), (32, 8, 1, 24), (19, 8, 8, 33), (19, 8, 5, 34),  # a row a block
+    (64, 8, 1, 95), (64, 8, 1, 96), (128, 8, 1, 256), (128, 8, 1, 257)])
+def test_dense_tail_ranges(setup_golden, dtype, batch, heads, groups, n_tail):
+    """Every way a tail is shared out, on both sides of each limit (on 148 SMs): clusters of one, two and four CTAs, shares of
+    more than one chunk of 256, more rows than SMs in both kernels; the largest logits in the last quarter of the tail,
+    so that every merge rescales."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(4, True, setup_golden), make_codec(4, True, setup_golden)
+    store = PackedStore(codec, batch, heads, capacity=40)
+    store.pack(vectors((batch, heads, 33, 128), 1, dtype), vectors((batch, heads, 33, 128), 2, dtype))
+    q = query((batch, heads * groups, 1), 3, dtype)
+    tk, tv = vectors((batch, heads, n_tail, 128), 4, dtype), vectors((batch, heads, n_tail, 128), 5, dtype)
+    tk[:, :, n_tail - (n_tail + 3) // 4:] *= 4
+    want = attend64(store, p, q, groups, tk, tv)
+    got = store.decode_attn(q, tail_k=tk, tail_v=tv)
+    assert rel_inf(got, want) <= ATTN_TOL[dtype]
+    assert torch.equal(got, store.decode_attn(q, tail_k=off_by_one(tk), tail_v=off_by_one(tv)))
+    assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("copies,n_tail", [(1, 70), (1, 300), (86, 5), (86, 200)])
+def test_dense_tail_of_padded_rows(setup_golden, dtype, copies, n_tail):
+    """A left-padded batch with a tail, few rows and more than there are SMs."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(4, True, setup_golden), make_codec(4, True, setup_golden)
+    starts = [0, 41, 69] * copies
+    store = PackedStore(codec, len(starts), 2, capacity=72)
+    store.pack(vectors((len(starts), 2, 70, 128), 1, dtype), vectors((len(starts), 2, 70, 128), 2, dtype))
+    store.set_seq_start(torch.tensor(starts, dtype=torch.int32, device="cuda"))
+    q = query((len(starts), 6, 1), 3, dtype)
+    tk, tv = vectors((len(starts), 2, n_tail, 128), 4, dtype), vectors((len(starts), 2, n_tail, 128), 5, dtype)
+    assert rel_inf(store.decode_attn(q, tail_k=tk, tail_v=tv), attend_tail64(store, p, q, 3, tk, tv, starts)) <= ATTN_TOL[dtype]
+
+
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("splits", [1, 2, 8, 9, 31, 32, 33, 41, 70])
 def test_split_merge(setup_golden, dtype, splits):

@@ -342,11 +342,11 @@ template <typename T> __device__ __forceinline__ void tq_load8(const T *p, bool 
 // values: sixteen threads cover a row with 16-byte loads and 32 rows are read side by side.
 // Returns this thread's element (head threadIdx.x / 128, column threadIdx.x % 128) of the
 // unnormalised sum; the maximum and the sum of every head are left in s_tm / s_tl.
-// What bounds it is the latency of two dependent trips to memory per 256 tokens; the row's tail is shared
-// out over the CTAs of a cluster (tq_merge_tails).
+// What bounds it is the latency of two dependent trips to memory per 256 tokens; where SMs are free for it, the
+// row's tail is shared out over the CTAs of a cluster (tq_merge_tails, tq_set_combine_tail).
 constexpr int kTailChunk = 256;
-constexpr int kTailTokensPerCta = 64;  // one pass of the logit loop; a CTA takes more only when all of them are used
-constexpr int kTailCtas = 4;           // CTAs of a cluster
+constexpr int kTailCtas = 4;         // CTAs of a cluster, at most
+constexpr int kRowTailTokens = 256;  // tail tokens that tq_combine_row_kernel takes, at most
 struct TailShared {
     float p[4][kTailChunk];
     float corr[4], m[4], l[4];
@@ -481,7 +481,6 @@ __device__ __forceinline__ bool tq_merge_tails(TailShared &sm, float &o, float &
 // releases this one as soon as the query and the tail are known to be there, so the tail is attended on
 // SMs that the decode kernel leaves free.  12001 packed + 300 dense tokens, 8 KV rows, launches recorded: 17.0 us
 // from query preparation to output; 28.2 us with one block per four heads that began after the decode kernel.
-// Four CTAs and not eight: a cluster's CTAs need free SMs of one GPC at the same time.
 template <typename T, bool TAIL>
 __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs a) {
     __shared__ __align__(16) float s_o[4][TQ_D];
@@ -647,6 +646,61 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
     }
 }
 
+// The combine of one query row per block of 128 threads, with a dense tail: what many rows with few tail tokens take (see
+// tq_set_combine_tail).  Sixteen of its blocks fit an SM, so that hundreds of rows are one wave where the blocks of
+// tq_combine_group_kernel, one to an SM, are several.  What bounds it is one trip to memory per four tail tokens.
+template <typename T>
+__global__ void __launch_bounds__(TQ_D) tq_combine_row_kernel(CombineArgs a) {
+    __shared__ float s_logit[kRowTailTokens];
+    __shared__ float s_o[TQ_D], s_q[TQ_D], s_red[4];
+    const int64_t row = blockIdx.x;  // b * Hq + hq
+    const int e = threadIdx.x, warp = e >> 5, lane = e & 31;
+    const int b = (int)(row / a.Hq), hkv = (int)(row % a.Hq) / a.G;
+    const float hs = 0.08838834764831845f;
+    int n_valid = a.n_splits;
+    if (a.seg_chunk > 0) {
+        const int64_t lo = (row / a.G) * (int64_t)a.seg_npad;
+        n_valid = (int)((lo + a.seg_npad - 1) / a.seg_chunk - lo / a.seg_chunk) + 1;
+    }
+    float M = -INFINITY;
+    for (int s = 0; s < n_valid; ++s) M = fmaxf(M, a.part_m[row * a.n_splits + s]);
+    const T *tk = (const T *)a.tail_k + b * a.tk_sb + hkv * a.tk_sh;
+    const T *tv = (const T *)a.tail_v + b * a.tv_sb + hkv * a.tv_sh;
+    s_q[e] = tq_to_float<T>(((const T *)a.q)[row * TQ_D + e]);
+    __syncthreads();
+    float wmax = -INFINITY;
+    for (int t = warp; t < a.n_tail; t += 4) {
+        const T *kr = tk + (int64_t)t * a.tk_st + 4 * lane;
+        float dot = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dot = fmaf(s_q[4 * lane + i], tq_to_float<T>(kr[i]), dot);
+        dot = tq_warp_sum(dot) * hs;
+        if (lane == 0) s_logit[t] = dot;
+        wmax = fmaxf(wmax, dot);
+    }
+    if (lane == 0) s_red[warp] = wmax;
+    __syncthreads();
+    M = fmaxf(M, fmaxf(fmaxf(s_red[0], s_red[1]), fmaxf(s_red[2], s_red[3])));
+    float L = 0.f, o = 0.f;
+    for (int s = 0; s < n_valid; ++s) {
+        const float ms = a.part_m[row * a.n_splits + s];
+        const float w = ms == -INFINITY ? 0.f : expf(ms - M);
+        L += a.part_l[row * a.n_splits + s] * w;
+        o += a.part_acc[(row * a.n_splits + s) * TQ_D + e] * w;
+    }
+    s_o[e] = o;
+    __syncthreads();
+    float out = 0.f;
+#pragma unroll 8
+    for (int d = 0; d < TQ_D; ++d) out = fmaf(s_o[d], __ldg(a.rot_v + d * TQ_D + e), out);
+    for (int t = 0; t < a.n_tail; ++t) {
+        const float p = expf(s_logit[t] - M);
+        L += p;
+        out = fmaf(p, tq_to_float<T>(tv[(int64_t)t * a.tv_st + e]), out);
+    }
+    ((T *)a.out)[row * TQ_D + e] = tq_from_float<T>(out / fmaxf(L, 1e-8f));
+}
+
 __device__ __forceinline__ unsigned long long tq_global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
@@ -722,6 +776,9 @@ static void configure_small_kernels() {
     prefer_max_shared(tq_combine_group_kernel<float, false>);
     prefer_max_shared(tq_combine_group_kernel<__half, false>);
     prefer_max_shared(tq_combine_group_kernel<__nv_bfloat16, false>);
+    prefer_max_shared(tq_combine_row_kernel<float>);
+    prefer_max_shared(tq_combine_row_kernel<__half>);
+    prefer_max_shared(tq_combine_row_kernel<__nv_bfloat16>);
     prefer_max_shared(tq_combine_group_kernel<float, true>);
     prefer_max_shared(tq_combine_group_kernel<__half, true>);
     prefer_max_shared(tq_combine_group_kernel<__nv_bfloat16, true>);
@@ -785,6 +842,10 @@ int32_t tq_launch_qprep_frag(tq_ctx *ctx, const void *q, int32_t q_dtype, int64_
 
 template <typename T>
 static cudaError_t launch_combine(const CombineArgs &a, dim3 grid, cudaStream_t stream, bool programmatic) {
+    if (a.n_tail > 0 && a.tail_rows) {
+        tq_combine_row_kernel<T><<<grid.x / ((a.G + 3) / 4) * a.G, TQ_D, 0, stream>>>(a);
+        return cudaGetLastError();
+    }
     if (a.n_tail == 0)
         return tq_launch_kernel(tq_combine_group_kernel<T, false>, grid, dim3(4 * TQ_D), 0, stream, programmatic, a);
     return tq_launch_cluster(tq_combine_group_kernel<T, true>, dim3(grid.x * a.tail_ctas), dim3(4 * TQ_D), sizeof(TailShared),
@@ -803,16 +864,37 @@ int32_t tq_launch_combine(const CombineArgs &a, int32_t q_dtype, int64_t rows, c
     return TQ_OK;
 }
 
-// The tail fields of the combine arguments: `tail_vec` when every row of both tensors starts on a 16-byte boundary.
-int32_t tq_set_combine_tail(CombineArgs &c, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tail, int32_t q_dtype) {
-    c.n_tail = n_tail, c.tail_k = c.tail_v = nullptr, c.tail_vec = false, c.tail_ctas = 0, c.tail_per_cta = 0;
+// The tail fields of the combine arguments: `tail_vec` when every row of both tensors starts on a 16-byte boundary, and
+// which kernel attends the tail of `kv_rows` KV rows.
+//
+// tq_combine_group_kernel needs an SM per block (four heads of a KV row), so that it takes 5 us more for every wave of blocks after
+// the first; tq_combine_row_kernel takes a sixteenth of an SM per head, but a trip to memory for every four tail tokens.  So the
+// more blocks there are to an SM, the longer the tail up to which the second is faster.  Measured where they cross (148 SMs,
+// 512 / 4096 packed tokens, the tail in L2 / in HBM; us row kernel against group kernel): 64 blocks nowhere (17.1 against 14.4 at
+// one token); 128 blocks at 12 / 8 tokens (19.7 against 21.0 at one, 38.9 against 37.7 at 16); 256 at 58 / 17 (35.6 against 38.7,
+// 75.8 against 71.0 at 33); 512 at 125 / 96 (62 against 74, 137.8 against 137.0 at 96): 8 tokens times the square of blocks per SM.
+//
+// In the group kernel a row's tail is split over the CTAs of a cluster where that pays.  A CTA takes 28 ns per token; a
+// cluster costs less than 64 tokens' time while its CTAs find half of the SMs free, 100 to 190 tokens' time up to all of them
+// (its CTAs need free SMs of one GPC at once), and more beyond (us for 1 / 2 / 4 CTAs, 512 packed tokens: 8 blocks, 300 tail
+// tokens 20.5 / 16.4 / 15.6, 128: 14.6 / 14.8; 32 blocks, 300: 20.7 / 16.8 / 20.2, 1000: 38.1 / 25.2 / 22.8; 64 blocks, 128:
+// 16.3 / 20.4, 512: 25.4 / 23.4 / 32.3; 128 blocks, 300: 28.7 / 35.8 / 53.8).
+int32_t tq_set_combine_tail(CombineArgs &c, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tail, int32_t q_dtype,
+                            int64_t kv_rows, int sm_count) {
+    c.n_tail = n_tail, c.tail_k = c.tail_v = nullptr, c.tail_vec = c.tail_rows = false, c.tail_ctas = 0, c.tail_per_cta = 0;
     c.tk_sb = c.tk_sh = c.tk_st = c.tv_sb = c.tv_sh = c.tv_st = 0;
     if (n_tail == 0) return TQ_OK;
     if (k->dtype != q_dtype || v->dtype != q_dtype) return TQ_ERR_ARG;
-    // as many CTAs as there are passes of 64 tokens, kTailCtas at most; none of them empty
-    const int passes = (n_tail + kTailTokensPerCta - 1) / kTailTokensPerCta, ctas = passes < kTailCtas ? passes : kTailCtas;
+    const int64_t blocks = kv_rows * ((c.G + 3) / 4);
+    c.tail_rows = 2 * blocks > sm_count && n_tail <= kRowTailTokens && n_tail <= 8 * blocks * blocks / ((int64_t)sm_count * sm_count);
+    int ctas = 1;
+    int64_t cost = n_tail;
+    for (int n = 2; n <= kTailCtas && n * blocks <= sm_count; n *= 2) {
+        const int64_t with = (n_tail + n - 1) / n + (2 * n * blocks <= sm_count ? 64 : 192);
+        if (with < cost) ctas = n, cost = with;
+    }
     c.tail_per_cta = (n_tail + ctas - 1) / ctas;
-    c.tail_ctas = (n_tail + c.tail_per_cta - 1) / c.tail_per_cta;
+    c.tail_ctas = (n_tail + c.tail_per_cta - 1) / c.tail_per_cta;  // (none of them empty)
     c.tail_k = k->data, c.tail_v = v->data;
     c.tk_sb = k->stride_b, c.tk_sh = k->stride_h, c.tk_st = k->stride_t;
     c.tv_sb = v->stride_b, c.tv_sh = v->stride_h, c.tv_st = v->stride_t;
@@ -915,7 +997,7 @@ int32_t tq_launch_decode_exact(tq_ctx *ctx, const void *q, int32_t q_dtype, int3
     c.gather_world = 0, c.parts = 0, c.part = 0, c.head_group = 0, c.exch_rows = 0;
     c.rot_v = ctx->rot_v;
     c.q = q, c.out = out, c.out_f32 = nullptr;
-    rc = tq_set_combine_tail(c, tail_k, tail_v, n_tail, q_dtype);
+    rc = tq_set_combine_tail(c, tail_k, tail_v, n_tail, q_dtype, (int64_t)cache->batch * cache->kv_heads, ctx->sm_count);
     if (rc) return rc;
     return tq_launch_combine(c, q_dtype, rows, stream, /*programmatic=*/true);
 }

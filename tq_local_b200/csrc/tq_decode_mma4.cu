@@ -737,7 +737,7 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
     c.rot_v = ctx->rot_v;
     c.q = q, c.out = out, c.out_f32 = extras ? extras->out_f32 : nullptr;
     if (c.out_f32 && (gather || n_tail)) return TQ_ERR_UNSUPPORTED;
-    rc = tq_set_combine_tail(c, tail_k, tail_v, n_tail, q_dtype);
+    rc = tq_set_combine_tail(c, tail_k, tail_v, n_tail, q_dtype, a.rows, ctx->sm_count);
     if (rc) return rc;
     return tq_launch_combine(c, q_dtype, rows, stream, /*programmatic=*/true);
 }

@@ -40,6 +40,7 @@ struct CombineArgs {
     const void *tail_k, *tail_v;
     int64_t tk_sb, tk_sh, tk_st, tv_sb, tv_sh, tv_st;
     bool tail_vec;  // every tail row starts on a 16-byte boundary
+    bool tail_rows;  // the tail is attended by tq_combine_row_kernel, a block per query row
     int tail_ctas, tail_per_cta;  // CTAs of a cluster that share a row's tail, and how many tokens each takes
 };
 
@@ -64,6 +65,7 @@ int32_t tq_launch_qprep_frag(tq_ctx *ctx, const void *q, int32_t q_dtype, int64_
                              const TqPackArgs *append, cudaStream_t stream);
 // `programmatic`: launch as a programmatic dependent of the preceding kernel (honoured by the
 // grouped variant, which waits for that kernel before it reads the partials).
-int32_t tq_set_combine_tail(CombineArgs &c, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tail, int32_t q_dtype);
+int32_t tq_set_combine_tail(CombineArgs &c, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tail, int32_t q_dtype,
+                            int64_t kv_rows, int sm_count);
 int32_t tq_launch_combine(const CombineArgs &a, int32_t q_dtype, int64_t rows, cudaStream_t stream,
                           bool programmatic = false);
