@@ -170,6 +170,32 @@ def test_dense_tail_of_padded_rows(setup_golden, dtype, copies, n_tail):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F32])
+def test_tail_alone_after_a_step(setup_golden, dtype):
+    """A tail without packed tokens, right behind a step of another layer whose last kernel starts its successor early and
+    whose output is the tail's newest token: attended as it is after that step."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec = make_codec(4, True, setup_golden)
+    first, second = PackedStore(codec, 1, 4, capacity=40), PackedStore(codec, 1, 4, capacity=8)
+    first.pack(vectors((1, 4, 33, 128), 1, dtype), vectors((1, 4, 33, 128), 2, dtype))
+    qs, tv = [query((1, 4, 1), 10 + i, dtype) for i in range(20)], vectors((1, 4, 5, 128), 4, dtype)
+    q, tk = query((1, 4, 1), 3, dtype), vectors((1, 4, 5, 128), 5, dtype)
+    got, tails = [], []
+    for x in qs:
+        row = torch.empty(1, 4, 1, 128, dtype=dtype, device="cuda")
+        first.decode_attn(x, out=row)
+        got.append(second.decode_attn(q, tail_k=row, tail_v=tv[:, :, :1]))
+        tails.append(row)
+        got.append(second.decode_attn(row, tail_k=tk, tail_v=tv))
+    torch.cuda.synchronize()
+    for i, row in enumerate(tails):
+        assert torch.equal(got[2 * i], tv[:, :, :1])  # one token: its value
+        again = second.decode_attn(row, tail_k=tk, tail_v=tv)
+        torch.cuda.synchronize()
+        assert torch.equal(got[2 * i + 1], again)
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("splits", [1, 2, 8, 9, 31, 32, 33, 41, 70])
 def test_split_merge(setup_golden, dtype, splits):
     """Every remainder of the merge's batches of 8 and 32 partials (one long row, so that the splits are used)."""
