@@ -156,11 +156,11 @@ def test_dense_tail_ranges(setup_golden, dtype, batch, heads, groups, n_tail):
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("copies,n_tail", [(1, 70), (1, 300), (86, 5), (86, 200)])
 def test_dense_tail_of_padded_rows(setup_golden, dtype, copies, n_tail):
-    """A left-padded batch with a tail, few rows and more than there are SMs."""
+    """A left-padded batch with a tail, a row with nothing but its tail among it, few rows and more than there are SMs."""
     from tq_local_b200.runtime.packed_store import PackedStore
 
     p, codec = oracle_params(4, True, setup_golden), make_codec(4, True, setup_golden)
-    starts = [0, 41, 69] * copies
+    starts = [0, 41, 70] * copies
     store = PackedStore(codec, len(starts), 2, capacity=72)
     store.pack(vectors((len(starts), 2, 70, 128), 1, dtype), vectors((len(starts), 2, 70, 128), 2, dtype))
     store.set_seq_start(torch.tensor(starts, dtype=torch.int32, device="cuda"))

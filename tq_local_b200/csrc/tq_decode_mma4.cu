@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
             for (int w = 0; w < kWarps; ++w) {
                 const float mw = s_m[w * 4 + tt];
                 const float sc = (mw == -INFINITY) ? 0.f : fast_exp2(mw - M);
-                Lsum += s_l[w * 4 + tt] * sc;
+                Lsum += (mw == -INFINITY) ? 0.f : s_l[w * 4 + tt] * sc;  // (a warp whose tokens are all masked has summed up undefined weights)
                 A += s_acc[w * 4 * TQ_D + idx] * sc;
             }
             const int64_t prow = (q_row0 + hh) * a.n_splits + split;
