@@ -373,3 +373,24 @@ def test_recorded_steps_of_several_layers(setup_golden, batch, heads, tokens):
             for a, b in zip(s.streams(), p.streams()):
                 assert torch.equal(a[:, :, :tokens + n + 1], b[:, :, :tokens + n + 1])
     assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("bits,qjl,batch,heads,groups,tokens", [(4, True, 4, 8, 4, 500), (4, True, 4, 8, 4, 1000), (4, True, 1, 8, 4, 8191),
+                                                              (4, False, 16, 2, 8, 77), (4, True, 6, 8, 4, 16), (3, True, 4, 4, 7, 2000)])
+def test_chained_attention_calls(setup_golden, bits, qjl, batch, heads, groups, tokens):
+    """Attention calls in a row, on both sides of the line up to which one starts the next early: each gives what it gives alone."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec = make_codec(bits, qjl, setup_golden)
+    stores = [PackedStore(codec, batch, heads, tokens) for _ in range(3)]
+    for i, store in enumerate(stores):
+        store.pack(vectors((batch, heads, tokens, 128), 2 * i, BF16), vectors((batch, heads, tokens, 128), 2 * i + 1, BF16))
+    qs = [query((batch, heads * groups, 1), 50 + i, BF16) for i in range(12)]
+    alone = []
+    for i, q in enumerate(qs):
+        alone.append(stores[i % 3].decode_attn(q))
+        torch.cuda.synchronize()
+    chained = [stores[i % 3].decode_attn(q) for i, q in enumerate(qs)]
+    for a, b in zip(alone, chained):
+        assert torch.equal(a, b)
+    assert codec.device_status() == 0

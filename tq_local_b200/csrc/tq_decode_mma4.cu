@@ -688,9 +688,17 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
     a.centers_k = ctx->centers_k, a.centers_v = ctx->centers_v;
     a.error_flag = ctx->error_flag;
     // (the wait for the peers that follows a gather is not one of the small kernels meant here)
+    // SMs that the combine kernel and the query preparation after it need.  One that also appends fits two blocks to an SM
+    // unless it stages matrices, and starting it early pays then too (16-token step of 4 x 8 rows without the sketch 9.4 us, 10.6 with
+    // its blocks counted singly).  Without an append two blocks to an SM cost more than the early start gives: 4 x 8 x 1000 tokens
+    // with the sketch 12.9 us against 12.1 without any early start, 16 x 2 x 16 of eight heads 11.5 against 10.6; there, and at
+    // eight more sizes on the edge, 0.5 to 0.9 us less when every block is counted.
     const int combine_blocks = a.rows * ((a.G + 3) / 4);
-    const int prologue_blocks = combine_blocks * (ctx->use_qjl ? 2 : 1) + (append ? append->n_kinds * append->B * append->H * append->S : 0);
-    a.sm_count = ctx->sm_count, a.next_blocks = gather || n_tail ? 0 : combine_blocks + (append && tq_stages_matrices(ctx, prologue_blocks) ? prologue_blocks : (prologue_blocks + 1) / 2);
+    const int qprep_blocks = combine_blocks * (ctx->use_qjl ? 2 : 1), append_blocks = append ? append->n_kinds * append->B * append->H * append->S : 0;
+    const int prologue_blocks = qprep_blocks + append_blocks;
+    const bool pairs = append && !tq_stages_matrices(ctx, prologue_blocks);
+    a.sm_count = ctx->sm_count;
+    a.next_blocks = gather || n_tail ? 0 : combine_blocks + (pairs ? (prologue_blocks + 1) / 2 : prologue_blocks);
     a.release_early = n_tail > 0 || (!len_ptr && a.next_blocks && tq_leaves_idle(plan, a.rows, a.sm_count, a.next_blocks));
     a.device = ctx->device;
     // Length on the device: the kernel plans for its own grid.  One CTA per SM, except that a

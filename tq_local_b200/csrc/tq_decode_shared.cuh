@@ -14,8 +14,8 @@ struct CombineArgs {
     // kernel derives seg_chunk / seg_npad itself, with the plan the decode kernel used.
     const int *len_ptr;
     int len_add, capacity, plan_rows, plan_ctas, plan_step;
-    // Small caches leave SMs idle: when `next_blocks` SMs (the combine blocks and the blocks of the query preparation that
-    // may follow, one or two of them to an SM) are free beside the decode kernel's CTAs, that kernel and this one release their
+    // Small caches leave SMs idle: when `next_blocks` SMs (for the combine blocks and the blocks of the query preparation that
+    // may follow) are free beside the decode kernel's CTAs, that kernel and this one release their
     // successors as soon as they start, and these fetch their matrix columns and plans while they wait.
     int sm_count, next_blocks;
     // Peer gather (KV-head sharding): when gather_world > 0 the finished rows go to every rank's
