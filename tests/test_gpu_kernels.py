@@ -68,6 +68,19 @@ def test_key_norm_mean(dtype, shape, form):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("shape", [(1, 1, 8191), (1, 1, 8192), (1, 1, 8193), (2, 5, 819), (2, 5, 820), (4, 8, 5003)])
+@pytest.mark.parametrize("form", ["contiguous", "unaligned"])
+def test_key_norm_mean_of_few_and_many(dtype, shape, form):
+    """Both sides of the size from which a lane makes eight loads, and more vectors than one round of the grid."""
+    from tq_local_b200.runtime.packed_store import key_norm_mean
+
+    x = vectors((*shape, 128), 3, dtype)
+    want = float(x.double().norm(dim=-1).mean())
+    x = off_by_one(x) if form == "unaligned" else x
+    assert abs(float(key_norm_mean(x)) - want) <= 128 * 2.0 ** -24 * want
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
 @pytest.mark.parametrize("groups", [1, 4, 5, 8])
 @pytest.mark.parametrize("n_tail", [1, 63, 64, 255, 256, 257, 700])
 def test_dense_tail(setup_golden, dtype, groups, n_tail):

@@ -246,9 +246,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) tq_dequant_rows_kernel(De
 // 16-byte loads (16 lanes of a 16-bit vector, 32 of an fp32 one), eight loads per lane in flight, and
 // the eight squared sums are reduced together (half of them change hands at every shuffle: 8 shuffles
 // instead of 32).  2.1 M bf16 vectors (537 MB): 107 us = 5.0 TB/s; one vector per warp and 2-byte
-// loads: 442 us.
-constexpr int kNormLoads = 8;
-template <typename T>
+// loads: 442 us.  Few vectors are bound by the latency of one trip instead: LOADS = 1 spreads them over as many warps as there are.
+template <typename T, int LOADS>
 __global__ void __launch_bounds__(256) tq_norm_sum_kernel(const T *x, int64_t sb, int64_t sh, int64_t st, int H, int S,
                                                           int64_t n_vec, bool vec, double *out) {
     constexpr int EPL = 16 / (int)sizeof(T);  // elements per lane
@@ -256,7 +255,7 @@ __global__ void __launch_bounds__(256) tq_norm_sum_kernel(const T *x, int64_t sb
     constexpr int VPL = 32 / LPV;             // vectors per load of a warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, off = (lane % LPV) * EPL;
     double acc = 0.0;
-    constexpr int kVecs = kNormLoads * VPL;  // vectors per warp and iteration
+    constexpr int kVecs = LOADS * VPL;  // vectors per warp and iteration
     for (int64_t v0 = ((int64_t)blockIdx.x * 8 + warp) * kVecs; v0 < n_vec; v0 += (int64_t)gridDim.x * 8 * kVecs) {
         const int64_t first = v0 + lane / LPV;
         int t, h;
@@ -267,9 +266,9 @@ __global__ void __launch_bounds__(256) tq_norm_sum_kernel(const T *x, int64_t sb
         } else {
             t = (int)(first % S), h = (int)((first / S) % H), b = first / ((int64_t)S * H);
         }
-        uint4 raw[kNormLoads];
+        uint4 raw[LOADS];
 #pragma unroll
-        for (int i = 0; i < kNormLoads; ++i) {
+        for (int i = 0; i < LOADS; ++i) {
             raw[i] = make_uint4(0, 0, 0, 0);
             if (first + i * VPL < n_vec) {
                 const T *src = x + b * sb + h * sh + (int64_t)t * st + off;
@@ -287,9 +286,9 @@ __global__ void __launch_bounds__(256) tq_norm_sum_kernel(const T *x, int64_t sb
                 if (++h == H) h = 0, ++b;
             }
         }
-        float ss[kNormLoads];
+        float ss[LOADS];
 #pragma unroll
-        for (int i = 0; i < kNormLoads; ++i) {
+        for (int i = 0; i < LOADS; ++i) {
             const T *e = reinterpret_cast<const T *>(&raw[i]);
             ss[i] = 0.f;
 #pragma unroll
@@ -300,7 +299,7 @@ __global__ void __launch_bounds__(256) tq_norm_sum_kernel(const T *x, int64_t sb
         }
         int o = LPV / 2;
 #pragma unroll
-        for (int n = kNormLoads / 2; n > 0; n >>= 1, o >>= 1) {
+        for (int n = LOADS / 2; n > 0; n >>= 1, o >>= 1) {
             const bool up = lane & o;  // this lane keeps the upper n of its 2n sums, its partner the lower ones
 #pragma unroll
             for (int i = 0; i < n; ++i) {
@@ -327,10 +326,15 @@ __global__ void __launch_bounds__(256) tq_norm_sum_kernel(const T *x, int64_t sb
 template <typename T> void launch_norm_sum(const tq_dense_desc *k, int32_t heads, int32_t n_tokens, int64_t n_vec, double *sum, cudaStream_t s) {
     const int64_t strides = (k->stride_b | k->stride_h | k->stride_t) * (int64_t)sizeof(T);
     const bool vec = !((strides | (int64_t)(uintptr_t)k->data) & 15);
-    const int per_block = 8 * kNormLoads * (sizeof(T) == 4 ? 1 : 2);
+    // (fill of the result and division included, bf16: 616 vectors 5.0 us with one load per lane, 5.7 with eight; 8000: 5.8 and 6.3,
+    // unaligned 6.0 and 7.5; above, the warps have more than one load to make anyway)
+    const int loads = n_vec <= 8192 ? 1 : 8, per_block = 8 * loads * (sizeof(T) == 4 ? 1 : 2);
     const int64_t blocks = (n_vec + per_block - 1) / per_block;
-    tq_norm_sum_kernel<T><<<(unsigned)(blocks < 592 ? blocks : 592), 256, 0, s>>>(
-        (const T *)k->data, k->stride_b, k->stride_h, k->stride_t, heads, n_tokens, n_vec, vec, sum);
+    const unsigned grid = (unsigned)(blocks < 592 ? blocks : 592);
+    if (loads == 1)
+        tq_norm_sum_kernel<T, 1><<<grid, 256, 0, s>>>((const T *)k->data, k->stride_b, k->stride_h, k->stride_t, heads, n_tokens, n_vec, vec, sum);
+    else
+        tq_norm_sum_kernel<T, 8><<<grid, 256, 0, s>>>((const T *)k->data, k->stride_b, k->stride_h, k->stride_t, heads, n_tokens, n_vec, vec, sum);
 }
 
 int grid_for(int64_t items, int sm_count) {
