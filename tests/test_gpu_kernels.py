@@ -257,6 +257,66 @@ def test_prefill_encoder(setup_golden, bits, qjl, dtype, shape):
     check_packed(store, O.pack_layer(k, v, p), k, v, p, f"{bits} {qjl} {dtype} {shape}")
 
 
+def with_boundaries(monkeypatch, setup_golden, bits, qjl, kind):
+    """A codec whose codebooks are not Lloyd-Max ones: what a caller of the C interface may bring."""
+    from types import SimpleNamespace
+
+    import numpy as np
+    from tq_local_b200.runtime import codec as codec_module
+
+    lloyd = codec_module.build_scalar_codebook
+
+    def build(dim, n_bits, grid_size):
+        book = lloyd(dim, n_bits, grid_size)
+        bnd = np.array(book.boundaries, dtype=np.float64)
+        if kind == "close":  # two boundaries a ten-thousandth of the width apart
+            bnd[1] = bnd[0] + 1e-4 * (bnd[-1] - bnd[0])
+        elif kind == "geometric":
+            half = 0.2 * 3.0 ** -np.arange(len(bnd) // 2)
+            bnd = np.concatenate((-half, [0.0], half[::-1]))
+        return SimpleNamespace(centers=book.centers, boundaries=bnd)
+
+    monkeypatch.setattr(codec_module, "build_scalar_codebook", build)
+    return make_codec(bits, qjl, setup_golden)
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("bits,qjl", [(3, False), (4, False), (3, True), (4, True)])
+@pytest.mark.parametrize("kind", ["close", "geometric"])
+def test_prefill_encoder_of_other_codebooks(setup_golden, monkeypatch, dtype, bits, qjl, kind):
+    """Codebooks that no uniform grid separates (the geometric one of seven boundaries: one does): codes against 64 bits, and at
+    the tensor cores' speed (the CUDA-core encoder takes more than ten times as long for these vectors)."""
+    import numpy as np
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    plain, codec = make_codec(bits, qjl, setup_golden), with_boundaries(monkeypatch, setup_golden, bits, qjl, kind)
+    k, v = vectors((1, 8, 9000, 128), 1, dtype), vectors((1, 8, 9000, 128), 2, dtype)
+    store = PackedStore(codec, 1, 8, 9000)
+    store.pack(k, v)
+    for x, codes, n_bits, rot, bnd in ((k, store.k_codes, codec.key_bits, codec.rot_k, codec.bnd_k), (v, store.v_codes, bits, codec.rot_v, codec.bnd_v)):
+        rows, edges = x.double().view(-1, 128), torch.from_numpy(bnd).double().cuda()
+        z = (rows / rows.norm(dim=1, keepdim=True)) @ torch.from_numpy(np.asarray(rot)).double().cuda().T
+        got = torch.from_numpy(O.unpack_codes(codes.reshape(-1, codes.shape[-1]).cpu().numpy(), n_bits, 128).astype(np.int64)).cuda()
+        off = got != torch.bucketize(z, edges)
+        assert not (off & ((z.unsqueeze(-1) - edges).abs().amin(-1) >= 1e-6)).any()
+        assert off.float().mean() < 1e-4
+    assert codec.device_status() == 0
+
+    def fastest(c):
+        s, best = PackedStore(c, 1, 8, 9000), float("inf")
+        for _ in range(12):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            s.length = 0
+            begin.record()
+            s.pack(k, v)
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, begin.elapsed_time(end))
+        return best
+
+    assert fastest(codec) <= 3 * fastest(plain)
+
+
 @pytest.mark.parametrize("dtype", [BF16, F16, F32])
 @pytest.mark.parametrize("qjl", [False, True])
 def test_prefill_encoder_extreme_rows(setup_golden, dtype, qjl):

@@ -177,7 +177,7 @@ int32_t tq_launch_decode_mma4(tq_ctx *ctx, const void *q, int32_t q_dtype, int32
 float tq_fit_power(float largest);  // the power of two that brings `largest` into [2^13, 2^14)
 bool tq_fit_grid(const float *bounds, int n, tq_ctx::Grid *g);
 float tq_build_operand_image(const float *m, uint16_t *image);
-// `k` null: values only.  TQ_ERR_UNSUPPORTED when a tensor's alignment or the codebook rules the kernel out.
+// `k` null: values only.  TQ_ERR_UNSUPPORTED when a tensor's alignment rules the kernel out.
 int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tokens,
                           const tq_cache_desc *cache, int32_t pos0, cudaStream_t stream);
 // TQ_ERR_UNSUPPORTED when the output's alignment rules the kernel out.

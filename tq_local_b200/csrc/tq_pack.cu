@@ -3,8 +3,8 @@
 // tq_pack_rows_kernel is the arithmetic-exact encoder: fp32 accumulation in a
 // fixed order, true division, the reference's tie rule (a value equal to a
 // boundary goes to the lower bin) and the reference's dtype round trip of the
-// reconstruction before the QJL residual.  It serves prefills whose tensors or
-// codebook the tensor-core kernel does not take; appends have a kernel of their own.
+// reconstruction before the QJL residual.  It serves prefills whose tensors
+// the tensor-core kernel does not take; appends have a kernel of their own.
 #include "tq_common.cuh"
 #include "tq_step_blocks.cuh"
 

@@ -118,19 +118,26 @@ __device__ __forceinline__ float fit_power(float v) {
 // in a uniform grid gives the number of boundaries in the cells before it and the one boundary that may lie
 // in its own (tq_fit_grid makes sure that there is no second one); the cell is a monotone function of z and
 // the boundaries' cells are formed by the same instructions, so the answer is that of comparing with all of them.
-// Against a binary search in shared memory this saves five instructions a coordinate at four bits.
+// Against a binary search in shared memory this saves five instructions a coordinate at four bits.  Codebooks that no grid
+// separates take that search (GRID false: four dependent loads, whose sixteen words lie in sixteen banks): 4 x 8 x 32768
+// bf16 keys and values, 4 bits with the sketch, 668 us against 480 (12 ms in the CUDA-core encoder).
 __device__ __forceinline__ uint32_t grid_cell(float z, const tq_ctx::Grid &g) {  // + 0x4B000000
     float t;
     asm("fma.rn.sat.f32 %0, %1, %2, %3;\n" : "=f"(t) : "f"(z), "f"(g.scale), "f"(g.shift));  // (NaN: 0)
     return __float_as_uint(fmaf(t, g.last, 8388608.f));
 }
-template <int BITS, int MUL> struct Search {
+template <int BITS, int MUL, bool GRID> struct Search {
     float b0, b1, b2;
     tq_ctx::Grid grid;
-    uint32_t table;
+    uint32_t table;  // of cells, or the boundaries
     __device__ __forceinline__ Search(const float *bounds, const uint2 *cells, const tq_ctx::Grid &g) : grid(g) {
         b0 = bounds[0], b1 = bounds[1], b2 = bounds[2];
-        table = smem_u32(cells) + 8 * (threadIdx.x % kCellCopies) - (0x4B000000u << 7);
+        table = GRID ? smem_u32(cells) + 8 * (threadIdx.x % kCellCopies) - (0x4B000000u << 7) : smem_u32(bounds);
+    }
+    __device__ __forceinline__ bool below(uint32_t offset, float z) const {  // the boundary at that byte offset
+        float b;
+        asm("ld.shared.f32 %0, [%1];\n" : "=f"(b) : "r"(table + offset));
+        return b < z;
     }
     __device__ __forceinline__ uint32_t operator()(float z) const {
         if (BITS == 1) return b0 < z ? MUL : 0u;
@@ -138,9 +145,17 @@ template <int BITS, int MUL> struct Search {
             const bool up = b1 < z;
             return (up ? 2u * MUL : 0u) + ((up ? b2 : b0) < z ? MUL : 0u);
         }
-        uint32_t bound, below;
-        asm("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(bound), "=r"(below) : "r"(grid_cell(z, grid) * (8u * kCellCopies) + table));
-        return below + (__uint_as_float(bound) < z ? MUL : 0u);
+        if (!GRID) {
+            uint32_t c = 0;  // (four times the boundaries known to be below)
+            if (BITS == 4) c = below(4 * 7, z) ? 32u : 0u;
+            c += below(c + 4 * 3, z) ? 16u : 0u;
+            c += below(c + 4 * 1, z) ? 8u : 0u;
+            c += below(c, z) ? 4u : 0u;
+            return c / 4 * MUL;
+        }
+        uint32_t bound, lower;
+        asm("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(bound), "=r"(lower) : "r"(grid_cell(z, grid) * (8u * kCellCopies) + table));
+        return lower + (__uint_as_float(bound) < z ? MUL : 0u);
     }
 };
 // Fills the grid's table (all threads of the CTA; barriers around it are the caller's).
@@ -198,7 +213,7 @@ struct PackTcShared {
     uint32_t tmem;
 };
 
-template <typename T, int BITS, bool QJL>
+template <typename T, int BITS, bool QJL, bool GRID>
 __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r, PackTcShared &sm, uint32_t images, uint32_t staged, int cta, int n_ctas) {
     using R = Raw<T>;
     constexpr int kTermsX = sizeof(T) == 4 ? 2 : 1;
@@ -288,7 +303,7 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
             for (int i = 0; i < R::kWords; ++i) asm volatile("" : "+r"(raw[i]));
         }
     };
-    const Search<BITS, QJL ? 4 : 1> search(sm.bounds, sm.cells, r.grid);
+    const Search<BITS, QJL ? 4 : 1, GRID> search(sm.bounds, sm.cells, r.grid);
     const int first = cta + n_ctas * group, stride = n_ctas * kGroups;
     if (first < a.n_tiles) request(first);
     int parity = 0;
@@ -461,7 +476,7 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
     if (timed_out) atomicExch(a.error_flag, 3);
 }
 
-template <typename T, int BITS, bool QJL>
+template <typename T, int BITS, bool QJL, bool GRID>
 __global__ void __launch_bounds__(kThreads, 1) tq_pack_tc_kernel(const __grid_constant__ PackTcArgs a) {
     constexpr int KEY_BITS = QJL ? BITS - 1 : BITS;
     extern __shared__ uint8_t smem_raw[];
@@ -496,13 +511,13 @@ __global__ void __launch_bounds__(kThreads, 1) tq_pack_tc_kernel(const __grid_co
     umma_fence_after();
     {
         const int bits = keys ? KEY_BITS : BITS;
-        if (bits > 2) {
+        if (GRID && bits > 2) {
             build_cells(sm.cells, sm.bounds, (1 << bits) - 1, r.grid, QJL && keys ? 4 : 1);
             __syncthreads();
         }
     }
-    if (keys) encode<T, KEY_BITS, QJL>(a, r, sm, images, staged, blockIdx.x, a.key_ctas);
-    else encode<T, BITS, false>(a, r, sm, images, staged, blockIdx.x - a.key_ctas, gridDim.x - a.key_ctas);
+    if (keys) encode<T, KEY_BITS, QJL, GRID>(a, r, sm, images, staged, blockIdx.x, a.key_ctas);
+    else encode<T, BITS, false, GRID>(a, r, sm, images, staged, blockIdx.x - a.key_ctas, gridDim.x - a.key_ctas);
     umma_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -560,25 +575,34 @@ float tq_build_operand_image(const float *m, uint16_t *image) {
     return 1.f / scale;
 }
 
-template <typename T, int BITS, bool QJL>
-static cudaError_t launch_tc(const PackTcArgs &a, int grid, int device, cudaStream_t stream) {
+template <typename T, int BITS, bool QJL, bool GRID>
+static cudaError_t launch_tc_search(const PackTcArgs &a, int grid, int device, cudaStream_t stream) {
     constexpr int smem = (QJL ? 2 : 1) * kUmmaImageBytes + (sizeof(T) == 2 ? kGroups * kStageBytes : 0) + 1024;
     // the attribute belongs to the (kernel, device) pair: one flag per device of this instantiation
     static bool configured[TQ_MAX_DEVICES] = {};
     if (device < 0 || device >= TQ_MAX_DEVICES) return cudaErrorInvalidDevice;
     if (!configured[device]) {
-        cudaError_t e = cudaFuncSetAttribute(tq_pack_tc_kernel<T, BITS, QJL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(tq_pack_tc_kernel<T, BITS, QJL, GRID>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         configured[device] = true;
     }
-    tq_pack_tc_kernel<T, BITS, QJL><<<grid, kThreads, smem, stream>>>(a);
+    tq_pack_tc_kernel<T, BITS, QJL, GRID><<<grid, kThreads, smem, stream>>>(a);
     return cudaGetLastError();
+}
+
+template <typename T, int BITS, bool QJL>
+static cudaError_t launch_tc(const PackTcArgs &a, int grid, int device, cudaStream_t stream, bool cells) {
+    if constexpr (BITS > 2) {
+        if (!cells) return launch_tc_search<T, BITS, QJL, false>(a, grid, device, stream);
+    }
+    return launch_tc_search<T, BITS, QJL, true>(a, grid, device, stream);  // (up to two bits: no search in shared memory at all)
 }
 
 int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc *v, int32_t n_tokens,
                           const tq_cache_desc *cache, int32_t pos0, cudaStream_t stream) {
     const int esize = v->dtype == TQ_DTYPE_F32 ? 4 : 2;
     PackTcArgs a = {};
+    bool cells = true;  // a grid separates the boundaries
     for (int i = 0; i < 2; ++i) {
         const tq_dense_desc *x = i == 0 ? k : v;
         if (!x) continue;
@@ -591,7 +615,7 @@ int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_de
         r.image = image.data, r.unscale = kUmmaRestore * image.unscale;
         r.bounds = i == 0 ? ctx->bounds_k : ctx->bounds_v;
         r.grid = i == 0 ? ctx->grid_k : ctx->grid_v;
-        if ((i == 0 ? ctx->key_bits : ctx->bits) > 2 && r.grid.last == 0.f) return TQ_ERR_UNSUPPORTED;  // (boundaries too close)
+        if ((i == 0 ? ctx->key_bits : ctx->bits) > 2 && r.grid.last == 0.f) cells = false;
     }
     const bool qjl = ctx->use_qjl && k;
     a.vec = vector_index(cache->batch, cache->kv_heads, n_tokens), a.pos0 = pos0;
@@ -615,9 +639,9 @@ int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_de
     cudaError_t e = cudaErrorInvalidValue;
 #define TQ_TC_CASE(T)                                                                                                     \
     switch (ctx->bits) {                                                                                                  \
-        case 2: e = qjl ? launch_tc<T, 2, true>(a, grid, ctx->device, stream) : launch_tc<T, 2, false>(a, grid, ctx->device, stream); break; \
-        case 3: e = qjl ? launch_tc<T, 3, true>(a, grid, ctx->device, stream) : launch_tc<T, 3, false>(a, grid, ctx->device, stream); break; \
-        case 4: e = qjl ? launch_tc<T, 4, true>(a, grid, ctx->device, stream) : launch_tc<T, 4, false>(a, grid, ctx->device, stream); break; \
+        case 2: e = qjl ? launch_tc<T, 2, true>(a, grid, ctx->device, stream, cells) : launch_tc<T, 2, false>(a, grid, ctx->device, stream, cells); break; \
+        case 3: e = qjl ? launch_tc<T, 3, true>(a, grid, ctx->device, stream, cells) : launch_tc<T, 3, false>(a, grid, ctx->device, stream, cells); break; \
+        case 4: e = qjl ? launch_tc<T, 4, true>(a, grid, ctx->device, stream, cells) : launch_tc<T, 4, false>(a, grid, ctx->device, stream, cells); break; \
         default: return TQ_ERR_UNSUPPORTED;                                                                               \
     }
     if (v->dtype == TQ_DTYPE_F32) {
