@@ -397,6 +397,48 @@ def test_dequantisation(setup_golden, bits, qjl, dtype, shape):
     assert codec.device_status() == 0
 
 
+@pytest.mark.parametrize("bits,qjl", MODES)
+@pytest.mark.parametrize("rows", ["gaussian", "one large element", "few large coordinates"])
+def test_fp32_dequantisation_is_as_exact_as_fp32_sums(setup_golden, bits, qjl, rows):
+    """fp32 results against 64 bits, also where every product of a sum has the same sign (codes that follow a row of the
+    rotation, as those of a vector with one large element do): the 2-norm of the errors stays below what 128 fp32
+    multiply-adds one after the other leave, 2.0e-7 of the result (measured over such rows: 1.96e-7 to 2.2e-7)."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec, n = make_codec(bits, qjl, setup_golden), 1 << 16
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    store = PackedStore(codec, 1, 1, n)
+    store.length = n
+    to64 = lambda a: torch.from_numpy(a).double().cuda()
+
+    def pack_bits(idx, b):
+        words = (idx.view(-1, 16, 8) << (b * torch.arange(8, device="cuda"))).sum(-1)
+        return torch.stack([(words >> (8 * i)) & 255 for i in range(b)], -1).to(torch.uint8).view(-1, 16 * b)
+
+    for which, b, rot, cen, codes, norms in (("keys", codec.key_bits, to64(codec.rot_k), to64(codec.cen_k), store.k_codes, store.k_norms),
+                                             ("values", bits, to64(codec.rot_v), to64(codec.cen_v), store.v_codes, store.v_norms)):
+        if rows == "gaussian":
+            z = torch.randn(n, 128, generator=gen, device="cuda", dtype=torch.float64) * 128 ** -0.5
+        elif rows == "one large element":
+            z = 4 * rot.T[torch.randint(0, 128, (n,), generator=gen, device="cuda")]
+        else:
+            x = torch.zeros(n, 128, device="cuda", dtype=torch.float64)
+            x.scatter_(1, torch.randint(0, 128, (n, 4), generator=gen, device="cuda"), torch.randn(n, 4, generator=gen, device="cuda", dtype=torch.float64))
+            z = x / x.norm(dim=1, keepdim=True) @ rot.T
+        idx = torch.bucketize(z, (cen[1:] + cen[:-1]) / 2)
+        norm = (11.3 * torch.exp(0.5 * torch.randn(n, generator=gen, device="cuda"))).half()
+        codes[0, 0].copy_(pack_bits(idx, b)), norms[0, 0].copy_(norm)
+        want = (cen[idx] @ rot) * norm.double()[:, None]
+        if which == "keys" and qjl:
+            sign = torch.randint(0, 2, (n, 128), generator=gen, device="cuda")
+            rnorm = (2 * torch.exp(0.5 * torch.randn(n, generator=gen, device="cuda"))).half()
+            store.k_signs[0, 0].copy_(pack_bits(sign, 1)), store.k_rnorms[0, 0].copy_(rnorm)
+            want += (2 * sign - 1).double() @ to64(codec.qjl) * (math.sqrt(math.pi / 2) / 128) * rnorm.double()[:, None]
+        got = store.dequant(which, dtype=F32)[0, 0].double()
+        assert float((got - want).norm() / want.norm()) <= 1.9e-7, which
+    assert codec.device_status() == 0
+
+
 @pytest.mark.parametrize("dtype", [BF16, F16, F32])
 def test_append_encoder_staging(setup_golden, dtype):
     """Appends of no more vectors than SMs keep the matrices in shared memory, larger ones read them from L2: the same

@@ -36,7 +36,7 @@ struct DequantTcArgs {
     void *out;
     int64_t ob, oh, ot;
     const uint16_t *image, *image2;  // R, S
-    float unscale, unscale2;         // undo the scales of R and the centres, and of S
+    float unscale, unscale2;         // undo the scales of R and the centres (a power of two), and of S
     const float *centers;            // 16 floats
     float cen_scale;
     int *error_flag;
@@ -93,9 +93,17 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
     constexpr bool kStaged = sizeof(T) == 2;
     const uint32_t my_stage = images + (QJL ? 2 : 1) * kUmmaImageBytes + group * kStageBytes + vrow * kStagePitch;
     auto group_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + group), "r"(kGroupThreads) : "memory"); };
-    // Everybody has stored its part of A and read the accumulators of the stage before: two products when A
+    // The tensor core rounds its running sum towards zero at every step.  A row with one large element, whose products all have
+    // one sign, loses 4e-7 of it; the fp32 results' sums of centres come in two pieces of four steps each, which leaves 2e-7, and
+    // half of that is given back by scaling one piece by kUmmaRestore.  Relative to 64 bits, 2-norm over 262144 rows, 3-bit
+    // values: rows with one large element 3.5e-7 in one piece, 1.5e-7 in two (fp32 multiply-adds one after the other: 2.0e-7), Gaussian
+    // rows 1.3e-7 and 1.1e-7 (2.0e-7).  8 x 16384 values 35.3 us in one piece, 37.5 in two.  The signs' sums stay below 1.1e-7 in one.
+    constexpr int kPieces = sizeof(T) == 4 ? 2 : 1;
+    const std::integral_constant<int, 0> first_piece;
+    const std::integral_constant<int, 1> second_piece;
+    // Everybody has stored its part of A and read the accumulators of the stage or piece before: two products when A
     // has one term (the signs), three when it has two.
-    auto gemm = [&](auto terms) {  // stage 0: the centres, two terms; stage 1: the signs, one
+    auto gemm = [&](auto terms, auto piece) {  // stage 0: the centres, two terms; stage 1: the signs, one
         constexpr int kTerms = decltype(terms)::value, stage = 2 - kTerms;
         tmem_st_wait();
         umma_fence_before();
@@ -106,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
                 if (!mbar_wait(smem_u32(&s_bar_image[stage]), 0)) timed_out = true;
                 landed |= 1u << stage;
             }
-            umma_issue<kTerms, true>(acc, a_hi, a_lo, images + stage * kUmmaImageBytes);
+            umma_issue<kTerms, true, decltype(piece)::value, kTerms == 2 ? kPieces : 1>(acc, a_hi, a_lo, images + stage * kUmmaImageBytes);
             umma_commit(bar_mma);
         }
     };
@@ -162,8 +170,8 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
             }
             tmem_st8(my_hi + 8 * c, hi), tmem_st8(my_lo + 8 * c, lo);
         }
-        gemm(std::integral_constant<int, 2>());
-        const float nf = tq_half_bits_to_float(nh) * a.unscale;
+        gemm(std::integral_constant<int, 2>(), first_piece);
+        const float nf = tq_half_bits_to_float(nh) * (sizeof(T) == 4 ? a.unscale : a.unscale * kUmmaRestore);
         const float rf = tq_half_bits_to_float(rh);
         const uint32_t signs = sw;
         T *const to = dst;
@@ -172,17 +180,43 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
         constexpr int kOutWords = kCoords * (int)sizeof(T) / 4;
         uint32_t o[kOutWords];  // this thread's 32 outputs
         const uint64_t nf2 = f32x2(nf, nf);
+        // fp32 results: o = combine(the accumulators, o), two at a time
+        auto accumulators = [&](auto combine) {
+            if constexpr (sizeof(T) == 4) {
+#pragma unroll
+                for (int q = 0; q < kCoords / 16; ++q) {
+                    uint32_t y[16];
+                    tmem_ld16(my_acc + 16 * q, y);
+#pragma unroll
+                    for (int e = 0; e < 16; e += 2) {
+                        uint32_t *p = o + 16 * q + e;
+                        float y0, y1;
+                        f32x2_split(combine(f32x2(__uint_as_float(y[e]), __uint_as_float(y[e + 1])), f32x2(__uint_as_float(p[0]), __uint_as_float(p[1]))), y0, y1);
+                        p[0] = __float_as_uint(y0), p[1] = __float_as_uint(y1);
+                    }
+                }
+            }
+        };
 #pragma unroll
         for (int q = 0; q < kCoords / 16; ++q) {
             uint32_t y[16];
             tmem_ld16(my_acc + 16 * q, y);
 #pragma unroll
             for (int e = 0; e < 16; e += 2) {
-                float y0, y1;
-                f32x2_split(f32x2_mul(f32x2(__uint_as_float(y[e]), __uint_as_float(y[e + 1])), nf2), y0, y1);
-                if constexpr (sizeof(T) == 4) o[16 * q + e] = __float_as_uint(y0), o[16 * q + e + 1] = __float_as_uint(y1);
-                else o[8 * q + e / 2] = pack2<T>(y0, y1);
+                if constexpr (sizeof(T) == 4) {
+                    o[16 * q + e] = y[e], o[16 * q + e + 1] = y[e + 1];
+                } else {
+                    float y0, y1;
+                    f32x2_split(f32x2_mul(f32x2(__uint_as_float(y[e]), __uint_as_float(y[e + 1])), nf2), y0, y1);
+                    o[8 * q + e / 2] = pack2<T>(y0, y1);
+                }
             }
+        }
+        if constexpr (kPieces == 2) {
+            gemm(std::integral_constant<int, 2>(), second_piece);
+            gemm_wait();
+            const uint64_t restore2 = f32x2(kUmmaRestore, kUmmaRestore);
+            accumulators([&](uint64_t y, uint64_t first) { return f32x2_mul(f32x2_fma(first, restore2, y), nf2); });
         }
         if constexpr (QJL) {
             // ---------------- A = signs: f16 1.0 with the complement of the sign bit on top
@@ -194,20 +228,20 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
                 for (int i = 0; i < 8; ++i) s[i] = 0x3C003C00u | ((w << (15 - 2 * i)) & 0x8000u) | ((w << (30 - 2 * i)) & 0x80000000u);
                 tmem_st8(my_hi + 8 * c, s);
             }
-            gemm(std::integral_constant<int, 1>());
+            gemm(std::integral_constant<int, 1>(), first_piece);
             gemm_wait();
             const float scale = 1.2533141373155003f / (float)TQ_D;  // sqrt(pi/2)/D
+            if constexpr (sizeof(T) == 4) {
+                const uint64_t rs2 = f32x2(a.unscale2 * rf * scale, a.unscale2 * rf * scale);
+                accumulators([&](uint64_t y, uint64_t rec) { return f32x2_fma(y, rs2, rec); });
+            } else {
 #pragma unroll
-            for (int q = 0; q < kCoords / 16; ++q) {
-                uint32_t y[16];
-                tmem_ld16(my_acc + 16 * q, y);
+                for (int q = 0; q < kCoords / 16; ++q) {
+                    uint32_t y[16];
+                    tmem_ld16(my_acc + 16 * q, y);
 #pragma unroll
-                for (int e = 0; e < 16; e += 2) {
-                    const float y0 = __uint_as_float(y[e]) * a.unscale2 * rf * scale, y1 = __uint_as_float(y[e + 1]) * a.unscale2 * rf * scale;
-                    if constexpr (sizeof(T) == 4) {
-                        o[16 * q + e] = __float_as_uint(__uint_as_float(o[16 * q + e]) + y0);
-                        o[16 * q + e + 1] = __float_as_uint(__uint_as_float(o[16 * q + e + 1]) + y1);
-                    } else {
+                    for (int e = 0; e < 16; e += 2) {
+                        const float y0 = __uint_as_float(y[e]) * a.unscale2 * rf * scale, y1 = __uint_as_float(y[e + 1]) * a.unscale2 * rf * scale;
                         const float2 r = unpack2<T>(o[8 * q + e / 2]), c = unpack2<T>(pack2<T>(y0, y1));
                         o[8 * q + e / 2] = pack2<T>(r.x + c.x, r.y + c.y);
                     }
@@ -280,7 +314,7 @@ int32_t tq_launch_dequant_tc(tq_ctx *ctx, const tq_cache_desc *cache, int32_t wh
     const tq_ctx::Image &image = key ? ctx->img_rot_k : ctx->img_rot_v;
     a.image = image.data, a.image2 = ctx->img_qjl.data;
     a.cen_scale = key ? ctx->cen_k_scale : ctx->cen_v_scale;
-    a.unscale = kUmmaRestore * image.unscale / a.cen_scale, a.unscale2 = kUmmaRestore * ctx->img_qjl.unscale;
+    a.unscale = image.unscale / a.cen_scale, a.unscale2 = kUmmaRestore * ctx->img_qjl.unscale;
     a.centers = key ? ctx->centers_k : ctx->centers_v;
     a.error_flag = ctx->error_flag;
     const int grid = a.n_tiles < ctx->sm_count ? a.n_tiles : ctx->sm_count;

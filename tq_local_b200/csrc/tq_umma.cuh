@@ -65,19 +65,23 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint32_t a_tmem, uint6
         : "memory");
 }
 // The MMAs of one contraction (one thread): A in `TERMS` f16 terms at a_hi, a_lo, the matrix image at b_addr,
-// out[n] = sum_k vec[k] * image[n][k], or image[k][n] when TRANSPOSED.
-template <int TERMS, bool TRANSPOSED> __device__ __forceinline__ void umma_issue(uint32_t d, uint32_t a_hi, uint32_t a_lo, uint32_t b_addr) {
+// out[n] = sum_k vec[k] * image[n][k], or image[k][n] when TRANSPOSED.  Of PIECES that are summed up outside the
+// tensor core, the first holds the products with a lo term.
+template <int TERMS, bool TRANSPOSED, int PIECE = 0, int PIECES = 1>
+__device__ __forceinline__ void umma_issue(uint32_t d, uint32_t a_hi, uint32_t a_lo, uint32_t b_addr) {
     const uint64_t desc = umma_desc<TRANSPOSED>(b_addr);
-    auto pass = [&](uint32_t a, uint32_t b_offset, uint32_t first) {
+    auto pass = [&](uint32_t a, uint32_t b_offset, uint32_t first, uint32_t from, uint32_t to) {
 #pragma unroll
-        for (uint32_t s = 0; s < 8; ++s) {  // (the address field counts 16-byte units and does not overflow)
+        for (uint32_t s = from; s < to; ++s) {  // (the address field counts 16-byte units and does not overflow)
             const uint32_t step = TRANSPOSED ? s * 16 * 128 : (s >> 2) * kUmmaSlabBytes + (s & 3) * 32;
-            umma_f16(d, a + 8 * s, desc + ((b_offset + step) >> 4), umma_instr<TRANSPOSED>(), first | (s > 0));
+            umma_f16(d, a + 8 * s, desc + ((b_offset + step) >> 4), umma_instr<TRANSPOSED>(), first | (s > from));
         }
     };
-    pass(a_hi, kUmmaTermBytes, 0);
-    if (TERMS == 2) pass(a_lo, 0, 1);
-    pass(a_hi, 0, 1);
+    if (PIECE == 0) {
+        pass(a_hi, kUmmaTermBytes, 0, 0, 8);
+        if (TERMS == 2) pass(a_lo, 0, 1, 0, 8);
+    }
+    pass(a_hi, 0, PIECE == 0, 8 * PIECE / PIECES, 8 * (PIECE + 1) / PIECES);
 }
 // The tensor core's accumulator drops what lies below its last place (rounds towards zero), which leaves a
 // result of eight full-size steps 1.5e-7 to 1.7e-7 too small on average (the slope of result against 64 bits,
