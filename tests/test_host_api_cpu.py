@@ -235,3 +235,53 @@ def test_unpacked_qmse_variant_matches_the_reference():
     assert out.metrics.variant == "qmse" and out.metrics.qmse_bits == int(g.z["gen_qmse_bits"])
     assert sorted(out.metrics.to_dict().keys()) == list(g.z["gen_metrics_keys"])
     assert out.metrics.turboquant_mse_packed_actual is None and out.metrics.reconstruction_quality is None
+
+
+class _PlanLibrary:
+    """Stands in for the library: a split every 256 tokens, a byte of scratch per head and split."""
+
+    def tq_decode_suggest_splits(self, handle, batch, kv_heads, seq_len):
+        return -(-seq_len // 256)
+
+    def tq_decode_workspace_bytes(self, batch, q_heads, splits):
+        return q_heads * splits
+
+
+def _plan_store(monkeypatch, base=None):
+    from types import SimpleNamespace
+
+    from tq_local_b200.runtime import ffi, packed_store
+
+    monkeypatch.setattr(ffi, "lib", lambda: _PlanLibrary())
+    calls = []
+
+    class Store(base or packed_store.PackedStore):
+        def _call(self, name, *args):
+            calls.append((args[3], args[8], args[9], args[11]))  # query heads, tail tokens, splits, scratch bytes
+
+    codec = SimpleNamespace(device=torch.device("cpu"), handle=None, use_qjl=True, key_bits=3, bits=4)
+    return Store(codec, 1, 2, capacity=8), calls
+
+
+def test_attention_plan_replaced_by_another_thread(monkeypatch):
+    """Two threads may attend through one store: a call keeps to the plan that it has looked at."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    class Raced(PackedStore):  # every look at the plan after a call's first finds another thread's, of fewer heads and splits
+        looks, mine = 0, None
+
+        @property
+        def _attn_plan(self):
+            self.looks += 1
+            return self.mine if self.looks == 1 else ((2, None, 1), 1, 2)
+
+        @_attn_plan.setter
+        def _attn_plan(self, plan):
+            self.mine = plan
+
+    store, calls = _plan_store(monkeypatch, Raced)
+    q = torch.zeros(1, 4, 1, 128, dtype=torch.bfloat16)
+    for _ in range(2):  # a new plan, then the kept one
+        store.looks = 0
+        store.decode_attn(q, seq_len=1000)
+        assert calls[-1][0] == 4 and calls[-1][2] == 4 and calls[-1][3] >= 16

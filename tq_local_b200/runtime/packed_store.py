@@ -187,10 +187,11 @@ class PackedStore:
             tk_ref = tv_ref = None
         # the split count and the scratch size only change when the length crosses a kernel step
         key = (hq, splits, (n + 511) >> 9)
-        if self._attn_plan is None or self._attn_plan[0] != key:
+        plan = self._attn_plan  # (read once: another thread may replace it)
+        if plan is None or plan[0] != key:
             splits = self.suggest_splits(n) if splits is None else int(splits)
-            self._attn_plan = (key, splits, int(ffi.lib().tq_decode_workspace_bytes(b, hq, splits)))
-        _, splits, need = self._attn_plan
+            plan = self._attn_plan = (key, splits, int(ffi.lib().tq_decode_workspace_bytes(b, hq, splits)))
+        _, splits, need = plan
         ws = self._workspace
         if ws is None or ws.numel() < need:
             ws = self._get_workspace(hq, splits)
