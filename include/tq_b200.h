@@ -133,6 +133,9 @@ int32_t tq_pack(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_desc *v, int
 size_t tq_decode_workspace_bytes(int32_t batch, int32_t q_heads, int32_t n_splits);
 /* A split count that fills the GPU for this shape (>= 1). */
 int32_t tq_decode_suggest_splits(tq_ctx *ctx, int32_t batch, int32_t kv_heads, int32_t seq_len);
+/* Tokens of a row that a decode CTA takes per step: tq_decode_suggest_splits is the same for all
+ * lengths that round up to the same multiple of it. */
+int32_t tq_decode_tokens_per_step(void);
 
 /* One decode step of attention straight from the packed cache.
  *   q     : [batch, q_heads, 128] contiguous, dtype q_dtype (one query token per sequence)

@@ -509,3 +509,14 @@ def test_chained_attention_calls(setup_golden, bits, qjl, batch, heads, groups, 
     for a, b in zip(alone, chained):
         assert torch.equal(a, b)
     assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("batch,heads", [(1, 1), (1, 8), (7, 4), (16, 8), (75, 4)])
+def test_split_count_within_a_kernel_step(setup_golden, batch, heads):
+    """What an attention call may keep: the suggested split count changes only between multiples of the kernel's step."""
+    from tq_local_b200.runtime import ffi
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    store, step = PackedStore(make_codec(4, True, setup_golden), batch, heads, 8), ffi.lib().tq_decode_tokens_per_step()
+    for k in list(range(40)) + [100, 255]:
+        assert len({store.suggest_splits(n) for n in (k * step + 1, k * step + 2, k * step + step // 2, k * step + step - 1, (k + 1) * step)}) == 1

@@ -240,6 +240,9 @@ def test_unpacked_qmse_variant_matches_the_reference():
 class _PlanLibrary:
     """Stands in for the library: a split every 256 tokens, a byte of scratch per head and split."""
 
+    def tq_decode_tokens_per_step(self):
+        return 256
+
     def tq_decode_suggest_splits(self, handle, batch, kv_heads, seq_len):
         return -(-seq_len // 256)
 
@@ -261,6 +264,15 @@ def _plan_store(monkeypatch, base=None):
 
     codec = SimpleNamespace(device=torch.device("cpu"), handle=None, use_qjl=True, key_bits=3, bits=4)
     return Store(codec, 1, 2, capacity=8), calls
+
+
+def test_attention_plan_follows_the_kernel_step(monkeypatch):
+    """The kept split count is that of the length at hand, whatever step the library's kernel has."""
+    store, calls = _plan_store(monkeypatch)
+    q = torch.zeros(1, 4, 1, 128, dtype=torch.bfloat16)
+    for n, splits in ((200, 1), (256, 1), (257, 2), (400, 2), (512, 2), (513, 3), (100, 1)):
+        store.decode_attn(q, seq_len=n)
+        assert calls[-1][2] == splits and calls[-1][3] >= 4 * splits, n
 
 
 def test_attention_plan_replaced_by_another_thread(monkeypatch):

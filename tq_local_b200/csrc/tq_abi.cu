@@ -241,6 +241,8 @@ extern "C" int32_t tq_decode_suggest_splits(tq_ctx *ctx, int32_t batch, int32_t 
     return (int32_t)(splits > 1024 ? 1024 : splits);
 }
 
+extern "C" int32_t tq_decode_tokens_per_step(void) { return tq_mma4_tokens_per_cta_step(); }
+
 extern "C" int32_t tq_device_status(tq_ctx *ctx, int32_t *status_out) {
     if (!ctx || !status_out) return TQ_ERR_ARG;
     int v = 0;

@@ -19,7 +19,7 @@ TQ_MAX_GROUPS = 8
 
 EXPORTS = (
     "tq_abi_version", "tq_last_cuda_error", "tq_ctx_create", "tq_ctx_destroy", "tq_pack",
-    "tq_decode_workspace_bytes", "tq_decode_suggest_splits", "tq_decode_attn", "tq_dequant",
+    "tq_decode_workspace_bytes", "tq_decode_suggest_splits", "tq_decode_tokens_per_step", "tq_decode_attn", "tq_dequant",
     "tq_key_norm_sum", "tq_profile_enable", "tq_profile_read", "tq_device_status", "tq_static_scratch_bytes",
     "tq_decode_attn_static", "tq_decode_step_workspace_bytes", "tq_decode_step_host", "tq_decode_step_dev",
     "tq_peer_buffer_create", "tq_peer_buffer_open", "tq_peer_buffer_close", "tq_peer_buffer_destroy",
@@ -97,6 +97,8 @@ def lib() -> C.CDLL:
     L.tq_decode_workspace_bytes.restype = C.c_size_t
     L.tq_decode_suggest_splits.argtypes = [C.c_void_p, C.c_int32, C.c_int32, C.c_int32]
     L.tq_decode_suggest_splits.restype = C.c_int32
+    L.tq_decode_tokens_per_step.argtypes = []
+    L.tq_decode_tokens_per_step.restype = C.c_int32
     L.tq_decode_attn.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.POINTER(CacheDesc), C.c_int32,
                                  C.POINTER(DenseDesc), C.POINTER(DenseDesc), C.c_int32, C.c_int32,
                                  C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]

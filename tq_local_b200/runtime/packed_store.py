@@ -40,6 +40,7 @@ class PackedStore:
         self._workspace: torch.Tensor | None = None
         self._step_plan = None
         self._attn_plan = None  # (what it depends on, split count, scratch bytes) of the last decode_attn
+        self._step_tokens = int(ffi.lib().tq_decode_tokens_per_step())
 
     # ------------------------------------------------------------------ storage
     def _alloc(self, capacity: int) -> None:
@@ -186,7 +187,7 @@ class PackedStore:
         else:
             tk_ref = tv_ref = None
         # the split count and the scratch size only change when the length crosses a kernel step
-        key = (hq, splits, (n + 511) >> 9)
+        key = (hq, splits, -(-n // self._step_tokens))
         plan = self._attn_plan  # (read once: another thread may replace it)
         if plan is None or plan[0] != key:
             splits = self.suggest_splits(n) if splits is None else int(splits)
