@@ -516,7 +516,8 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
     }
     tq_grid_dependency_wait();
     {   // thread (e, dq) merges the splits of head dq.  Up to four, the usual number with many rows: everything is
-        // requested in one batch and merged in registers (8 x 8 x 32768: 0.2 us less than the other way).  More: 32 at a
+        // requested in one batch and merged in registers (sixty pairs of runs each: 0.65 +- 0.08 us less than the other way for
+        // 8 x 8 x 32768 tokens, 0.45 to 0.6 +- 0.02 for six smaller caches, 1.5 for 64 x 8 x 500 of one head).  More: 32 at a
         // time, lane s of each warp holds split s's maximum and weight, the accumulator columns are requested
         // eight splits at a time.  (The kernel takes 5.6 us for 33 splits of 4 rows; with one thread walking all
         // splits twice it took 10.8, with maxima, sums and columns of eight splits in every thread 1.1 us more.)
