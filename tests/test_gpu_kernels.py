@@ -211,7 +211,7 @@ def test_tail_alone_after_a_step(setup_golden, dtype):
 @pytest.mark.parametrize("dtype", [BF16, F32])
 @pytest.mark.parametrize("splits", [1, 2, 8, 9, 31, 32, 33, 41, 70])
 def test_split_merge(setup_golden, dtype, splits):
-    """Every remainder of the merge's batches of 8 and 32 partials (one long row, so that the splits are used)."""
+    """Split counts around the merge's batches of 8 and 32 partials (fp32: as many partials; bf16: fewer, see the next)."""
     from tq_local_b200.runtime.packed_store import PackedStore
 
     p, codec = oracle_params(3, True, setup_golden), make_codec(3, True, setup_golden)
@@ -439,19 +439,135 @@ def test_fp32_dequantisation_is_as_exact_as_fp32_sums(setup_golden, bits, qjl, r
     assert codec.device_status() == 0
 
 
+MANY = (1, 8, 16001)  # 1001 tiles of 128 vectors, the last of 8: three tiles and more for each group of warps of either kernel
+
+
+def unpack_on_gpu(codes, bits):
+    """[..., 16 * bits] code bytes -> [vectors, 128] indices."""
+    b = codes.reshape(-1, 16, bits).long()
+    words = sum(b[..., i] << (8 * i) for i in range(bits))
+    return ((words.unsqueeze(-1) >> (bits * torch.arange(8, device=codes.device))) & ((1 << bits) - 1)).reshape(-1, 128)
+
+
+def tables64(codec):
+    return {name: torch.from_numpy(getattr(codec, name)).double().cuda() for name in ("rot_k", "rot_v", "cen_k", "cen_v", "bnd_k", "bnd_v")}
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("bits,qjl", MODES)
+def test_prefill_encoder_of_many_tiles(setup_golden, bits, qjl, dtype):
+    """Every group of warps walks several tiles: codes and norms against 64 bits; signs and residual norms against the
+    CUDA-core encoder (which takes the same vectors when they are not 16-byte aligned).  A tile's rows under another tile's
+    number, or a tile encoded twice, differ in half of the sign bits and in most codes."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec = make_codec(bits, qjl, setup_golden)
+    t = tables64(codec)
+    k, v = vectors((*MANY, 128), 1, dtype), vectors((*MANY, 128), 2, dtype)
+    store, exact = (PackedStore(codec, MANY[0], MANY[1], MANY[2] + 3) for _ in range(2))
+    for s in (store, exact):
+        s.pack(k[:, :, :3], v[:, :, :3])  # (an odd position to append at)
+    store.pack(k, v)
+    exact.pack(off_by_one(k), off_by_one(v))
+    same = torch.ones(k[..., 0].numel(), dtype=torch.bool, device="cuda")
+    for x, codes, norms, n_bits, rot, edges in ((k, store.k_codes, store.k_norms, codec.key_bits, t["rot_k"], t["bnd_k"]),
+                                                (v, store.v_codes, store.v_norms, bits, t["rot_v"], t["bnd_v"])):
+        rows = x.double().view(-1, 128)
+        norm = rows.norm(dim=1)
+        z = rows / norm[:, None] @ rot.T
+        off = unpack_on_gpu(codes[:, :, 3:MANY[2] + 3], n_bits) != torch.bucketize(z, edges)
+        assert not (off & ((z.unsqueeze(-1) - edges).abs().amin(-1) >= 1e-6)).any() and off.float().mean() < 1e-4
+        ulps = norms[:, :, 3:MANY[2] + 3].reshape(-1).view(torch.int16).int() - norm.half().view(torch.int16).int()
+        assert ulps.abs().max() <= 1
+    if qjl:
+        cut = lambda s, name: getattr(s, name)[:, :, 3:MANY[2] + 3]
+        same = (cut(store, "k_codes") == cut(exact, "k_codes")).all(-1) & (cut(store, "k_norms") == cut(exact, "k_norms"))
+        flips = (unpack_on_gpu(cut(store, "k_signs"), 1) != unpack_on_gpu(cut(exact, "k_signs"), 1)).sum(-1).view(same.shape)
+        ulps = (cut(store, "k_rnorms").view(torch.int16).int() - cut(exact, "k_rnorms").view(torch.int16).int()).abs()
+        # (a residual whose reconstruction rounds to the other neighbour in a few of its elements: some signs near zero)
+        assert same.float().mean() > 0.99 and flips[same].max() <= 16 and flips[same].float().mean() < 0.128
+        assert (ulps[same] <= 1).float().mean() > 0.999
+    assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("bits,qjl", MODES)
+def test_dequantisation_of_many_tiles(setup_golden, bits, qjl, dtype):
+    """The same for the dequantisation, every element against 64 bits, from an odd token on."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec = make_codec(bits, qjl, setup_golden)
+    t = tables64(codec)
+    store = PackedStore(codec, MANY[0], MANY[1], MANY[2] + 3)
+    store.pack(vectors((MANY[0], MANY[1], MANY[2] + 3, 128), 1, dtype), vectors((MANY[0], MANY[1], MANY[2] + 3, 128), 2, dtype))
+    cut = lambda x: x[:, :, 3:MANY[2] + 3]
+    unit = {F32: 2.0 ** -24, F16: 2.0 ** -11, BF16: 2.0 ** -8}[dtype]
+    for which, b, rot, cen, codes, norms in (("keys", codec.key_bits, t["rot_k"], t["cen_k"], store.k_codes, store.k_norms),
+                                             ("values", bits, t["rot_v"], t["cen_v"], store.v_codes, store.v_norms)):
+        want = (cen[unpack_on_gpu(cut(codes), b)] @ rot) * cut(norms).reshape(-1, 1).double()
+        rounded = want.abs()  # what is rounded to the type on the way
+        if which == "keys" and qjl:
+            part = 2.0 * unpack_on_gpu(cut(store.k_signs), 1).double() - 1.0
+            part = part @ torch.from_numpy(codec.qjl).double().cuda() * (math.sqrt(math.pi / 2) / 128) * cut(store.k_rnorms).reshape(-1, 1).double()
+            want = want + part
+            rounded += part.abs() + want.abs()
+        got = store.dequant(which, 3, dtype=dtype).double().view(-1, 128)
+        # fp32 sums of 128 products (as in test_dequantisation), half a place of every rounding, fp16 subnormals
+        room = 2e-6 * want.abs().max() + 1.01 * unit * rounded + 2.0 ** -24
+        assert ((got - want).abs() <= room).all(), which
+    assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [BF16, F32])
+@pytest.mark.parametrize("partials", [1, 2, 3, 4, 5, 8, 9, 31, 32, 33, 64, 65])
+def test_merge_of_every_number_of_partials(setup_golden, dtype, partials):
+    """One long row cut into exactly that many partials: the kernel's step times ``partials`` tokens (the last partial of few)
+    and one split more, so that a CTA takes one step."""
+    from tq_local_b200.runtime import ffi
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    step = ffi.lib().tq_decode_tokens_per_step()
+    p, codec = oracle_params(3, True, setup_golden), make_codec(3, True, setup_golden)
+    n = step * (partials - 1) + 3
+    store = PackedStore(codec, 1, 1, capacity=n)
+    store.pack(vectors((1, 1, n, 128), 1, dtype), vectors((1, 1, n, 128), 2, dtype))
+    q = query((1, 5, 1), 3, dtype)
+    # 16-bit: the plan needs at least ceil(step / (splits - 1)) tokens a partial; fp32: splits partials
+    splits = partials + 1 if dtype == BF16 else partials
+    assert rel_inf(store.decode_attn(q, splits=splits), attend64(store, p, q, 5)) <= ATTN_TOL[dtype]
+
+
+@pytest.mark.parametrize("batch,tokens", [(23, 2100), (10, 5582), (3, 23964)])
+def test_merge_of_rows_cut_at_different_places(setup_golden, batch, tokens):
+    """Chunks that begin inside rows, so that rows have different numbers of partials: two and three, four and five (on
+    both sides of what is merged at once), sixteen and seventeen, with 148 SMs."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(4, True, setup_golden), make_codec(4, True, setup_golden)
+    store = PackedStore(codec, batch, 3, capacity=tokens)
+    store.pack(vectors((batch, 3, tokens, 128), 1, BF16), vectors((batch, 3, tokens, 128), 2, BF16))
+    q = query((batch, 15, 1), 3, BF16)
+    want = attend64(store, p, q, 5)
+    for splits in (None, 2, 7):
+        assert rel_inf(store.decode_attn(q, splits=splits), want) <= ATTN_TOL[BF16], splits
+
+
 @pytest.mark.parametrize("dtype", [BF16, F16, F32])
 def test_append_encoder_staging(setup_golden, dtype):
     """Appends of no more vectors than SMs keep the matrices in shared memory, larger ones read them from L2: the same
-    bits (two 74-vector tensors against two of 76; 148 SMs)."""
+    bits."""
     from tq_local_b200.runtime.packed_store import PackedStore
 
     codec = make_codec(4, True, setup_golden)
-    k, v = vectors((1, 2, 38, 128), 1, dtype), vectors((1, 2, 38, 128), 2, dtype)
-    few, more = PackedStore(codec, 1, 2, 40), PackedStore(codec, 1, 2, 40)
-    few.pack(k[:, :, :37], v[:, :, :37])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = sms // 4  # tokens of two heads, keys and values: 4 n blocks
+    assert 4 * n <= sms < 4 * (n + 1)
+    k, v = vectors((1, 2, n + 1, 128), 1, dtype), vectors((1, 2, n + 1, 128), 2, dtype)
+    few, more = PackedStore(codec, 1, 2, n + 8), PackedStore(codec, 1, 2, n + 8)
+    few.pack(k[:, :, :n], v[:, :, :n])
     more.pack(k, v)
     for a, b in zip(few.streams(), more.streams()):
-        assert torch.equal(a[:, :, :37], b[:, :, :37])
+        assert torch.equal(a[:, :, :n], b[:, :, :n])
     assert codec.device_status() == 0
 
 
