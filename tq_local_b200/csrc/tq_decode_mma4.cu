@@ -577,7 +577,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
         float l_all = l_run[hl];
 #pragma unroll
         for (int sft = 4; sft <= 16; sft <<= 1) l_all += __shfl_xor_sync(0xffffffffu, l_all, sft);
-        if (g == 0) s_m[warp * 4 + t] = m_run[hl], s_l[warp * 4 + t] = l_all;
+        // (a warp whose tokens are all masked has summed up undefined weights)
+        if (g == 0) s_m[warp * 4 + t] = m_run[hl], s_l[warp * 4 + t] = m_run[hl] == -INFINITY ? 0.f : l_all;
         // A warp's 512 accumulators are laid out [mt][lane][2], so the 8-byte stores of a warp
         // and the reads of 32 consecutive elements below both touch every bank once.
 #pragma unroll
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
             for (int w = 0; w < kWarps; ++w) {
                 const float mw = s_m[w * 4 + tt];
                 const float sc = (mw == -INFINITY) ? 0.f : fast_exp2(mw - M);
-                Lsum += (mw == -INFINITY) ? 0.f : s_l[w * 4 + tt] * sc;  // (a warp whose tokens are all masked has summed up undefined weights)
+                Lsum += s_l[w * 4 + tt] * sc;
                 A += s_acc[w * 4 * TQ_D + idx] * sc;
             }
             const int64_t prow = (q_row0 + hh) * a.n_splits + split;
