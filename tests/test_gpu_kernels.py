@@ -491,6 +491,37 @@ def test_prefill_encoder_of_many_tiles(setup_golden, bits, qjl, dtype):
 
 
 @pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("rows", ["gaussian", "four outlier channels", "four coordinates of 128"])
+def test_prefill_encoder_is_as_exact_as_three_terms(setup_golden, dtype, rows):
+    """How often the encoder's fp32-like sums decide otherwise than 64 bits do, over 16.8 M coordinates.  Measured over twice as
+    many, any of these rows: 3 to 17 codes and 51 to 80 signs (fp32 rows, which round no reconstruction, 9 to 14); with operands
+    in three bf16 terms 5 to 89 codes and 257 to 410 signs (38 to 53).  The limits lie between, for half as many."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    codec, n = make_codec(4, True, setup_golden), 1 << 17
+    t = tables64(codec)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(n, 128, generator=gen, device="cuda")
+    if rows == "four outlier channels":
+        x[:, [3, 40, 77, 101]] *= 30
+    elif rows == "four coordinates of 128":
+        x = torch.zeros_like(x).scatter_(1, torch.randint(0, 128, (n, 4), generator=gen, device="cuda"), x[:, :4])
+    x = x.to(dtype)
+    store = PackedStore(codec, 1, 1, n)
+    store.pack(x.view(1, 1, n, 128), x.view(1, 1, n, 128))
+    x64 = x.double()
+    unit = x64 / x64.norm(dim=1, keepdim=True)
+    key_codes = unpack_on_gpu(store.k_codes, codec.key_bits)
+    assert int((key_codes != torch.bucketize(unit @ t["rot_k"].T, t["bnd_k"])).sum()) <= 20
+    assert int((unpack_on_gpu(store.v_codes, 4) != torch.bucketize(unit @ t["rot_v"].T, t["bnd_v"])).sum()) <= 20
+    rec = ((t["cen_k"][key_codes] @ t["rot_k"]) * store.k_norms.view(-1, 1).double()).float().to(dtype).double()
+    projected = (x64 - rec) @ torch.from_numpy(codec.qjl).double().cuda().T
+    off = int((unpack_on_gpu(store.k_signs, 1).bool() != (projected >= 0)).sum())
+    assert off <= (16 if dtype == F32 else 80)
+    assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
 @pytest.mark.parametrize("bits,qjl", MODES)
 def test_dequantisation_of_many_tiles(setup_golden, bits, qjl, dtype):
     """The same for the dequantisation, every element against 64 bits, from an odd token on."""
