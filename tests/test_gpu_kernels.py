@@ -240,6 +240,21 @@ def test_fp32_attention(setup_golden, bits, qjl, groups, n):
 MODES = [(2, False), (3, False), (4, False), (2, True), (3, True), (4, True)]
 
 
+@pytest.mark.parametrize("bits,qjl", [(2, False), (3, False), (4, False), (2, True), (3, True), (4, True)])
+@pytest.mark.parametrize("groups", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("n", [1, 6, 17, 31, 33, 130, 513])
+def test_16bit_attention_unrounded(setup_golden, bits, qjl, groups, n):
+    """The tensor-core kernels at every code width, on both sides of a tile, a warp's tokens and a step, against 64 bits."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    dtype = (BF16, F16)[(n + groups) % 2]
+    p, codec = oracle_params(bits, qjl, setup_golden), make_codec(bits, qjl, setup_golden)
+    store = PackedStore(codec, 2, 3, capacity=n)
+    store.pack(vectors((2, 3, n, 128), 5 + n, dtype), vectors((2, 3, n, 128), 6 + n, dtype))
+    q = query((2, 3 * groups, 1), 7 + n, dtype)
+    assert rel_inf(store.decode_attn_f32(q), attend64(store, p, q, groups)) <= 2e-3
+
+
 @pytest.mark.parametrize("dtype", [BF16, F16, F32])
 @pytest.mark.parametrize("bits,qjl", MODES)
 @pytest.mark.parametrize("shape", [(1, 1, 1024), (1, 8, 129), (3, 5, 127)])

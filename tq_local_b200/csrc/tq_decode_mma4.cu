@@ -23,15 +23,20 @@
 //            (a mask keeps sign bit n of each of four bytes in place, so an operand byte is
 //            2^n or 0 and costs one logic instruction per four signs; the projected query is
 //            16-bit fixed point in two s8 terms, divided by 2^n behind bit n, n = 0..3)
-//   values   O^T[128 x (4 heads x {P, 0})] += Vdeq^T[128 x 16 tok] * P                   f16 m16n8k16
+//   values   O^T[64 pairs of coordinates x (4 heads x parity)] += Vdeq^T[64 x (8 tok x parity)] * P   f16 m16n8k16
+//            (K runs over a token's two coordinates of a pair as well as over tokens, and a column takes the weight
+//            at its own parity and 0 at the other: as many MMAs as with a row per coordinate and half of the columns empty)
 // A operands are built in registers from the packed words.  The contraction order of an
 // MMA is free, so every lane gets codes that sit together in memory:
 //   keys    lane (g, t): dims [32t, 32t+32) of two tokens of a 16-token tile; two
 //           neighbouring codes index a per-lane-replicated shared-memory table of f16x2
 //           centre pairs (slot e, lane l -> bank l: no bank conflicts);
-//   values  lane (g, t): dims [16g, 16g+16) of tokens t, t+4, t+8, t+12; the codes of two
-//           tokens are interleaved with bit-selects so one look-up yields the (token a,
-//           token b) f16x2 that the MMA wants along its K axis.
+//   values  lane (g, t): dims [16g, 16g+16) of tokens t, t+4, t+8, t+12; two neighbouring codes of a token
+//           index the table as they lie in memory.  (With a row per coordinate, K runs over tokens alone and the codes of
+//           two tokens have to be interleaved first, 16 instructions per 16 tokens, and twice the accumulator registers are
+//           held: 8 x 8 x 32768 tokens 80.2 - 81.5 us instead of 75.3 - 78.8, 4 x 8 x 131072 at 3 bits 146.2 instead of 140.0, query
+//           preparation to output.  The wide variant needs all eight columns for its heads and keeps that form; with pairs it takes twice
+//           the value MMAs, 55.1 -> 56.4 us for 8 x 4 x 32768 of seven heads.)
 // Softmax is online, base 2, in registers; P*|v| goes to f16 and is transposed with
 // movmatrix.  Per-CTA partials (max, sum, acc) go to the workspace; tq_combine_group_kernel
 // merges splits, un-rotates and casts.
@@ -314,6 +319,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
     const float kB = kA * (1.2533141373155003f / (float)TQ_D);     // ... * sqrt(pi/2)/D
     const uint32_t lane_k = kTableAddr + lane * 4;        // key copies: bytes [0, 128) of every slot
     const uint32_t lane_v = kTableAddr + 128 + lane * 4;  // value copies: bytes [128, 256)
+    // column g of a value MMA (narrow) is coordinate parity g % 2 of head g / 2: which half of its operand is not 0
+    const uint32_t sel_first = g & 1 ? 0x1044u : 0x4410u, sel_second = g & 1 ? 0x3244u : 0x4432u;
     bool timed_out = false;
     bool first_segment = true;
 
@@ -385,9 +392,11 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
     float m_run[NH], l_run[NH];
 #pragma unroll
     for (int hl = 0; hl < NH; ++hl) m_run[hl] = -INFINITY, l_run[hl] = 0.f;
-    float o[8][4];
+    // narrow: o[mt][j] = coordinate 16g + 4mt + j of head t; wide: o[mt][2 * r + hl] = coordinate 16g + 2mt + r of head 2t + hl
+    constexpr int kAcc = WIDE ? 8 : 4;
+    float o[kAcc][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    for (int i = 0; i < kAcc; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
 
     for (int it = 0; it < n_iter; ++it) {
         const int base = my_first + it * kCtaStep;
@@ -423,7 +432,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
                 for (int w = 0; w < KB; ++w) wa[w] = pa[w], wb[w] = pb[w];
                 wa[KB] = wb[KB] = 0;
             }
-            float d1[4] = {0.f, 0.f, 0.f, 0.f};
+            float d1[4];
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
                 constexpr int W = 2 * KB;
@@ -432,7 +441,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
                 const uint32_t a1 = lds_abs(slot_addr(wb, o0, lane_k));
                 const uint32_t a2 = lds_abs(slot_addr(wa, o1, lane_k));
                 const uint32_t a3 = lds_abs(slot_addr(wb, o1, lane_k));
-                mma_f16(d1, a0, a1, a2, a3, bq[s][0], bq[s][1]);
+                if (s == 0) mma_f16_first(d1, a0, a1, a2, a3, bq[s][0], bq[s][1]);
+                else mma_f16(d1, a0, a1, a2, a3, bq[s][0], bq[s][1]);
             }
             float lgA[NH], lgB[NH];
             {
@@ -448,8 +458,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
                 const uint32_t sa = reinterpret_cast<const uint32_t *>(spS + slotA * 16)[t];
                 const uint32_t sb = reinterpret_cast<const uint32_t *>(spS + slotB * 16)[t];
                 const uint32_t sa4 = sa >> 4, sb4 = sb >> 4;
-                int d2[4] = {0, 0, 0, 0};
-                int d2l[4] = {0, 0, 0, 0};  // wide: the lo-term products
+                int d2[4], d2l[4];  // (wide: d2l holds the lo-term products)
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
                     // sign bit n of every byte stays where it is (value 2^n or 0); the projected
@@ -458,8 +467,13 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
                     const uint32_t a1 = sb & (0x01010101u << n);
                     const uint32_t a2 = sa4 & (0x01010101u << n);
                     const uint32_t a3 = sb4 & (0x01010101u << n);
-                    mma_s8(d2, a0, a1, a2, a3, bp[n][0], bp[n][1]);
-                    if (WIDE) mma_s8(d2l, a0, a1, a2, a3, bp[(WIDE ? 4 : 0) + n][0], bp[(WIDE ? 4 : 0) + n][1]);
+                    if (n == 0) mma_s8_first(d2, a0, a1, a2, a3, bp[n][0], bp[n][1]);
+                    else mma_s8(d2, a0, a1, a2, a3, bp[n][0], bp[n][1]);
+                    if (WIDE) {
+                        constexpr int kLo = QJL && WIDE ? 4 : 0;
+                        if (n == 0) mma_s8_first(d2l, a0, a1, a2, a3, bp[kLo + n][0], bp[kLo + n][1]);
+                        else mma_s8(d2l, a0, a1, a2, a3, bp[kLo + n][0], bp[kLo + n][1]);
+                    }
                 }
                 const float rnA = tq_half_bits_to_float(rn[slotA]) * kB, rnB = tq_half_bits_to_float(rn[slotB]) * kB;
 #pragma unroll
@@ -498,11 +512,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
                 const float sc = fast_exp2(m_run[hl] - nm[hl]);
                 l_run[hl] *= sc;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) o[i][hl] *= sc, o[i][2 + hl] *= sc;
+                for (int i = 0; i < kAcc; ++i) {
+                    o[i][hl] *= sc, o[i][2 + hl] *= sc;
+                    if (!WIDE) o[i][1] *= sc, o[i][3] *= sc;
+                }
                 m_run[hl] = nm[hl];
             }
         }
-        uint32_t pb[2][2];
+        uint32_t px[2][2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int slotA = 16 * i + (g >> 1) + 4 * (g & 1);
@@ -516,36 +533,46 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
                 wA[hl] = pA * vnA, wB[hl] = pB * vnB;
                 if (tail) wA[hl] = pA > 0.f ? wA[hl] : 0.f, wB[hl] = pB > 0.f ? wB[hl] : 0.f;
             }
-            // rows = token slots, cols = this lane's heads (narrow: head t and an unused column)
-            // -> transpose to rows = columns
-            pb[i][0] = movmatrix_trans(pack_half2(wA[0], wA[1]));
-            pb[i][1] = movmatrix_trans(pack_half2(wB[0], wB[1]));
+            // rows = token slots, columns = this lane's heads (narrow: head t twice) -> transposed: tokens
+            // t and t + 4 (then t + 8 and t + 12) of the tile for the head of column g
+            px[i][0] = movmatrix_trans(pack_half2(wA[0], WIDE ? wA[1] : wA[0]));
+            px[i][1] = movmatrix_trans(pack_half2(wB[0], WIDE ? wB[1] : wB[0]));
         }
         // ------------------------------------------------------------ values
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const uint8_t *vrow = spV + (16 * i + t) * (16 * VB);
-            const uint64_t w0 = lds_v_chunk<VB>(vrow, g);                    // token t      (k-slot 2t)
-            const uint64_t w1 = lds_v_chunk<VB>(vrow + 4 * 16 * VB, g);      // token t+4    (k-slot 2t+1)
-            const uint64_t w2 = lds_v_chunk<VB>(vrow + 8 * 16 * VB, g);      // token t+8    (k-slot 2t+8)
-            const uint64_t w3 = lds_v_chunk<VB>(vrow + 12 * 16 * VB, g);     // token t+12   (k-slot 2t+9)
-            constexpr uint64_t me = even_field_mask<VB>();
-            const uint64_t x01 = (w0 & me) | ((w1 << VB) & (me << VB));
-            const uint64_t y01 = ((w0 >> VB) & me) | (w1 & (me << VB));
-            const uint64_t x23 = (w2 & me) | ((w3 << VB) & (me << VB));
-            const uint64_t y23 = ((w2 >> VB) & me) | (w3 & (me << VB));
-            const uint32_t xa[3] = {(uint32_t)x01, (uint32_t)(x01 >> 32), 0u};
-            const uint32_t ya[3] = {(uint32_t)y01, (uint32_t)(y01 >> 32), 0u};
-            const uint32_t xb[3] = {(uint32_t)x23, (uint32_t)(x23 >> 32), 0u};
-            const uint32_t yb[3] = {(uint32_t)y23, (uint32_t)(y23 >> 32), 0u};
+            uint64_t w[4];  // tokens t, t + 4, t + 8, t + 12 of the tile
 #pragma unroll
-            for (int mt = 0; mt < 8; ++mt) {
-                constexpr int W = 2 * VB;
-                const uint32_t a0 = lds_abs(slot_addr(xa, mt * W, lane_v));
-                const uint32_t a1 = lds_abs(slot_addr(ya, mt * W, lane_v));
-                const uint32_t a2 = lds_abs(slot_addr(xb, mt * W, lane_v));
-                const uint32_t a3 = lds_abs(slot_addr(yb, mt * W, lane_v));
-                mma_f16(o[mt], a0, a1, a2, a3, pb[i][0], pb[i][1]);
+            for (int k = 0; k < 4; ++k) w[k] = lds_v_chunk<VB>(spV + (16 * i + 4 * k + t) * (16 * VB), g);
+            constexpr int W = 2 * VB;
+            if constexpr (WIDE) {
+                // the columns hold eight heads: two tokens' codes are interleaved, so that a look-up yields what the MMA wants along K
+                constexpr uint64_t me = even_field_mask<VB>();
+                const uint64_t x01 = (w[0] & me) | ((w[1] << VB) & (me << VB)), y01 = ((w[0] >> VB) & me) | (w[1] & (me << VB));
+                const uint64_t x23 = (w[2] & me) | ((w[3] << VB) & (me << VB)), y23 = ((w[2] >> VB) & me) | (w[3] & (me << VB));
+                const uint32_t xa[3] = {(uint32_t)x01, (uint32_t)(x01 >> 32), 0u}, ya[3] = {(uint32_t)y01, (uint32_t)(y01 >> 32), 0u};
+                const uint32_t xb[3] = {(uint32_t)x23, (uint32_t)(x23 >> 32), 0u}, yb[3] = {(uint32_t)y23, (uint32_t)(y23 >> 32), 0u};
+#pragma unroll
+                for (int mt = 0; mt < 8; ++mt) {
+                    const uint32_t a0 = lds_abs(slot_addr(xa, mt * W, lane_v)), a1 = lds_abs(slot_addr(ya, mt * W, lane_v));
+                    const uint32_t a2 = lds_abs(slot_addr(xb, mt * W, lane_v)), a3 = lds_abs(slot_addr(yb, mt * W, lane_v));
+                    mma_f16(o[mt], a0, a1, a2, a3, px[i][0], px[i][1]);
+                }
+            } else {
+                // half of the columns would be empty: a row of A is a pair of coordinates as it lies in memory, K runs over (token,
+                // parity) and a column is (head, parity), with the weight at its own parity and 0 at the other
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const uint32_t b0 = prmt(px[i][k], 0u, sel_first), b1 = prmt(px[i][k], 0u, sel_second);
+                    const uint32_t x0[3] = {(uint32_t)w[2 * k], (uint32_t)(w[2 * k] >> 32), 0u};
+                    const uint32_t x1[3] = {(uint32_t)w[2 * k + 1], (uint32_t)(w[2 * k + 1] >> 32), 0u};
+#pragma unroll
+                    for (int mt = 0; mt < 4; ++mt) {
+                        const uint32_t a0 = lds_abs(slot_addr(x0, 2 * mt * W, lane_v)), a1 = lds_abs(slot_addr(x0, (2 * mt + 1) * W, lane_v));
+                        const uint32_t a2 = lds_abs(slot_addr(x1, 2 * mt * W, lane_v)), a3 = lds_abs(slot_addr(x1, (2 * mt + 1) * W, lane_v));
+                        mma_f16(o[mt], a0, a1, a2, a3, b0, b1);
+                    }
+                }
             }
         }
         }  // at least one token at or after t_lo
@@ -579,16 +606,20 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
         for (int sft = 4; sft <= 16; sft <<= 1) l_all += __shfl_xor_sync(0xffffffffu, l_all, sft);
         // (a warp whose tokens are all masked has summed up undefined weights)
         if (g == 0) s_m[warp * 4 + t] = m_run[hl], s_l[warp * 4 + t] = m_run[hl] == -INFINITY ? 0.f : l_all;
-        // A warp's 512 accumulators are laid out [mt][lane][2], so the 8-byte stores of a warp
-        // and the reads of 32 consecutive elements below both touch every bank once.
+        // A warp's 512 accumulators are laid out [mt][lane][4 coordinates] (wide: [2]), so its 16- or 8-byte stores
+        // and the reads of 32 consecutive elements below both touch every bank the same number of times.
+        constexpr int kEach = WIDE ? 2 : 4;
 #pragma unroll
-        for (int mt = 0; mt < 8; ++mt)
-            *reinterpret_cast<float2 *>(s_acc + warp * 4 * TQ_D + mt * 64 + lane * 2) = make_float2(o[mt][hl], o[mt][2 + hl]);
+        for (int mt = 0; mt < kAcc; ++mt) {
+            float *to = s_acc + warp * 4 * TQ_D + (mt * 32 + lane) * kEach;
+            if (WIDE) *reinterpret_cast<float2 *>(to) = make_float2(o[mt][hl], o[mt][2 + hl]);
+            else *reinterpret_cast<float4 *>(to) = make_float4(o[mt][0], o[mt][1], o[mt][2], o[mt][3]);
+        }
         __syncthreads();
         for (int idx = threadIdx.x; idx < 4 * TQ_D; idx += blockDim.x) {
-            // element idx of that layout: accumulator tile mt of lane (gg, tt), column pair member j
-            const int mt = idx >> 6, gg = (idx & 63) >> 3, tt = (idx >> 1) & 3, j = idx & 1;
-            const int d = 16 * gg + 2 * mt + j;
+            // element idx of that layout: coordinate j of accumulator tile mt of lane (gg, tt)
+            const int j = idx % kEach, from = idx / kEach % 32, mt = idx / (32 * kEach), gg = from >> 2, tt = from & 3;
+            const int d = 16 * gg + kEach * mt + j;
             const int hh = WIDE ? 2 * tt + hl : tt;
             if (hh >= G) continue;
             float M = -INFINITY;
