@@ -518,9 +518,11 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
     {   // thread (e, dq) merges the splits of head dq.  Up to four, the usual number with many rows: everything is
         // requested in one batch and merged in registers (sixty pairs of runs each: 0.65 +- 0.08 us less than the other way for
         // 8 x 8 x 32768 tokens, 0.45 to 0.6 +- 0.02 for six smaller caches, 1.5 for 64 x 8 x 500 of one head).  More: 32 at a
-        // time, lane s of each warp holds split s's maximum and weight, the accumulator columns are requested
-        // eight splits at a time.  (The kernel takes 5.6 us for 33 splits of 4 rows; with one thread walking all
-        // splits twice it took 10.8, with maxima, sums and columns of eight splits in every thread 1.1 us more.)
+        // time, lane s of each warp holds split s's maximum and weight, and all accumulator columns are requested before
+        // the first is used: one trip to L2, where eight at a time took one for every eight (eight layer steps of nine splits
+        // 98.5 -> 96.6 us, 32768 tokens of seven heads in 33 splits 17.45 -> 17.2, of four heads 19.1 -> 18.9).  (With one
+        // thread walking all splits twice the kernel took twice as long, with maxima, sums and columns of eight splits in every
+        // thread 1.1 us more.)
         const int g = dq;
         float o = 0.f, L = 0.f, Mx = -INFINITY;
         if (g < n_heads) {
@@ -542,21 +544,21 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
             } else for (int s0 = 0; s0 < n_valid; s0 += 32) {
                 const int n = min(32, n_valid - s0);
                 const float *acc = a.part_acc + (slot0 + s0) * TQ_D + e;
-                float pa[8];
+                float pa[32];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) pa[i] = i < n ? acc[i * TQ_D] : 0.f;
+                for (int i = 0; i < 32; ++i) pa[i] = i < n ? acc[i * TQ_D] : 0.f;
                 const float pm = lane < n ? a.part_m[slot0 + s0 + lane] : -INFINITY;
                 const float pl = lane < n ? a.part_l[slot0 + s0 + lane] : 0.f;
                 const float M = fmaxf(Mx, tq_warp_max(pm));
                 const float corr = Mx == -INFINITY ? 0.f : expf(Mx - M);
                 const float w = pm == -INFINITY ? 0.f : expf(pm - M);
                 L = L * corr + tq_warp_sum(pl * w), o *= corr, Mx = M;
-                for (int i0 = 0; i0 < n; i0 += 8) {
-                    float cur[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) cur[i] = pa[i], pa[i] = i0 + 8 + i < n ? acc[(i0 + 8 + i) * TQ_D] : 0.f;
+                for (int i0 = 0; i0 < 32; i0 += 8) {
+                    if (i0 < n) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) o = fmaf(cur[i], __shfl_sync(0xffffffffu, w, i0 + i), o);
+                        for (int i = i0; i < i0 + 8; ++i) o = fmaf(pa[i], __shfl_sync(0xffffffffu, w, i), o);
+                    }
                 }
             }
         }
