@@ -15,14 +15,20 @@
 // that one group's CUDA-core work runs beside the other group's MMAs.  Four threads share a vector (32
 // coordinates each).  The A operand is written to TMEM (tcgen05.st, no swizzle, no bank conflicts), so
 // shared memory is left for the matrices: R_k (stage 1; stage 2 reads the same image transposed) and S stay
-// resident and nothing is reloaded between the stages.  Rows of 16-bit vectors come through shared memory, one
-// bulk copy each: read straight from global memory by the threads that own them they took 2048 of the 4500
-// L1 wavefronts of a value tile, which bounded it.  A group owns 256 TMEM columns: 128 of accumulator, 64 for each term of A.
+// resident and nothing is reloaded between the stages.  Rows of 16-bit vectors come through shared memory, copied
+// by all warps, 16 bytes a lane and sixteen lanes to a row: read by the threads that own them they took 2048 of the 4500
+// L1 wavefronts of a value tile, which bounded it, and as a bulk copy per row they are issued lane by lane by the warps that are
+// waited for (2 x 8 x 32768 bf16 vectors a tensor 220 us instead of 209).  A group owns 256 TMEM columns: 128 of accumulator, 64 for each term of A.
 // The first CTAs of a launch encode keys and the others values, in the proportion of their costs.
-// What bounds it is the chain of a key tile - store A, MMA, read back, three times - with two tiles in flight, which
-// is what 512 TMEM columns hold (tensor pipe 34 %, issue slots 54 %, L1 33 % busy).  8 x 8 x 32768 bf16 keys and
-// values, 4 bits with the sketch: 907 us; 1306 us with two threads a vector that read their own rows and a binary search;
-// 2189 us with three-term bf16 operands in shared memory, one tile at a time.
+// What bounds it is the CUDA-core work between the contractions: time stamps in one CTA show both groups in step, so that their
+// instructions share the schedulers, then their MMAs follow one another (1150 cycles for sixteen, 1660 for 24, alone or beside
+// shared-memory and TMEM traffic).  The issuing thread is elected in a converged warp and the accumulator's address is
+// uniform, which leaves an instruction or two per MMA: with a thread chosen by its index the operands went through vector
+// registers, and sixteen MMAs took 2000 - 2400 cycles to issue between the other warps' instructions.
+// 2 x 8 x 32768 keys and values, 4 bits with the sketch: bf16 242 -> 203 us, f16 252 -> 194; 3 bits 259 -> 213, 269 -> 194; 4 bits
+// without 142 -> 128, 124 -> 114 (before: look-ups one by one, bulk copies, issue by index).  All sixteen warps of a
+// group on one tile at a time with dedicated loading and issuing warps, two tiles in flight: 262 us and more, too few warps to hide the
+// latencies of a phase.
 // Every mbarrier wait is bounded and reports through the device status word.
 #include <math.h>
 #include <string.h>
@@ -139,23 +145,38 @@ template <int BITS, int MUL, bool GRID> struct Search {
         asm("ld.shared.f32 %0, [%1];\n" : "=f"(b) : "r"(table + offset));
         return b < z;
     }
-    __device__ __forceinline__ uint32_t operator()(float z) const {
-        if (BITS == 1) return b0 < z ? MUL : 0u;
-        if (BITS == 2) {
-            const bool up = b1 < z;
-            return (up ? 2u * MUL : 0u) + ((up ? b2 : b0) < z ? MUL : 0u);
+    // Eight coordinates at a time: eight look-ups under way and no more registers.  (Written one by one, the look-ups of 32 coordinates
+    // were all moved ahead of the comparisons, whose outcomes were then packed into registers and spilled: twice 8 x 32768 bf16 keys
+    // and values 234 us instead of 203, eight at a time with the comparison as a predicated instruction 236.)
+    __device__ __forceinline__ void operator()(const float (&z)[8], uint32_t *code) const {
+        if (BITS == 1) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) code[e] = b0 < z[e] ? MUL : 0u;
+        } else if (BITS == 2) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const bool up = b1 < z[e];
+                code[e] = (up ? 2u * MUL : 0u) + ((up ? b2 : b0) < z[e] ? MUL : 0u);
+            }
+        } else if (!GRID) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                uint32_t c = 0;  // (four times the boundaries known to be below)
+                if (BITS == 4) c = below(4 * 7, z[e]) ? 32u : 0u;
+                c += below(c + 4 * 3, z[e]) ? 16u : 0u;
+                c += below(c + 4 * 1, z[e]) ? 8u : 0u;
+                c += below(c, z[e]) ? 4u : 0u;
+                code[e] = c / 4 * MUL;
+            }
+        } else {
+            uint32_t bound[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(bound[e]), "=r"(code[e]) : "r"(grid_cell(z[e], grid) * (8u * kCellCopies) + table));
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                code[e] += __uint_as_float(bound[e]) < z[e] ? MUL : 0u;
         }
-        if (!GRID) {
-            uint32_t c = 0;  // (four times the boundaries known to be below)
-            if (BITS == 4) c = below(4 * 7, z) ? 32u : 0u;
-            c += below(c + 4 * 3, z) ? 16u : 0u;
-            c += below(c + 4 * 1, z) ? 8u : 0u;
-            c += below(c, z) ? 4u : 0u;
-            return c / 4 * MUL;
-        }
-        uint32_t bound, lower;
-        asm("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(bound), "=r"(lower) : "r"(grid_cell(z, grid) * (8u * kCellCopies) + table));
-        return lower + (__uint_as_float(bound) < z ? MUL : 0u);
     }
 };
 // Fills the grid's table (all threads of the CTA; barriers around it are the caller's).
@@ -209,7 +230,7 @@ struct PackTcShared {
     float sq[kGroups][2][kParts][kUmmaRows];   // squared norms: [group][tile parity][part of the coordinates][vector]
     float big[kGroups][2][kParts][kUmmaRows];  // largest magnitudes of parts whose squared norm is zero
     float rs[kGroups][kParts][kUmmaRows];         // squared residual norms
-    uint64_t bar_image[2], bar_mma[kGroups], bar_rows[kGroups];
+    uint64_t bar_image[2], bar_mma[kGroups], bar_rows[kGroups][4];
     uint32_t tmem;
 };
 
@@ -220,12 +241,11 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
     const int tid = threadIdx.x, group = tid / kGroupThreads, warp = tid >> 5;
     const int vrow = tid & (kUmmaRows - 1);            // this thread's vector within the tile (= its TMEM lane)
     const int part = (tid / kUmmaRows) % kParts;       // which part of the coordinates it works on
-    const uint32_t acc = sm.tmem + group * 256, a_hi = acc + 128, a_lo = acc + 192;
+    const uint32_t acc = __shfl_sync(0xffffffffu, sm.tmem + group * 256, 0), a_hi = acc + 128, a_lo = acc + 192;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t my_acc = acc + lanes + kCoords * part, my_hi = a_hi + lanes + kCoords / 2 * part, my_lo = my_hi + 64;
     const uint32_t bar_mma = smem_u32(&sm.bar_mma[group]);
-    const bool issuer = (tid & (kGroupThreads - 1)) == 0;
-    bool timed_out = false;
+    const bool issuer = __shfl_sync(0xffffffffu, tid & (kGroupThreads - 1), 0) == 0;  // a group's first warp
     uint32_t mma_phase = 0;
     uint32_t landed = 0;  // issuer: the images seen in shared memory
 
@@ -235,10 +255,10 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
         tmem_st_wait();
         umma_fence_before();
         group_sync();
-        if (issuer) {
+        if (issuer && elect_one()) {  // (always the same thread of the warp: `landed`, and what a commit covers, are its own)
             umma_fence_after();
             if (!(landed >> image & 1)) {
-                if (!mbar_wait(smem_u32(&sm.bar_image[image]), 0)) timed_out = true;
+                if (!mbar_wait(smem_u32(&sm.bar_image[image]), 0)) atomicExch(a.error_flag, 3);
                 landed |= 1u << image;
             }
             umma_issue<decltype(terms)::value, decltype(transposed)::value>(acc, a_hi, a_lo, images + image * kUmmaImageBytes);
@@ -246,7 +266,7 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
         }
     };
     auto gemm_wait = [&]() {
-        if (!mbar_wait(bar_mma, mma_phase)) timed_out = true;
+        if (!mbar_wait(bar_mma, mma_phase)) atomicExch(a.error_flag, 3);
         mma_phase ^= 1;
         __syncwarp();  // the issuer took its own path; tcgen05.ld is warp-collective
         umma_fence_after();
@@ -254,10 +274,10 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
     const std::integral_constant<int, 1> one_term;
     const std::integral_constant<int, 2> two_terms;
 
-    // Rows of 16-bit vectors are staged in shared memory (requested by the threads of part 0, a row each); fp32
+    // Rows of 16-bit vectors are staged in shared memory (each warp requests eight of its quadrant's); fp32
     // rows, for which there is no room, come straight from global memory.
     constexpr bool kStaged = sizeof(T) == 2;
-    const uint32_t my_stage = staged + group * kStageBytes + vrow * kStagePitch, bar_rows = smem_u32(&sm.bar_rows[group]);
+    const uint32_t my_stage = staged + group * kStageBytes + vrow * kStagePitch, bar_rows = smem_u32(&sm.bar_rows[group][warp & 3]);
     uint32_t raw[R::kWords];  // this thread's part of the vector, as stored
     int64_t row = 0;          // the vector's cache row (< 0: no vector)
     uint32_t rows_phase = 0;
@@ -269,10 +289,14 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
         const T *src = reinterpret_cast<const T *>(r.x) + b * r.sb + h * r.sh + (int64_t)t * r.st;
         row = valid ? b * a.cache_sb + h * a.cache_sh + a.pos0 + t : -1;
         if constexpr (kStaged) {
-            if (part == 0) {
-                mbar_expect_tx(bar_rows, 2 * TQ_D);
-                tma_load_1d(my_stage, src, 2 * TQ_D, bar_rows);
+            const int lane = tid & 31;
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {  // eight of the warp's 32 rows (the other parts' warps take the others), sixteen lanes to a row
+                const int from = 8 * part + i + (lane >> 4);
+                const uint64_t at = __shfl_sync(0xffffffffu, reinterpret_cast<uint64_t>(src), from);
+                async_copy16(my_stage + (from - lane) * kStagePitch + 16 * (lane & 15), reinterpret_cast<const void *>(at + 16 * (lane & 15)));
             }
+            async_arrive(bar_rows);
         } else {
 #pragma unroll
             for (int i = 0; i < R::kWords / 4; ++i) {
@@ -292,7 +316,7 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
     };
     auto rows_wait = [&]() {
         if constexpr (kStaged) {
-            if (!mbar_wait(bar_rows, rows_phase)) timed_out = true;
+            if (!mbar_wait(bar_rows, rows_phase)) atomicExch(a.error_flag, 3);
             rows_phase ^= 1;
         }
     };
@@ -396,10 +420,12 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
             uint32_t z[16], code[16];
             tmem_ld16(my_acc + 16 * q, z);
 #pragma unroll
-            for (int e = 0; e < 16; e += 2) {
-                float z0, z1;
-                f32x2_split(f32x2_mul(f32x2(__uint_as_float(z[e]), __uint_as_float(z[e + 1])), inv2), z0, z1);
-                code[e] = search(z0), code[e + 1] = search(z1);
+            for (int h = 0; h < 16; h += 8) {
+                float x[8];
+#pragma unroll
+                for (int e = 0; e < 8; e += 2)
+                    f32x2_split(f32x2_mul(f32x2(__uint_as_float(z[h + e]), __uint_as_float(z[h + e + 1])), inv2), x[e], x[e + 1]);
+                search(x, code + h);
             }
             put_codes<BITS, QJL ? 4 : 1>(words, q, code);
             if (QJL) {
@@ -473,7 +499,6 @@ __device__ __forceinline__ void encode(const PackTcArgs &a, const PackTcRole &r,
             }
         }
     }
-    if (timed_out) atomicExch(a.error_flag, 3);
 }
 
 template <typename T, int BITS, bool QJL, bool GRID>
@@ -500,7 +525,10 @@ __global__ void __launch_bounds__(kThreads, 1) tq_pack_tc_kernel(const __grid_co
     }
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&sm.bar_image[i]), 1);
-        for (int i = 0; i < kGroups; ++i) mbar_init(smem_u32(&sm.bar_mma[i]), 1), mbar_init(smem_u32(&sm.bar_rows[i]), kUmmaRows);
+        for (int i = 0; i < kGroups; ++i) {
+            mbar_init(smem_u32(&sm.bar_mma[i]), 1);
+            for (int q = 0; q < 4; ++q) mbar_init(smem_u32(&sm.bar_rows[i][q]), kUmmaRows);  // (32 threads of four warps)
+        }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         umma_load_image(images, r.image, smem_u32(&sm.bar_image[0]));  // (every CTA has at least one tile)

@@ -31,9 +31,17 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, ui
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 // Rows of 16-bit vectors staged in shared memory lie 272 bytes apart: 16-byte accesses of a warp to one
-// column of 32 rows touch every bank the same number of times.  One bulk copy moves a row.
+// column of 32 rows touch every bank the same number of times.
 constexpr int kStagePitch = 2 * TQ_D + 16;
 constexpr int kStageBytes = kUmmaRows * kStagePitch;
+
+// 16 bytes to shared memory without a register in between; `async_arrive` counts on `bar` when this thread's copies are there.
+__device__ __forceinline__ void async_copy16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];\n" ::"r"(bar) : "memory");
+}
 
 // One matrix image to shared memory (one thread; `bar` counts one arrival and the bytes).
 __device__ __forceinline__ void umma_load_image(uint32_t dst, const uint16_t *image, uint32_t bar) {
@@ -53,6 +61,13 @@ template <bool TRANSPOSED> __device__ __forceinline__ uint64_t umma_desc(uint32_
 // Instruction descriptor: D = f32, A = B = f16, A K-major, N = 128, M = 128.
 template <bool TRANSPOSED> __host__ __device__ constexpr uint32_t umma_instr() {
     return (1u << 4) | (TRANSPOSED ? 1u << 16 : 0u) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+// One thread of a converged warp, in a form that lets the compiler keep what the branch needs in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
 }
 
 // D[128 x 128] (+)= A[128 x 16] (TMEM, two f16 per column) * B (shared memory)
