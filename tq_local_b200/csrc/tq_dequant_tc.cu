@@ -6,10 +6,12 @@
 // structure is the prefill encoder's: one persistent CTA per SM, two groups of sixteen warps that each walk
 // their own tiles, four threads to a vector, A written to TMEM, the matrices resident in shared memory; the two
 // contractions of a key go one after the other through the group's one accumulator, the first result waiting as
-// packed T.  16-bit rows leave through shared memory, one bulk copy each.
-// Bound, like the encoder, by the chain of a tile with two in flight.  8 x 32768 bf16 keys with the sketch 57 us,
-// values 40 us (HBM floor 13 each); 1123 and 571 us with fp32 multiply-adds and the matrix read from L2 per vector,
-// 66 and 46 us with two threads a vector and direct stores.
+// packed T.  16-bit rows leave through shared memory, sixteen lanes to a row.
+// Bound, like the encoder, by the CUDA-core work between the contractions.  8 x 32768 bf16, keys with the sketch and values: 93.5 us with the
+// issuing thread chosen by its index and a bulk copy per row, issued lane by lane by the warps that all others then waited
+// for; 78.5 with an elected issuer whose operands stay in uniform registers and the groups' contractions one after the
+// other (80.0 without that order); 72.4 with rows that all warps copy out, 16 bytes a lane (HBM floor 26; 1694 us with fp32
+// multiply-adds and the matrix read from L2 per vector).
 #include <math.h>
 
 #include <type_traits>
@@ -59,7 +61,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t s_cen[16];  // f16 hi term | lo term << 16 of a scaled centre
     __shared__ uint64_t s_bar_image[2], s_bar_mma[kGroups];
-    __shared__ uint32_t s_tmem;
+    __shared__ uint32_t s_tmem, s_turn;  // (see turn_take)
     const uint32_t images = (smem_u32(smem_raw) + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
     const int tid = threadIdx.x, warp = tid >> 5, group = tid / kGroupThreads;
     if (tid < 16) {
@@ -72,6 +74,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
     if (tid == 0) {
+        s_turn = 0;
         for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&s_bar_image[i]), 1), mbar_init(smem_u32(&s_bar_mma[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -83,11 +86,11 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
     umma_fence_after();
 
     const int vrow = tid & (kUmmaRows - 1), part = (tid / kUmmaRows) % kParts;
-    const uint32_t acc = s_tmem + group * 256, a_hi = acc + 128, a_lo = acc + 192;
+    const uint32_t acc = __shfl_sync(0xffffffffu, s_tmem + group * 256, 0), a_hi = acc + 128, a_lo = acc + 192;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t my_acc = acc + lanes + kCoords * part, my_hi = a_hi + lanes + kCoords / 2 * part, my_lo = my_hi + 64;
     const uint32_t bar_mma = smem_u32(&s_bar_mma[group]);
-    const bool issuer = (tid & (kGroupThreads - 1)) == 0;
+    const bool issuer = __shfl_sync(0xffffffffu, tid & (kGroupThreads - 1), 0) == 0;  // a group's first warp
     bool timed_out = false;
     uint32_t mma_phase = 0, landed = 0;
     constexpr bool kStaged = sizeof(T) == 2;
@@ -97,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
     // one sign, loses 4e-7 of it; the fp32 results' sums of centres come in two pieces of four steps each, which leaves 2e-7, and
     // half of that is given back by scaling one piece by kUmmaRestore.  Relative to 64 bits, 2-norm over 262144 rows, 3-bit
     // values: rows with one large element 3.5e-7 in one piece, 1.5e-7 in two (fp32 multiply-adds one after the other: 2.0e-7), Gaussian
-    // rows 1.3e-7 and 1.1e-7 (2.0e-7).  8 x 16384 values 35.3 us in one piece, 37.5 in two.  The signs' sums stay below 1.1e-7 in one.
+    // rows 1.3e-7 and 1.1e-7 (2.0e-7).  The signs' sums stay below 1.1e-7 in one.
     constexpr int kPieces = sizeof(T) == 4 ? 2 : 1;
     const std::integral_constant<int, 0> first_piece;
     const std::integral_constant<int, 1> second_piece;
@@ -108,14 +111,16 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
         tmem_st_wait();
         umma_fence_before();
         group_sync();
-        if (issuer) {
+        if (issuer && elect_one()) {
             umma_fence_after();
             if (!(landed >> stage & 1)) {
                 if (!mbar_wait(smem_u32(&s_bar_image[stage]), 0)) timed_out = true;
                 landed |= 1u << stage;
             }
+            if (!turn_take(&s_turn)) timed_out = true;
             umma_issue<kTerms, true, decltype(piece)::value, kTerms == 2 ? kPieces : 1>(acc, a_hi, a_lo, images + stage * kUmmaImageBytes);
             umma_commit(bar_mma);
+            turn_give(&s_turn);
         }
     };
     auto gemm_wait = [&]() {
@@ -153,7 +158,6 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
     if (first < a.n_tiles) fetch(first);
     for (int tile = first; tile < a.n_tiles; tile += stride) {
         // ---------------- A = centres[codes]
-        if (kStaged) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
         __syncwarp();  // (tcgen05.st is warp-collective)
 #pragma unroll
         for (int c = 0; c < kCoords / 16; ++c) {
@@ -249,14 +253,17 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
             }
         }
         if constexpr (kStaged) {
-            // (the rows of the tile before have left: their threads waited for that before this tile's first barrier)
+            // (every warp has read its rows of the tile before: it did so ahead of this tile's first barrier)
 #pragma unroll
             for (int i = 0; i < kOutWords; i += 4) sts128(my_stage + 2 * kCoords * part + 4 * i, o[i], o[i + 1], o[i + 2], o[i + 3]);
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             group_sync();
-            if (part == 0) {
-                if (to) tma_store_1d(to, my_stage, 2 * TQ_D);
-                asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+            const int lane = tid & 31;
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {  // eight of the warp's 32 rows (the other parts' warps take the others), sixteen lanes to a row
+                const int from = 8 * part + i + (lane >> 4);
+                T *const row = reinterpret_cast<T *>(__shfl_sync(0xffffffffu, reinterpret_cast<uint64_t>(to), from));
+                const uint4 v = lds128(my_stage + (from - lane) * kStagePitch + 16 * (lane & 15));
+                if (row) reinterpret_cast<uint4 *>(row)[lane & 15] = v;
             }
         } else if (to) {
 #pragma unroll
@@ -264,7 +271,6 @@ __global__ void __launch_bounds__(kThreads, 1) tq_dequant_tc_kernel(const __grid
                 *reinterpret_cast<uint4 *>(reinterpret_cast<uint32_t *>(to) + kOutWords * part + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
         }
     }
-    if (kStaged) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     if (timed_out) atomicExch(a.error_flag, 3);
     umma_fence_before();
     __syncthreads();

@@ -18,10 +18,6 @@ constexpr int kUmmaSlabBytes = 128 * 128;              // 128 rows x 64 f16 (one
 constexpr int kUmmaTermBytes = 2 * kUmmaSlabBytes;     // one f16 term of a 128 x 128 matrix: 32 KB
 constexpr int kUmmaImageBytes = 2 * kUmmaTermBytes;    // hi and lo terms: 64 KB
 
-// Shared memory to global (one thread; complete once its bulk group is).
-__device__ __forceinline__ void tma_store_1d(void *dst, uint32_t src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
@@ -108,6 +104,15 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 }
 __device__ __forceinline__ void umma_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void umma_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+
+// The contractions of a CTA's two groups one after the other (a lock in shared memory, held while a batch is issued): left to
+// themselves the MMAs of both alternate, and the group that was first waits for the other's as well.
+__device__ __forceinline__ bool turn_take(uint32_t *turn) {
+    for (uint32_t i = 0; i < kSpinLimit; ++i)
+        if (atomicCAS(turn, 0u, 1u) == 0u) return true;
+    return false;
+}
+__device__ __forceinline__ void turn_give(uint32_t *turn) { atomicExch(turn, 0u); }
 
 // Byte offset of element (row, k) inside one f16 term of an image (two 64-wide slabs, 128-byte swizzle).
 __host__ __device__ inline int umma_operand_offset(int row, int k) {
