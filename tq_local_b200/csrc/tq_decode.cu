@@ -593,10 +593,13 @@ __global__ void __launch_bounds__(4 * TQ_D) tq_combine_group_kernel(CombineArgs 
     {   // thread (e, dq) un-rotates rows d in [32 dq, 32 dq + 32) for all heads
         float out[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const int d = 32 * dq + i;
+        for (int i = 0; i < 32; i += 4) {
 #pragma unroll
-            for (int g = 0; g < 4; ++g) out[g] = fmaf(s_o[g][d], rv[i], out[g]);
+            for (int g = 0; g < 4; ++g) {
+                const float4 o = *reinterpret_cast<const float4 *>(&s_o[g][32 * dq + i]);
+                out[g] = fmaf(o.x, rv[i], out[g]), out[g] = fmaf(o.y, rv[i + 1], out[g]);
+                out[g] = fmaf(o.z, rv[i + 2], out[g]), out[g] = fmaf(o.w, rv[i + 3], out[g]);
+            }
         }
 #pragma unroll
         for (int g = 0; g < 4; ++g) s_part[dq][g][e] = out[g];

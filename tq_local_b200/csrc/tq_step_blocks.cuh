@@ -111,16 +111,19 @@ __device__ __forceinline__ uint32_t tq_assemble_word(const uint8_t *codes, int w
 // Encode one vector (item < n_vec: kind first_kind, else the next kind) and write it at its
 // cache row.  fp32 arithmetic in a fixed order: partial sums over four 32-row quarters, then
 // (p0 + p1) + (p2 + p3).
-// A key with a sketch is a chain of three mat-vecs.  STAGED (128 KB of dynamic shared memory, for launches of no more
-// blocks than SMs): the matrices of the second and third are requested by bulk copy before anything else and wait in
-// shared memory; otherwise their columns are read from L2 in turn, 64 KB a mat-vec and a microsecond of the chain
-// (eight recorded layer steps at 4099 tokens, 32 blocks each: 104 us against 107).
-constexpr int kStagedMatrices = 2 * TQ_D * TQ_D * 4;
+// A key with a sketch is a chain of three mat-vecs, and the whole step waits for it.  STAGED (64 KB of dynamic shared memory and all
+// registers of an SM, for launches of no more blocks than SMs): the columns of the first two matrices are in registers before the
+// vector is there, the third matrix was requested by bulk copy before anything else and its column takes the first one's registers
+// while the codes are found; the bitstream, a loop of byte reads, is assembled by a warp of its own at the end.  From the vector's
+// arrival to the last store 2.3 us; 3.4 with two matrices staged, columns taken from shared memory between two barriers and the bitstream
+// before the second mat-vec; otherwise the columns are read from L2 in turn, 64 KB a mat-vec and a microsecond of the chain.
+constexpr int kStagedMatrices = TQ_D * TQ_D * 4;
 inline bool tq_stages_matrices(const tq_ctx *ctx, int64_t blocks) { return ctx->use_qjl && blocks <= ctx->sm_count; }
 template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_pack_small_block(const TqPackArgs &a, int64_t item) {
-    extern __shared__ __align__(128) float s_matrices[];
+    extern __shared__ __align__(128) float s_matrix[];
     __shared__ __align__(8) uint64_t s_bar;
-    __shared__ float s_x[TQ_D], s_u[TQ_D], s_part[4][TQ_D], s_red[4];
+    __shared__ __align__(16) float s_u[TQ_D];
+    __shared__ float s_part[3][4][TQ_D], s_red[2][4];  // [mat-vec], [norm]: a stage's are not written again
     __shared__ uint8_t s_code[TQ_D];
     __shared__ float s_bnd[16], s_cen[16];
     const int tid = threadIdx.x, j = tid & (TQ_D - 1), dq = tid >> 7, lane = tid & 31;
@@ -134,16 +137,19 @@ template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_
     const int bits = a.bits[kind];
     const bool residual = QJL && kind == 0;
     if (STAGED && residual && tid == 0) {
-        const uint32_t bar = smem_u32(&s_bar), dst = smem_u32(s_matrices);
+        const uint32_t bar = smem_u32(&s_bar);
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         mbar_expect_tx(bar, kStagedMatrices);
-        tma_load_1d(dst, a.rot_k, kStagedMatrices / 2, bar);
-        tma_load_1d(dst + kStagedMatrices / 2, a.qjl_t, kStagedMatrices / 2, bar);
+        tma_load_1d(smem_u32(s_matrix), a.qjl_t, kStagedMatrices, bar);
     }
     float m[32];
     tq_load_column(m, a.rot_t[kind], dq, j);  // (codec constants: fetched before the wait)
+    float m2[STAGED ? 32 : 1];
+    if constexpr (STAGED) {
+        if (residual) tq_load_column(m2, a.rot_k, dq, j);
+    }
     if (tid < 16) s_bnd[tid] = a.bounds[kind][tid], s_cen[tid] = a.centers_k[tid];
     // the new vectors and the append position come from, and the cache may still be read by, the
     // preceding kernel of the stream
@@ -159,72 +165,81 @@ template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_
     }
     const int64_t row = b * a.cache_sb + h * a.cache_sh + pos0 + t;
 
-    auto block_norm = [&](float v) {  // sqrt of the sum of v*v over the 128 threads with dq == 0
+    auto block_norm = [&](float v, int which) {  // sqrt of the sum of v*v over the 128 threads with dq == 0
         float ss = dq == 0 ? v * v : 0.f;
         ss = tq_warp_sum(ss);
-        if (dq == 0 && lane == 0) s_red[j >> 5] = ss;
+        if (dq == 0 && lane == 0) s_red[which][j >> 5] = ss;
         __syncthreads();
-        const float tot = (s_red[0] + s_red[1]) + (s_red[2] + s_red[3]);
-        __syncthreads();
-        return sqrtf(tot);
+        return sqrtf((s_red[which][0] + s_red[which][1]) + (s_red[which][2] + s_red[which][3]));
     };
-    // partial of out[j] = sum_d vec[d] * m[d][j] over this thread's quarter of d
-    auto quarter = [&](const float *vec) {
+    // out[j] = sum_d u[d] * c[d][j]: the partial over this thread's quarter of d, and the sum of the four
+    auto mat_vec = [&](const float (&c)[32], int which) {
         float acc = 0.f;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) acc = fmaf(vec[32 * dq + i], m[i], acc);
-        s_part[dq][j] = acc;
+        for (int i = 0; i < 32; i += 4) {
+            const float4 u = *reinterpret_cast<const float4 *>(s_u + 32 * dq + i);
+            acc = fmaf(u.x, c[i], acc), acc = fmaf(u.y, c[i + 1], acc), acc = fmaf(u.z, c[i + 2], acc), acc = fmaf(u.w, c[i + 3], acc);
+        }
+        s_part[which][dq][j] = acc;
     };
-    auto finish = [&]() {
+    auto finish = [&](int which) {
         __syncthreads();
-        const float r = (s_part[0][j] + s_part[1][j]) + (s_part[2][j] + s_part[3][j]);
-        __syncthreads();
-        return r;
+        return (s_part[which][0][j] + s_part[which][1][j]) + (s_part[which][2][j] + s_part[which][3][j]);
+    };
+    auto put_word = [&](int w) {  // a word of the bitstream
+        ((uint32_t *)(a.codes[kind] + row * (int64_t)(16 * bits)))[w] = tq_assemble_word(s_code, w, bits);
     };
 
     const float x = tq_to_float<T>(src[j]);
-    const float nrm = block_norm(x);
+    const float nrm = block_norm(x, 0);
     const float safe = nrm > 0.0f ? nrm : 1.0f;
-    if (dq == 0) s_x[j] = x, s_u[j] = x / safe;
+    if (dq == 0) s_u[j] = x / safe;
     __syncthreads();
-    quarter(s_u);
-    auto next_column = [&](int i) {  // (a barrier separates the copies' request from every thread's wait)
-        if (STAGED) {
+    mat_vec(m, 0);
+    if (residual) {
+        if constexpr (STAGED) {  // (a barrier separates the copy's request from every thread's wait)
             if (!mbar_wait(smem_u32(&s_bar), 0) && tid == 0) atomicExch(a.error_flag, 3);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) m[e] = s_matrices[i * TQ_D * TQ_D + (32 * dq + e) * TQ_D + j];
+            for (int e = 0; e < 32; ++e) m[e] = s_matrix[(32 * dq + e) * TQ_D + j];
         } else {
-            tq_load_column(m, i == 0 ? a.rot_k : a.qjl_t, dq, j);
+            tq_load_column(m, a.rot_k, dq, j);  // in flight while the codes are formed
         }
-    };
-    if (residual) next_column(0);  // in flight while the codes are formed
-    const float z = finish();
+    }
+    const float z = finish(0);
     int idx = 0;
 #pragma unroll
     for (int e = 0; e < 15; ++e) idx += (s_bnd[e] < z) ? 1 : 0;
-    if (dq == 0) s_code[j] = (uint8_t)idx;
     const uint16_t nh = tq_float_to_half_bits(safe);
     if (tid == 0) a.norms[kind][row] = nh;
+    if (dq == 0) {
+        s_code[j] = (uint8_t)idx;
+        if (residual) s_u[j] = s_cen[idx];
+    }
     __syncthreads();
-    if (tid < 4 * bits) ((uint32_t *)(a.codes[kind] + row * (int64_t)(16 * bits)))[tid] = tq_assemble_word(s_code, tid, bits);
-
-    if (residual) {
-        __syncthreads();
-        if (dq == 0) s_u[j] = s_cen[idx];
-        __syncthreads();
-        quarter(s_u);  // sum_j c[j] * R_k[j][d], d = this thread's column
-        next_column(1);
-        const float rec = finish();
-        const float res = s_x[j] - tq_round_through<T>(rec * tq_half_bits_to_float(nh));
-        const float rn = block_norm(res);
+    if (!residual) {
+        if (tid < 4 * bits) put_word(tid);
+        return;
+    }
+    if constexpr (QJL) {
+        // sum_j c[j] * R_k[j][d], d = this thread's column
+        if constexpr (STAGED) {
+            mat_vec(m2, 1);
+        } else {
+            mat_vec(m, 1);
+            tq_load_column(m, a.qjl_t, dq, j);
+        }
+        const float rec = finish(1);
+        const float res = x - tq_round_through<T>(rec * tq_half_bits_to_float(nh));
+        const float rn = block_norm(res, 1);
         const float rsafe = rn > 0.0f ? rn : 1.0f;
         if (dq == 0) s_u[j] = res / rsafe;
         __syncthreads();
-        quarter(s_u);
-        const float pr = finish();
+        mat_vec(m, 2);
+        const float pr = finish(2);
         const uint32_t mask = __ballot_sync(0xffffffffu, pr >= 0.0f);
         if (dq == 0 && lane == 0) ((uint32_t *)(a.signs + row * 16))[j >> 5] = mask;
         if (tid == 0) a.rnorms[row] = tq_float_to_half_bits(rsafe);
+        if (tid >= TQ_D && tid < TQ_D + 4 * bits) put_word(tid - TQ_D);
     }
 }
 
@@ -237,7 +252,8 @@ template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_
 // Fragment layout per head: 8 lane variants (part * 4 + t) of 26 words: 16 rotated-query
 // words, 8 projected-query words, scale, bias.
 template <typename T> __device__ __forceinline__ void tq_qprep_block(const TqQprepArgs &a, int64_t blk) {
-    __shared__ float s_q[4][TQ_D], s_o[4][TQ_D];
+    __shared__ __align__(16) float s_q[4][TQ_D];
+    __shared__ float s_o[4][TQ_D];
     __shared__ float s_part[4][4][TQ_D];  // [quarter of d][head][column]
     __shared__ int s_x[4][TQ_D];
     __shared__ float s_scale[4], s_bias[4];
@@ -254,15 +270,17 @@ template <typename T> __device__ __forceinline__ void tq_qprep_block(const TqQpr
     tq_load_column(m, proj ? a.qjl_t : a.rot_k_t, dq, j);  // (codec constants: fetched before the wait)
     tq_grid_dependency_wait();   // the query comes from the preceding kernel of the stream
     tq_launch_dependents();      // the decode kernel may begin its set-up now
-    if (dq < G) s_q[dq][j] = tq_to_float<T>(((const T *)a.q)[(head0 + dq) * TQ_D + j]);
+    s_q[dq][j] = dq < G ? tq_to_float<T>(((const T *)a.q)[(head0 + dq) * TQ_D + j]) : 0.f;
     __syncthreads();
     {
         float r[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const int d = 32 * dq + i;
+        for (int i = 0; i < 32; i += 4) {
 #pragma unroll
-            for (int g = 0; g < 4; ++g) r[g] = fmaf(g < G ? s_q[g][d] : 0.f, m[i], r[g]);
+            for (int g = 0; g < 4; ++g) {
+                const float4 q = *reinterpret_cast<const float4 *>(&s_q[g][32 * dq + i]);
+                r[g] = fmaf(q.x, m[i], r[g]), r[g] = fmaf(q.y, m[i + 1], r[g]), r[g] = fmaf(q.z, m[i + 2], r[g]), r[g] = fmaf(q.w, m[i + 3], r[g]);
+            }
         }
 #pragma unroll
         for (int g = 0; g < 4; ++g) s_part[dq][g][j] = r[g];
