@@ -94,7 +94,7 @@ struct Mma4Args {
     // planned by the kernel for its own grid.
     const int *len_ptr;
     int len_add, capacity;
-    const uint32_t *frag;  // per query head: TQ_FRAG_ROW_WORDS words, see tq_qprep_frag_kernel
+    const uint32_t *frag;  // per query head: TQ_FRAG_ROW_WORDS words, see tq_qprep_block
     float *part_m, *part_l, *part_acc;
     const float *centers_k, *centers_v;
     int *error_flag;  // set to 1 when a bounded wait ran out
@@ -358,24 +358,24 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
     uint32_t bp[QJL ? 4 * NH : 1][2];  // wide: [0, 4) hi terms, [4, 8) lo terms
     float sign_scale[NH], sign_bias[NH];  // for the heads this lane owns in the softmax
     {
-        const uint32_t *head_frag = a.frag + (q_row0 + (live ? hcol : 0)) * TQ_FRAG_ROW_WORDS;
-        const uint2 *fr = reinterpret_cast<const uint2 *>(head_frag + (part * 4 + t) * 26);
+        const int plane = 8 * G;
+        const uint2 *planes = reinterpret_cast<const uint2 *>(a.frag + q_row0 * TQ_FRAG_ROW_WORDS);
+        const uint2 *fr = planes + 8 * (live ? hcol : 0) + 4 * part + t;
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
-            const uint2 v = __ldg(fr + s);
+            const uint2 v = __ldg(fr + s * plane);
             bq[s][0] = live ? v.x : 0u, bq[s][1] = live ? v.y : 0u;
         }
         if (QJL) {
 #pragma unroll
             for (int n = 0; n < 4; ++n) {
-                const uint2 v = __ldg(fr + 8 + n);
+                const uint2 v = __ldg(fr + (8 + n) * plane);
                 bp[n][0] = live ? v.x : 0u, bp[n][1] = live ? v.y : 0u;
             }
             if (WIDE) {
-                const uint2 *fl = reinterpret_cast<const uint2 *>(head_frag + (4 + t) * 26);
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
-                    const uint2 v = __ldg(fl + 8 + n);
+                    const uint2 v = __ldg(fr + (8 + n) * plane + 4);
                     bp[(QJL && WIDE ? 4 : 0) + n][0] = live ? v.x : 0u, bp[(QJL && WIDE ? 4 : 0) + n][1] = live ? v.y : 0u;
                 }
             }
@@ -383,9 +383,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
 #pragma unroll
         for (int hl = 0; hl < NH; ++hl) {
             const int head = WIDE ? 2 * t + hl : t;
-            const uint32_t *mine = a.frag + (q_row0 + (head < G ? head : 0)) * TQ_FRAG_ROW_WORDS;
-            sign_scale[hl] = QJL ? __uint_as_float(__ldg(mine + 24)) : 0.f;
-            sign_bias[hl] = QJL ? __uint_as_float(__ldg(mine + 25)) : 0.f;
+            const uint2 v = QJL ? __ldg(planes + 12 * plane + (head < G ? head : 0)) : make_uint2(0u, 0u);
+            sign_scale[hl] = __uint_as_float(v.x), sign_bias[hl] = __uint_as_float(v.y);
         }
     }
     if (seg_no == 0) TQ_STAMP(3);

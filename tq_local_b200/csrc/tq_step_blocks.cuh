@@ -38,13 +38,14 @@ struct TqQprepArgs {
     const void *q;          // [kv_rows * G][128] in the query dtype
     const float *rot_k_t;   // R_k^T[d][j]
     const float *qjl_t;     // S^T[d][i]
-    uint32_t *frag;         // [kv_rows * G][TQ_FRAG_WORDS]
+    uint32_t *frag;         // [kv_rows * G][TQ_FRAG_ROW_WORDS]
     int G, use_qjl;
     int64_t kv_rows;
 };
 
-// Words per query head in the fragment area: 8 lane variants of 26 words, padded to the size
-// of the rotated + projected query rows the area overlays in the decode workspace.
+// Words per query head in the fragment area: the size of the rotated + projected query rows the area overlays in the decode
+// workspace.  A KV row's fragments begin at its first head's words: twelve planes of [8 G] pairs of words, in the order of
+// the decode kernel's lanes (see tq_qprep_block), then two floats a head.
 #define TQ_FRAG_ROW_WORDS (2 * TQ_D + 8)
 
 // How the decode kernel cuts the (batch, KV head) rows, laid end to end and each padded to
@@ -249,8 +250,10 @@ template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_
 // blocks rotate their heads (q @ R_k^T) and write the f16 hi / lo MMA fragments; the next
 // kv_rows * ceil(G / 4) blocks project them (q @ S^T), quantise the result to 16-bit fixed
 // point and write the s8 hi / lo fragments with the scale and bias that undo it.
-// Fragment layout per head: 8 lane variants (part * 4 + t) of 26 words: 16 rotated-query
-// words, 8 projected-query words, scale, bias.
+// Fragment layout per KV row: planes p of 8 G pairs of words, pair 8 h + 4 part + t of head h: planes 0..7 the rotated query's words 2p
+// and 2p + 1 for lane (part, t), planes 8..11 the projected query's; then scale and bias of every head.  The decode kernel's
+// lanes read a plane in one piece: with the 26 words of a (head, part, t) side by side every lane's load took a sector of
+// its own, in each of sixteen warps: 1.05 us between the wait and the first iteration, 0.8 now.
 template <typename T> __device__ __forceinline__ void tq_qprep_block(const TqQprepArgs &a, int64_t blk) {
     __shared__ __align__(16) float s_q[4][TQ_D];
     __shared__ float s_o[4][TQ_D];
@@ -288,21 +291,26 @@ template <typename T> __device__ __forceinline__ void tq_qprep_block(const TqQpr
     __syncthreads();
     s_o[dq][j] = (s_part[0][dq][j] + s_part[1][dq][j]) + (s_part[2][dq][j] + s_part[3][dq][j]);  // head dq
     __syncthreads();
+    uint2 *const planes = reinterpret_cast<uint2 *>(a.frag + R * a.G * TQ_FRAG_ROW_WORDS);
     if (!proj) {
-        // one thread per word: G heads x 8 variants x 16 words; dims 32t + 4*(k/2) + 2*(k%2) + {0, 1}
-        for (int w = tid; w < G * 8 * 16; w += blockDim.x) {
-            const int variant = w >> 4, k = w & 15;
-            const int hcol = variant >> 3, part = (variant >> 2) & 1, t = variant & 3;
-            const int d0 = 32 * t + 4 * (k >> 1) + 2 * (k & 1);
-            float x[2];
+        // one thread per pair of words: G heads x 8 variants x 8 pairs; dims 32t + 4p + {0, 1} and {2, 3}
+        for (int w = tid; w < G * 8 * 8; w += blockDim.x) {
+            const int p = w / (8 * G), at = w % (8 * G);
+            const int hcol = at >> 3, part = (at >> 2) & 1, d0 = 32 * (at & 3) + 4 * p;
+            uint32_t word[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const float v = s_o[hcol][d0 + i];
-                const float hi = __half2float(__float2half_rn(v));
-                x[i] = part ? (v - hi) : hi;
+                float x[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float v = s_o[hcol][d0 + 2 * i + e];
+                    const float hi = __half2float(__float2half_rn(v));
+                    x[e] = part ? (v - hi) : hi;
+                }
+                const __half2 hh = __floats2half2_rn(x[0], x[1]);
+                word[i] = *reinterpret_cast<const uint32_t *>(&hh);
             }
-            const __half2 hh = __floats2half2_rn(x[0], x[1]);
-            a.frag[(head0 + hcol) * TQ_FRAG_ROW_WORDS + (variant & 7) * 26 + k] = *reinterpret_cast<const uint32_t *>(&hh);
+            planes[p * 8 * a.G + 8 * h0 + at] = make_uint2(word[0], word[1]);
         }
         return;
     }
@@ -327,25 +335,23 @@ template <typename T> __device__ __forceinline__ void tq_qprep_block(const TqQpr
         }
     }
     __syncthreads();
-    // G heads x 8 variants x 10 words: s8 hi / lo terms behind sign bits (n + 4 rr) + 8j, scale, bias.
+    // G heads x 8 variants x 4 pairs of words: s8 hi / lo terms behind sign bits (n + 4 rr) + 8j; then scale and bias.
     // The decode kernel's operand byte for such a bit is 2^n (the bit is masked in place, not moved),
     // so the term stored here is x / 2^n, rounded: at most three of the sixteen bits are given up.
-    for (int w = tid; w < G * 8 * 10; w += blockDim.x) {
-        const int variant = w / 10, k = w % 10;
-        const int hcol = variant >> 3, part = (variant >> 2) & 1, t = variant & 3;
-        uint32_t word = 0;
-        if (k < 8) {
-            const int n = k >> 1, rr = k & 1;
+    for (int w = tid; w < G * 8 * 4; w += blockDim.x) {
+        const int n = w / (8 * G), at = w % (8 * G);
+        const int hcol = at >> 3, part = (at >> 2) & 1, t = at & 3;
+        uint32_t word[2] = {0, 0};
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr)
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj) {
                 const int x16 = (s_x[hcol][32 * t + (n + 4 * rr) + 8 * jj] + ((1 << n) >> 1)) >> n;
                 const int hi8 = (x16 + 128) >> 8;
                 const int lo8 = x16 - (hi8 << 8);
-                word |= (uint32_t)((part ? lo8 : hi8) & 0xff) << (8 * jj);
+                word[rr] |= (uint32_t)((part ? lo8 : hi8) & 0xff) << (8 * jj);
             }
-        } else {
-            word = __float_as_uint(k == 8 ? s_scale[hcol] : s_bias[hcol]);
-        }
-        a.frag[(head0 + hcol) * TQ_FRAG_ROW_WORDS + (variant & 7) * 26 + 16 + k] = word;
+        planes[(8 + n) * 8 * a.G + 8 * h0 + at] = make_uint2(word[0], word[1]);
     }
+    if (tid < G) planes[12 * 8 * a.G + h0 + tid] = make_uint2(__float_as_uint(s_scale[tid]), __float_as_uint(s_bias[tid]));
 }
