@@ -195,6 +195,28 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
     // so that these few bytes do not queue behind the ring's first fill
     const float ck = a.centers_k[lane & 15], cv = a.centers_v[lane & 15];
 
+    // A warp belongs to ring group gq and is its warp wq (see below).
+    const int gq = warp % kGroups, wq = warp / kGroups;
+    // ---- per-lane replicated f16x2 centre-pair tables (keys in the low half of each slot); a warp fills one slot at a time, lane l
+    // writing words l and 32+l (no bank conflicts).  The warps that set no ring slot up begin at once, beside the
+    // length's arrival, the plan and the first fills, and take three quarters of it: eight layer steps at 4099 tokens 90.6 us, 92.3
+    // with all warps building it after the first fills, 4 x 4 x 8191 of seven heads 71.9 and 73.7 (four layers).  The wide variant
+    // with the sketch, which fills its 128 registers, loses more in its loop than it gains (8 x 4 x 32768 of seven heads
+    // 56.0 against 54.2) and builds the table late.  The largest caches take 0.5 us more (8 x 8 x 32768 75.2 against 74.7).
+    constexpr bool kEarly = !(WIDE && QJL);
+    auto build_table = [&](int from, int to, int first, int stride) {
+        constexpr int mk = (1 << KB) - 1, mv = (1 << VB) - 1;
+        for (int e = from + first; e < to; e += stride) {
+            uint32_t *slot = table + e * kSlotWords;
+            const float klo = __shfl_sync(0xffffffffu, ck, e & mk), khi = __shfl_sync(0xffffffffu, ck, (e >> KB) & mk);
+            const float vlo = __shfl_sync(0xffffffffu, cv, e & mv), vhi = __shfl_sync(0xffffffffu, cv, (e >> VB) & mv);
+            slot[lane] = pack_half2(klo, khi);
+            slot[32 + lane] = pack_half2(vlo, vhi);
+        }
+    };
+    static_assert(kGroupWarps == 2 * kStages, "half of the warps set ring slots up");
+    if (kEarly && wq >= kStages) build_table(0, 192, gq + kGroups * (wq - kStages), kWarps / 2);
+
     int N = a.N, n_pad = a.n_pad, chunk = a.chunk, stable_len = a.stable_len;
     if (a.len_ptr) {
         stable_len = *a.len_ptr;
@@ -212,7 +234,6 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
     // schedulers, so the schedulers carry identical loads and the groups finish together (with
     // consecutive warps per group every scheduler held one warp of each group, the groups ran at
     // different rates and the slowest one finished 4.5 us after the fastest, alone on the SM).
-    const int gq = warp % kGroups, wq = warp / kGroups;
     auto slot_u32 = [&](int st) -> uint32_t {
         const int q = gq * kStages + st;
         return q < slots_low ? dyn_base + q * L::kBytes : high_base + (q - slots_low) * L::kBytes;
@@ -299,19 +320,8 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
         }
     }
 
-    // ---- per-lane replicated f16x2 centre-pair tables (keys in the low half of each slot);
-    // a warp fills one slot at a time, lane l writing words l and 32+l (no bank conflicts)
-    {
-        constexpr int mk = (1 << KB) - 1, mv = (1 << VB) - 1;
-        for (int e = warp; e < kEntries; e += kWarps) {
-            uint32_t *slot = table + e * kSlotWords;
-            const float klo = __shfl_sync(0xffffffffu, ck, e & mk), khi = __shfl_sync(0xffffffffu, ck, (e >> KB) & mk);
-            const float vlo = __shfl_sync(0xffffffffu, cv, e & mv), vhi = __shfl_sync(0xffffffffu, cv, (e >> VB) & mv);
-            slot[lane] = pack_half2(klo, khi);
-            slot[32 + lane] = pack_half2(vlo, vhi);
-        }
-    }
-
+    if (!kEarly) build_table(0, kEntries, warp, kWarps);
+    else if (wq < kStages) build_table(192, kEntries, gq + kGroups * wq, kWarps / 2);
     __syncthreads();  // tables complete
     TQ_STAMP(1);
 
