@@ -197,26 +197,6 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
 
     // A warp belongs to ring group gq and is its warp wq (see below).
     const int gq = warp % kGroups, wq = warp / kGroups;
-    // ---- per-lane replicated f16x2 centre-pair tables (keys in the low half of each slot); a warp fills one slot at a time, lane l
-    // writing words l and 32+l (no bank conflicts).  The warps that set no ring slot up begin at once, beside the
-    // length's arrival, the plan and the first fills, and take three quarters of it: eight layer steps at 4099 tokens 90.6 us, 92.3
-    // with all warps building it after the first fills, 4 x 4 x 8191 of seven heads 71.9 and 73.7 (four layers).  The wide variant
-    // with the sketch, which fills its 128 registers, loses more in its loop than it gains (8 x 4 x 32768 of seven heads
-    // 56.0 against 54.2) and builds the table late.  The largest caches take 0.5 us more (8 x 8 x 32768 75.2 against 74.7).
-    constexpr bool kEarly = !(WIDE && QJL);
-    auto build_table = [&](int from, int to, int first, int stride) {
-        constexpr int mk = (1 << KB) - 1, mv = (1 << VB) - 1;
-        for (int e = from + first; e < to; e += stride) {
-            uint32_t *slot = table + e * kSlotWords;
-            const float klo = __shfl_sync(0xffffffffu, ck, e & mk), khi = __shfl_sync(0xffffffffu, ck, (e >> KB) & mk);
-            const float vlo = __shfl_sync(0xffffffffu, cv, e & mv), vhi = __shfl_sync(0xffffffffu, cv, (e >> VB) & mv);
-            slot[lane] = pack_half2(klo, khi);
-            slot[32 + lane] = pack_half2(vlo, vhi);
-        }
-    };
-    static_assert(kGroupWarps == 2 * kStages, "half of the warps set ring slots up");
-    if (kEarly && wq >= kStages) build_table(0, 192, gq + kGroups * (wq - kStages), kWarps / 2);
-
     int N = a.N, n_pad = a.n_pad, chunk = a.chunk, stable_len = a.stable_len;
     if (a.len_ptr) {
         stable_len = *a.len_ptr;
@@ -320,8 +300,22 @@ __global__ void __launch_bounds__(kWarps * 32, 1) tq_decode_mma4_kernel(Mma4Args
         }
     }
 
-    if (!kEarly) build_table(0, kEntries, warp, kWarps);
-    else if (wq < kStages) build_table(192, kEntries, gq + kGroups * wq, kWarps / 2);
+    // ---- per-lane replicated f16x2 centre-pair tables (keys in the low half of each slot); a warp fills one slot at a time, lane l
+    // writing words l and 32+l (no bank conflicts).  The warps that set no ring slot up build all of it, beside the first fills that the
+    // others request.  By all warps after those fills: 4 x 4 x 8192 of seven heads 16.5 us instead of 16.0, 1 x 8 x 4099
+    // 11.07 instead of 10.86, 64 x 8 x 500 48.5 instead of 47.1.  Three quarters of it ahead of the length and the rest by the others gave the loop
+    // below slower code: 8 x 8 x 32768 75.6 instead of 74.8, 4 x 8 x 131072 at 3 bits 139.1 instead of 137.1.
+    static_assert(kGroupWarps == 2 * kStages, "half of the warps set ring slots up");
+    if (wq >= kStages) {
+        constexpr int mk = (1 << KB) - 1, mv = (1 << VB) - 1;
+        for (int e = gq + kGroups * (wq - kStages); e < kEntries; e += kWarps / 2) {
+            uint32_t *slot = table + e * kSlotWords;
+            const float klo = __shfl_sync(0xffffffffu, ck, e & mk), khi = __shfl_sync(0xffffffffu, ck, (e >> KB) & mk);
+            const float vlo = __shfl_sync(0xffffffffu, cv, e & mv), vhi = __shfl_sync(0xffffffffu, cv, (e >> VB) & mv);
+            slot[lane] = pack_half2(klo, khi);
+            slot[32 + lane] = pack_half2(vlo, vhi);
+        }
+    }
     __syncthreads();  // tables complete
     TQ_STAMP(1);
 
