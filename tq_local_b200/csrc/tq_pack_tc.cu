@@ -656,11 +656,15 @@ int32_t tq_launch_pack_tc(tq_ctx *ctx, const tq_dense_desc *k, const tq_dense_de
     a.signs = cache->k_signs, a.rnorms = cache->k_rnorms;
     a.n_tiles = (int)((a.vec.n + kUmmaRows - 1) / kUmmaRows);
     // One CTA per SM.  With tiles enough for all of them, keys with the sketch get the share of the SMs that
-    // their cost asks for (2 x 8 x 32768 bf16 at 66, 68, 70, 72 %: 220, 211, 203, 214 us; 3 bits 214, 213, 227, 240; f16 211, 203, 194, 194); with few
-    // tiles each side gets a CTA
-    // per tile, and no SM two (8 x 1000 vectors a tensor: 16 us, 31 us in two launches).
+    // their cost asks for, which depends on the type (fp32 rows go straight to registers, which tells most on values) and on
+    // what the bits leave to search.  2 x 8 x 32768 vectors a tensor, us at 92, 94, 98 and 103 of 148 SMs: bf16 4 bits 236, 229, 221, 210,
+    // 3 bits 230, 223, 215, 229, 2 bits 206, 199, 193, 214; f16 3 bits 225, 219, 209, 200 (4 and 2 bits alike); fp32 4 bits
+    // 399, 389, 403, 446, 3 bits 365, 375, 405, 447, 2 bits 330, 340, 364, 401.  The same places are best from 8 x 11000 to
+    // 40 x 20011 vectors.  With few tiles each side gets a CTA per tile, and no SM two (8 x 1000 vectors a tensor:
+    // 16 us, 31 us in two launches).
     const int sms = ctx->sm_count;
-    int key_ctas = !k ? 0 : qjl ? sms * 7 / 10 : sms / 2, val_ctas = sms - key_ctas;
+    const int share = v->dtype == TQ_DTYPE_F32 ? (ctx->bits == 4 ? 640 : 625) : v->dtype == TQ_DTYPE_BF16 && ctx->bits < 4 ? 665 : 700;  // of 1000
+    int key_ctas = !k ? 0 : qjl ? sms * share / 1000 : sms / 2, val_ctas = sms - key_ctas;
     if (k && a.n_tiles <= sms / 2) key_ctas = val_ctas = a.n_tiles;
     key_ctas = key_ctas < a.n_tiles ? key_ctas : a.n_tiles, val_ctas = val_ctas < a.n_tiles ? val_ctas : a.n_tiles;
     a.key_ctas = key_ctas;
