@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(4 * TQ_D, STAGED ? 1 : 2) tq_step_prologue_ker
     if ((int)blockIdx.x < n_qprep)
         tq_qprep_block<T>(qa, blockIdx.x);
     else
-        tq_pack_small_block<T, QJL, STAGED>(pa, (int64_t)blockIdx.x - n_qprep);
+        tq_pack_small_block<T, QJL, STAGED, true>(pa, (int64_t)blockIdx.x - n_qprep);
 }
 
 // Publishing rows to the peers and waiting for theirs (system scope, PTX memory model):

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) tq_pack_rows_kernel(PackA
 // one 512-thread block per vector, see tq_pack_small_block.
 template <typename T, bool QJL, bool STAGED>
 __global__ void __launch_bounds__(4 * TQ_D, STAGED ? 1 : 2) tq_pack_small_kernel(PackArgs a) {
-    tq_pack_small_block<T, QJL, STAGED>(a, blockIdx.x);
+    tq_pack_small_block<T, QJL, STAGED, false>(a, blockIdx.x);
 }
 
 struct DequantArgs {

@@ -1,8 +1,8 @@
 // Block-level bodies of the latency-bound kernels of a decode step: query preparation and
 // the append of the step's new key / value vectors.  They live in a header so that one
 // launch can run both kinds of block side by side (tq_step_prologue_kernel) and the
-// stand-alone kernels share the same code.  Every body is written for 512 threads and at
-// most 64 registers, so two blocks fit an SM and a whole step's prologue is one wave.
+// stand-alone kernels share the same code.  Every body is written for 512 threads; all but the staged append
+// (see kStagedMatrices) are held to 64 registers, so that two blocks fit an SM and a whole step's prologue is one wave.
 //
 // All mat-vecs use the same shape: thread (j, dq) owns output column j and the 32 matrix
 // rows [32 dq, 32 dq + 32); its 32 matrix elements are loaded into registers in one batch
@@ -112,15 +112,17 @@ __device__ __forceinline__ uint32_t tq_assemble_word(const uint8_t *codes, int w
 // Encode one vector (item < n_vec: kind first_kind, else the next kind) and write it at its
 // cache row.  fp32 arithmetic in a fixed order: partial sums over four 32-row quarters, then
 // (p0 + p1) + (p2 + p3).
-// A key with a sketch is a chain of three mat-vecs, and the whole step waits for it.  STAGED (64 KB of dynamic shared memory and all
-// registers of an SM, for launches of no more blocks than SMs): the columns of the first two matrices are in registers before the
+// A key with a sketch is a chain of three mat-vecs, and the whole step waits for it.  STAGED (64 KB of dynamic shared memory and
+// over 100 registers a thread, so one block to an SM, for launches of no more blocks than SMs): the columns of the first two matrices are in registers before the
 // vector is there, the third matrix was requested by bulk copy before anything else and its column takes the first one's registers
 // while the codes are found; the bitstream, a loop of byte reads, is assembled by a warp of its own at the end.  From the vector's
 // arrival to the last store 2.3 us; 3.4 with two matrices staged, columns taken from shared memory between two barriers and the bitstream
 // before the second mat-vec; otherwise the columns are read from L2 in turn, 64 KB a mat-vec and a microsecond of the chain.
+// DEPENDENT: launched ahead of the kernel that brings the vector.  Else the vector is there, and its load goes ahead of the second
+// column's, 64 KB that its norm would wait for (append of 1 x 8 tokens 5.28 us, 5.17 like this).
 constexpr int kStagedMatrices = TQ_D * TQ_D * 4;
 inline bool tq_stages_matrices(const tq_ctx *ctx, int64_t blocks) { return ctx->use_qjl && blocks <= ctx->sm_count; }
-template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_pack_small_block(const TqPackArgs &a, int64_t item) {
+template <typename T, bool QJL, bool STAGED, bool DEPENDENT> __device__ __forceinline__ void tq_pack_small_block(const TqPackArgs &a, int64_t item) {
     extern __shared__ __align__(128) float s_matrix[];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ __align__(16) float s_u[TQ_D];
@@ -149,7 +151,7 @@ template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_
     tq_load_column(m, a.rot_t[kind], dq, j);  // (codec constants: fetched before the wait)
     float m2[STAGED ? 32 : 1];
     if constexpr (STAGED) {
-        if (residual) tq_load_column(m2, a.rot_k, dq, j);
+        if (DEPENDENT && residual) tq_load_column(m2, a.rot_k, dq, j);
     }
     if (tid < 16) s_bnd[tid] = a.bounds[kind][tid], s_cen[tid] = a.centers_k[tid];
     // the new vectors and the append position come from, and the cache may still be read by, the
@@ -192,6 +194,9 @@ template <typename T, bool QJL, bool STAGED> __device__ __forceinline__ void tq_
     };
 
     const float x = tq_to_float<T>(src[j]);
+    if constexpr (STAGED && !DEPENDENT) {
+        if (residual) tq_load_column(m2, a.rot_k, dq, j);  // (behind the vector, which nobody had to wait for)
+    }
     const float nrm = block_norm(x, 0);
     const float safe = nrm > 0.0f ? nrm : 1.0f;
     if (dq == 0) s_u[j] = x / safe;
