@@ -776,7 +776,6 @@ static void configure_small_kernels() {
     prefer_max_shared(tq_qprep_kernel<float>);
     prefer_max_shared(tq_qprep_kernel<__half>);
     prefer_max_shared(tq_qprep_kernel<__nv_bfloat16>);
-    prefer_max_shared(tq_qprep_frag_kernel<float>);
     prefer_max_shared(tq_qprep_frag_kernel<__half>);
     prefer_max_shared(tq_qprep_frag_kernel<__nv_bfloat16>);
     prefer_max_shared(tq_combine_group_kernel<float, false>);
@@ -788,9 +787,6 @@ static void configure_small_kernels() {
     prefer_max_shared(tq_combine_group_kernel<float, true>);
     prefer_max_shared(tq_combine_group_kernel<__half, true>);
     prefer_max_shared(tq_combine_group_kernel<__nv_bfloat16, true>);
-    prefer_max_shared(tq_step_prologue_kernel<float, true, true>);
-    prefer_max_shared(tq_step_prologue_kernel<float, true, false>);
-    prefer_max_shared(tq_step_prologue_kernel<float, false, false>);
     prefer_max_shared(tq_step_prologue_kernel<__half, true, true>);
     prefer_max_shared(tq_step_prologue_kernel<__half, true, false>);
     prefer_max_shared(tq_step_prologue_kernel<__half, false, false>);
@@ -834,13 +830,12 @@ static cudaError_t launch_prologue(tq_ctx *ctx, const TqQprepArgs &qa, const TqP
 int32_t tq_launch_qprep_frag(tq_ctx *ctx, const void *q, int32_t q_dtype, int64_t kv_rows, int G, uint32_t *frag,
                              const TqPackArgs *append, cudaStream_t stream) {
     configure_small_kernels();
-    if (G > 8) return TQ_ERR_UNSUPPORTED;
+    if (G > 8 || q_dtype == TQ_DTYPE_F32) return TQ_ERR_UNSUPPORTED;  // (fp32 caches take the exact kernel, with tq_launch_qprep)
     TqQprepArgs qa;
     qa.q = q, qa.rot_k_t = ctx->rot_k_t, qa.qjl_t = ctx->qjl_t, qa.frag = frag;
     qa.G = G, qa.use_qjl = ctx->use_qjl, qa.kv_rows = kv_rows;
     cudaError_t e;
-    if (q_dtype == TQ_DTYPE_F32) e = launch_prologue<float>(ctx, qa, append, stream);
-    else if (q_dtype == TQ_DTYPE_F16) e = launch_prologue<__half>(ctx, qa, append, stream);
+    if (q_dtype == TQ_DTYPE_F16) e = launch_prologue<__half>(ctx, qa, append, stream);
     else e = launch_prologue<__nv_bfloat16>(ctx, qa, append, stream);
     TQ_CUDA_CHECK(e);
     return TQ_OK;
