@@ -240,19 +240,63 @@ def test_fp32_attention(setup_golden, bits, qjl, groups, n):
 MODES = [(2, False), (3, False), (4, False), (2, True), (3, True), (4, True)]
 
 
-@pytest.mark.parametrize("bits,qjl", [(2, False), (3, False), (4, False), (2, True), (3, True), (4, True)])
+# The unrounded 16-bit kernels against 64 bits, relative to the largest output: weights and value centres are f16 (2^-11 each),
+# key centres too, which moves a logit of order 1 by a few 2^-12: 2e-3 in all.  Typical is a tenth of it, since roundings of many
+# tokens cancel.
+UNROUNDED_TOL = 2e-3
+
+
+@pytest.mark.parametrize("bits,qjl", MODES)
 @pytest.mark.parametrize("groups", [1, 2, 3, 4, 5, 8])
-@pytest.mark.parametrize("n", [1, 6, 17, 31, 33, 130, 513])
-def test_16bit_attention_unrounded(setup_golden, bits, qjl, groups, n):
-    """The tensor-core kernels at every code width, on both sides of a tile, a warp's tokens and a step, against 64 bits."""
+@pytest.mark.parametrize("dtype", [BF16, F16])
+def test_16bit_attention_unrounded(setup_golden, bits, qjl, groups, dtype):
+    """The tensor-core kernels at every code width, on both sides of and at a tile of 16 tokens, a warp's 32 and a step of 512."""
     from tq_local_b200.runtime.packed_store import PackedStore
 
-    dtype = (BF16, F16)[(n + groups) % 2]
     p, codec = oracle_params(bits, qjl, setup_golden), make_codec(bits, qjl, setup_golden)
-    store = PackedStore(codec, 2, 3, capacity=n)
-    store.pack(vectors((2, 3, n, 128), 5 + n, dtype), vectors((2, 3, n, 128), 6 + n, dtype))
-    q = query((2, 3 * groups, 1), 7 + n, dtype)
-    assert rel_inf(store.decode_attn_f32(q), attend64(store, p, q, groups)) <= 2e-3
+    store = PackedStore(codec, 2, 3, capacity=513)
+    for n in (1, 6, 15, 16, 17, 31, 32, 33, 130, 511, 512, 513):
+        store.length = 0
+        store.pack(vectors((2, 3, n, 128), 5 + n, dtype), vectors((2, 3, n, 128), 6 + n, dtype))
+        q = query((2, 3 * groups, 1), 7 + n, dtype)
+        assert rel_inf(store.decode_attn_f32(q), attend64(store, p, q, groups)) <= UNROUNDED_TOL, n
+
+
+@pytest.mark.parametrize("bits,qjl", MODES)
+@pytest.mark.parametrize("groups", [1, 3, 4, 5, 8])
+@pytest.mark.parametrize("dtype", [BF16, F16])
+def test_16bit_attention_of_long_rows(setup_golden, bits, qjl, groups, dtype):
+    """Up to ten iterations a warp under growing logits, so that the accumulators are rescaled again and again; whole rows to a CTA
+    and rows cut by chunks, with the last steps empty for some warps."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(bits, qjl, setup_golden), make_codec(bits, qjl, setup_golden)
+    n = 5003
+    k = vectors((1, 3, n, 128), 1, F32) * torch.linspace(0.2, 1.2, n, device="cuda")[:, None]
+    store = PackedStore(codec, 1, 3, capacity=n)
+    store.pack(k.to(dtype), vectors((1, 3, n, 128), 2, dtype))
+    q = query((1, 3 * groups, 1), 3, dtype)
+    want = attend64(store, p, q, groups)
+    for splits in (1, 3, 4, None):
+        assert rel_inf(store.decode_attn_f32(q, splits=splits), want) <= UNROUNDED_TOL, splits
+    assert codec.device_status() == 0
+
+
+@pytest.mark.parametrize("bits,qjl", MODES)
+@pytest.mark.parametrize("groups", [2, 4, 5, 8])
+@pytest.mark.parametrize("dtype", [BF16, F16])
+def test_16bit_attention_of_many_rows(setup_golden, bits, qjl, groups, dtype):
+    """More rows than SMs and a ragged length: a CTA goes from one row to the next and merges its warps for each of them."""
+    from tq_local_b200.runtime.packed_store import PackedStore
+
+    p, codec = oracle_params(bits, qjl, setup_golden), make_codec(bits, qjl, setup_golden)
+    store = PackedStore(codec, 41, 8, capacity=700)
+    for n in (67, 700):
+        store.length = 0
+        store.pack(vectors((41, 8, n, 128), 5 + n, dtype), vectors((41, 8, n, 128), 6 + n, dtype))
+        q = query((41, 8 * groups, 1), 7 + n, dtype)
+        assert rel_inf(store.decode_attn_f32(q), attend64(store, p, q, groups)) <= UNROUNDED_TOL, n
+    assert codec.device_status() == 0
 
 
 @pytest.mark.parametrize("dtype", [BF16, F16, F32])

@@ -215,12 +215,13 @@ template <typename T, bool QJL, bool STAGED, bool DEPENDENT> __device__ __forcei
     int idx = 0;
 #pragma unroll
     for (int e = 0; e < 15; ++e) idx += (s_bnd[e] < z) ? 1 : 0;
-    const uint16_t nh = tq_float_to_half_bits(safe);
-    if (tid == 0) a.norms[kind][row] = nh;
     if (dq == 0) {
         s_code[j] = (uint8_t)idx;
         if (residual) s_u[j] = s_cen[idx];
     }
+    // (after the codes: ahead of them, 32 x 8 tokens without the sketch take 7.64 us instead of 7.18, 1 x 8 3.38 instead of 3.26)
+    const uint16_t nh = tq_float_to_half_bits(safe);
+    if (tid == 0) a.norms[kind][row] = nh;
     __syncthreads();
     if (!residual) {
         if (tid < 4 * bits) put_word(tid);
