@@ -25,7 +25,7 @@
 // shared-memory and TMEM traffic).  The issuing thread is elected in a converged warp and the accumulator's address is
 // uniform, which leaves an instruction or two per MMA: with a thread chosen by its index the operands went through vector
 // registers, and sixteen MMAs took 2000 - 2400 cycles to issue between the other warps' instructions.
-// 2 x 8 x 32768 keys and values, 4 bits with the sketch: bf16 242 -> 203 us, f16 252 -> 194; 3 bits 259 -> 213, 269 -> 194; 4 bits
+// 2 x 8 x 32768 keys and values, 4 bits with the sketch: bf16 242 -> 203 us, f16 252 -> 194; 3 bits 259 -> 215, 269 -> 200; 4 bits
 // without 142 -> 128, 124 -> 114 (before: look-ups one by one, bulk copies, issue by index).  All sixteen warps of a
 // group on one tile at a time with dedicated loading and issuing warps, two tiles in flight: 262 us and more, too few warps to hide the
 // latencies of a phase.
